@@ -283,3 +283,74 @@ def tolerance(case):
         # taken twice differs by 2e-4 in norm (most of it in the loss) and 4e-3 in the worst element.
         return {'rel': 1e-3, 'max': 0.02}
     return {'rel': 2.5e-3, 'max': 0.06} if case['dtype'] == 'fp16' else {'rel': 2e-2, 'max': 0.5}
+
+
+# ----------------------------------------------------------------------------
+# The same pass in 64 bits, in plain torch
+# ----------------------------------------------------------------------------
+def _exact_layer(case, state):
+    train, top_k, experts = case['train'], case['top_k'], case['experts']
+    dtype, glu = _DTYPES[case['dtype']], case['mlp'] == 'glu'
+    names = [name for name, _ in state['layer'].named_parameters()]
+    params = [p.detach().double().requires_grad_(train) for p in state['params']]
+    by_name = {name.rsplit('.', 1)[-1]: p for name, p in zip(names, params)}
+    x = state['x'].detach().double().requires_grad_(train)
+    rows = x.reshape(-1, case['hidden'])
+    logits = rows @ by_name['weight'].t()
+    with torch.no_grad():       # the choice is made on scores rounded to the layer's type, ties to the lowest id
+        rounded = logits.to(dtype).double().softmax(-1).to(dtype)
+        choice = torch.sort(rounded.float(), dim=-1, descending=True, stable=True)[1][:, :top_k]
+    scores = logits.softmax(-1)
+    weights = scores.gather(1, choice)
+    if glu:
+        weights = weights / weights.abs().sum(-1, keepdim=True)
+    counts = torch.bincount(choice.flatten(), minlength=experts)
+    capacity = int(top_k * case['tokens'] / experts) or int(counts.max())
+    out = 0
+    for e in range(experts):
+        token, slot = (choice == e).nonzero(as_tuple=True)      # in token order
+        if not case['dropless']:
+            token, slot = token[:capacity], slot[:capacity]
+        w1, w2 = by_name['w1'].view(experts, -1, by_name['w1'].shape[-1])[e], by_name['w2'].view(
+            experts, -1, case['hidden'])[e]
+        z = rows[token] @ (w1.t() if case['dropless'] else w1)
+        if glu:
+            h = F.silu(z) * (rows[token] @ by_name['v1'].view(experts, -1, case['hidden'])[e].t())
+        else:
+            h = F.gelu(z, approximate='tanh')
+        y = (h @ w2) * weights[token, slot].unsqueeze(1)
+        out = out + torch.zeros_like(rows).index_add(0, token, y)
+    if 'bias' in by_name:
+        out = out + by_name['bias']
+    out = out.view(x.shape)
+    if not train:
+        return out
+    aux = experts * 0.1 / (case['tokens'] * top_k) * torch.dot(counts.double(), scores.mean(0))
+    grads = torch.autograd.grad([out, aux], [x] + params, [state['dy'].double(), state['one'].double()])
+    return [out.detach(), aux.detach(), *grads]
+
+
+def _exact_gmm(case, state):
+    a, b = (state[n].detach().double().requires_grad_(True) for n in ('a', 'b'))
+    sizes = state['sizes'].tolist()
+    out = torch.cat([part @ (b[g].t() if case['trans_b'] else b[g]) for g, part in enumerate(a.split(sizes))])
+    return [out.detach(), *torch.autograd.grad(out, [a, b], state['dy'].double())]
+
+
+def _exact_sparse(case, state):
+    x, w1, w2 = (state[n].detach().double().requires_grad_(True) for n in ('x', 'w1', 'w2'))
+    topo = state['topo']
+    present = torch.zeros(case['rows'] // _BLOCK, case['cols'] // _BLOCK, device='cuda', dtype=torch.float64)
+    present[topo.row_indices.long(), topo.column_indices.long()] = 1
+    mask = present.repeat_interleave(_BLOCK, 0).repeat_interleave(_BLOCK, 1)
+    out = (F.gelu(x @ w1.t(), approximate='tanh') * mask) @ w2
+    return [out.detach(), *torch.autograd.grad(out, [x, w1, w2], state['dy'].double())]
+
+
+def exact(case, seed):
+    if case['kind'] == 'step':
+        return None
+    # The expert loop keeps one [tokens, hidden] array per expert for its backward pass.
+    if case['kind'] == 'layer' and 8 * case['tokens'] * case['hidden'] * case['experts'] > 40e9:
+        return None
+    return {'layer': _exact_layer, 'gmm': _exact_gmm, 'sparse': _exact_sparse}[case['kind']](case, prepare(case, seed))
