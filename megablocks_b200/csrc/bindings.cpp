@@ -20,7 +20,8 @@ at::Tensor gather_rows_op(const at::Tensor& x, const at::Tensor& indices, const 
                        const at::Tensor& padded_bins, int64_t top_k, int64_t out_rows);
 at::Tensor scatter_rows_op(const at::Tensor& x, const at::Tensor& indices, const at::Tensor& bin_ids,
                         const c10::optional<at::Tensor>& weights, const at::Tensor& bins,
-                        const at::Tensor& padded_bins, int64_t top_k, int64_t tokens);
+                        const at::Tensor& padded_bins, int64_t top_k, int64_t tokens,
+                        const c10::optional<at::Tensor>& bias);
 at::Tensor scatter_wgrad_op(const at::Tensor& x, const at::Tensor& grad, const at::Tensor& indices,
                          const at::Tensor& bin_ids, const at::Tensor& bins, const at::Tensor& padded_bins,
                          int64_t top_k);
@@ -29,7 +30,7 @@ at::Tensor binned_gather_rows(const at::Tensor& x, const at::Tensor& indices,
                               int64_t top_k);
 at::Tensor binned_scatter_rows(const at::Tensor& x, const at::Tensor& indices,
                                const c10::optional<at::Tensor>& weights, const at::Tensor& bins, int64_t top_k,
-                               int64_t tokens);
+                               int64_t tokens, const c10::optional<at::Tensor>& bias);
 at::Tensor binned_scatter_wgrad(const at::Tensor& x, const at::Tensor& grad, const at::Tensor& indices,
                                 const at::Tensor& bins, int64_t top_k);
 

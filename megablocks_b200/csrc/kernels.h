@@ -45,8 +45,8 @@ cudaError_t gather_rows(DType type, const void* x, const int* indices, const voi
 // capacity < 0: padded layout; capacity >= 0: binned layout [E, capacity].
 cudaError_t inverse_map(const int* indices, const int* bins, const int* padded_bins, int num_bins, int n,
                         int capacity, int* inverse_filled_minus_one, cudaStream_t stream);
-cudaError_t combine_rows(DType type, const void* x, const int* inverse, const void* weights, int top_k,
-                         int64_t tokens, int cols, void* out, cudaStream_t stream);
+cudaError_t combine_rows(DType type, const void* x, const int* inverse, const void* weights, const void* bias,
+                         int top_k, int64_t tokens, int cols, void* out, cudaStream_t stream);
 cudaError_t scatter_wgrad(DType type, const void* x, const void* grad, const int* inverse, int top_k,
                           int64_t copies, int cols, void* wgrad, cudaStream_t stream);
 

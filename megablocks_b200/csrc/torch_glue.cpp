@@ -265,11 +265,20 @@ at::Tensor gather_rows_op(const at::Tensor& x, const at::Tensor& indices, const 
   return out;
 }
 
+static void check_out_bias(const c10::optional<at::Tensor>& bias, const at::Tensor& x) {
+  if (!bias.has_value()) return;
+  TORCH_CHECK(bias->is_cuda() && bias->get_device() == x.get_device() && bias->is_contiguous() && bias->dim() == 1 &&
+                  bias->scalar_type() == x.scalar_type() && bias->numel() == x.size(-1),
+              "bias must be a contiguous vector of one value per column, of the rows' type");
+}
+
 at::Tensor scatter_rows_op(const at::Tensor& x, const at::Tensor& indices, const at::Tensor& bin_ids,
                            const c10::optional<at::Tensor>& weights, const at::Tensor& bins,
-                           const at::Tensor& padded_bins, int64_t top_k, int64_t tokens) {
+                           const at::Tensor& padded_bins, int64_t top_k, int64_t tokens,
+                           const c10::optional<at::Tensor>& bias) {
   MB_CHECK_CUDA(x); MB_CHECK_CONTIG(x);
   TORCH_CHECK(x.dim() == 2, "scatter expects x[rows, hidden]");
+  check_out_bias(bias, x);
   check_index(indices, "indices"); check_index(bins, "bins"); check_index(padded_bins, "padded_bins");
   check_weights(weights, x, indices.numel());
   (void)bin_ids;
@@ -278,7 +287,7 @@ at::Tensor scatter_rows_op(const at::Tensor& x, const at::Tensor& indices, const
   if (out.numel() == 0) return out;
   at::Tensor inverse = build_inverse(indices, bins, padded_bins, -1);
   MB_CUDA_OK(combine_rows(float_code(x.scalar_type()), x.data_ptr(), inverse.data_ptr<int>(), opt_ptr(weights),
-                          int(top_k), tokens, int(x.size(1)), out.data_ptr(), stream()));
+                          opt_ptr(bias), int(top_k), tokens, int(x.size(1)), out.data_ptr(), stream()));
   MB_LAUNCHED(1);
   return out;
 }
@@ -323,9 +332,10 @@ at::Tensor binned_gather_rows(const at::Tensor& x, const at::Tensor& indices,
 
 at::Tensor binned_scatter_rows(const at::Tensor& x, const at::Tensor& indices,
                                const c10::optional<at::Tensor>& weights, const at::Tensor& bins, int64_t top_k,
-                               int64_t tokens) {
+                               int64_t tokens, const c10::optional<at::Tensor>& bias) {
   MB_CHECK_CUDA(x); MB_CHECK_CONTIG(x);
   TORCH_CHECK(x.dim() == 3, "binned_scatter expects x[experts, capacity, hidden]");
+  check_out_bias(bias, x);
   check_index(indices, "indices"); check_index(bins, "bins");
   check_weights(weights, x, indices.numel());
   c10::cuda::CUDAGuard guard(x.device());
@@ -333,7 +343,7 @@ at::Tensor binned_scatter_rows(const at::Tensor& x, const at::Tensor& indices,
   if (out.numel() == 0) return out;
   at::Tensor inverse = build_inverse(indices, bins, bins, int(x.size(1)));
   MB_CUDA_OK(combine_rows(float_code(x.scalar_type()), x.data_ptr(), inverse.data_ptr<int>(), opt_ptr(weights),
-                          int(top_k), tokens, int(x.size(2)), out.data_ptr(), stream()));
+                          opt_ptr(bias), int(top_k), tokens, int(x.size(2)), out.data_ptr(), stream()));
   MB_LAUNCHED(1);
   return out;
 }

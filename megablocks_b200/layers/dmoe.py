@@ -86,7 +86,7 @@ class ParallelDroplessMLP(moe.ParallelMLP):
         return indices, bin_ids, bins, padded_bins, tokens_per_expert
 
     # -- block-sparse layout ---------------------------------------------------
-    def sparse_forward_once(self, x, expert_weights, top_experts):
+    def sparse_forward_once(self, x, expert_weights, top_experts, bias=None):
         expert_weights = expert_weights.flatten()
         top_experts = top_experts.flatten()
         with torch.no_grad():
@@ -97,7 +97,7 @@ class ParallelDroplessMLP(moe.ParallelMLP):
         with torch.no_grad():
             topo = self.topology(x, padded_bins)
         x = self.mlp(x, topo)
-        x = ops.padded_scatter(x, indices, bin_ids, expert_weights, bins, padded_bins, self.top_k)
+        x = ops.padded_scatter(x, indices, bin_ids, expert_weights, bins, padded_bins, self.top_k, bias)
         return x, tokens_per_expert
 
     def sparse_permute_and_compute(self, x, tokens_per_expert, indices, bin_ids, expert_weights, bins,
@@ -115,21 +115,22 @@ class ParallelDroplessMLP(moe.ParallelMLP):
         return ops.padded_scatter(x, indices, bin_ids, expert_weights, bins, padded_bins, top_k)
 
     # -- grouped layout --------------------------------------------------------
-    def grouped_forward_once(self, x, expert_weights, top_experts):
+    def grouped_forward_once(self, x, expert_weights, top_experts, bias=None):
         expert_weights = expert_weights.flatten()
         top_experts = top_experts.flatten()
         with torch.no_grad():
             indices, bin_ids, bins, tokens_per_expert = self.indices_and_bins(top_experts)
+        kw = {} if bias is None else dict(bias=bias)
         out = self.grouped_permute_and_compute(x, tokens_per_expert, indices, bin_ids, expert_weights, bins, -1,
-                                               self.top_k)
+                                               self.top_k, **kw)
         return out, tokens_per_expert
 
     def grouped_permute_and_compute(self, x, tokens_per_expert, indices, bin_ids, expert_weights, bins,
-                                    expert_capactiy, top_k):
+                                    expert_capactiy, top_k, bias=None):
         x = x.reshape(-1, x.shape[-1])
         x = ops.gather(x, indices, bin_ids, bins, top_k)
         x = self.mlp(x, tokens_per_expert, bins=bins)      # bins = prefix sum of tokens_per_expert
-        return ops.scatter(x, indices, bin_ids, expert_weights, bins, top_k)
+        return ops.scatter(x, indices, bin_ids, expert_weights, bins, top_k, bias)
 
     # -- expert parallel over peer memory ----------------------------------------
     def parallel_forward_once(self, x, expert_weights, top_experts):
@@ -146,10 +147,17 @@ class ParallelDroplessMLP(moe.ParallelMLP):
                                                 mlp._grouped_view(w2), v1, w1_kn=False, expert_capacity=0)
 
     # -- dispatch --------------------------------------------------------------
+    _bias_steps = ('forward_once', '_forward_once', 'sparse_forward_once', 'grouped_forward_once',
+                   'grouped_permute_and_compute')
+
     def forward_once(self, x, expert_weights, top_experts):
+        return self._forward_once(x, expert_weights, top_experts, None)
+
+    def _forward_once(self, x, expert_weights, top_experts, bias):
+        kw = {} if bias is None else dict(bias=bias)
         if self.args.mlp_impl == 'sparse':
-            return self.sparse_forward_once(x, expert_weights, top_experts)
-        return self.grouped_forward_once(x, expert_weights, top_experts)
+            return self.sparse_forward_once(x, expert_weights, top_experts, **kw)
+        return self.grouped_forward_once(x, expert_weights, top_experts, **kw)
 
     def permute_and_compute(self, x, tokens_per_expert, indices, bin_ids, expert_weights, bins, expert_capactiy,
                             top_k):
@@ -158,6 +166,9 @@ class ParallelDroplessMLP(moe.ParallelMLP):
                                                    expert_capactiy, top_k)
         return self.grouped_permute_and_compute(x, tokens_per_expert, indices, bin_ids, expert_weights, bins,
                                                 expert_capactiy, top_k)
+
+
+ParallelDroplessMLP._bias_base = ParallelDroplessMLP
 
 
 class _LazyTopology(sparse.Matrix):

@@ -128,15 +128,38 @@ class ParallelMLP(torch.nn.Module):
         indices, bin_ids, bins, _, tokens_per_expert = ops.route_plan(top_expert, self.num_experts)
         return indices, bin_ids, bins, tokens_per_expert
 
+    # -- output bias ----------------------------------------------------------
+    # Steps between `forward` and the un-permutation; a subclass that replaces one of them gets the
+    # bias added after it, as before.
+    _bias_steps = ('forward_once', '_forward_once', 'permute_and_compute')
+
+    def _unpermute_bias(self, x: torch.Tensor):
+        """The output bias if the un-permutation kernel can add it on its way out, else ``None``.
+
+        Only where the sum has the type of the activations (no autocast, no sharded parameter).
+        """
+        bias = self.bias
+        if (bias is None or self.args.return_bias or not x.is_cuda or bias.dtype != x.dtype
+                or x.dtype not in (torch.bfloat16, torch.float16, torch.float32) or not bias.is_contiguous()
+                or bias.device != x.device or hasattr(bias, 'to_local') or torch.is_autocast_enabled('cuda')):
+            return None
+        base, cls = self._bias_base, type(self)
+        stock = getattr(self.forward_fn, '__func__', None) is base.forward_once and all(
+            getattr(cls, name) is getattr(base, name) for name in base._bias_steps)
+        return bias if stock else None
+
     # -- single device --------------------------------------------------------
     def permute_and_compute(self, x, tokens_per_expert, indices, bin_ids, expert_weights, bins, expert_capacity,
-                            top_k):
+                            top_k, bias=None):
         x = x.reshape(-1, x.shape[-1])
         x = ops.binned_gather(x, indices, bins, expert_capacity, top_k)
         x = self.mlp(x)
-        return ops.binned_scatter(x, indices, expert_weights, bins, top_k)
+        return ops.binned_scatter(x, indices, expert_weights, bins, top_k, bias)
 
     def forward_once(self, x: torch.Tensor, expert_weights: torch.Tensor, top_experts: torch.Tensor):
+        return self._forward_once(x, expert_weights, top_experts, None)
+
+    def _forward_once(self, x, expert_weights, top_experts, bias):
         expert_weights = expert_weights.flatten()
         top_experts = top_experts.flatten()
         with torch.no_grad():
@@ -146,8 +169,9 @@ class ParallelMLP(torch.nn.Module):
             if capacity == 0:
                 # Dropless by padding: the output shape depends on the data.
                 capacity = int(torch.max(tokens_per_expert).item())
+        kw = {} if bias is None else dict(bias=bias)
         x = self.permute_and_compute(x, tokens_per_expert, indices, bin_ids, expert_weights, bins, capacity,
-                                     self.top_k)
+                                     self.top_k, **kw)
         return x, tokens_per_expert
 
     # -- expert parallel ------------------------------------------------------
@@ -295,16 +319,23 @@ class ParallelMLP(torch.nn.Module):
     def forward(self, x: torch.Tensor, scores: torch.Tensor, expert_weights: torch.Tensor,
                 top_experts: torch.Tensor):
         in_shape = x.size()
-        x, tokens_per_expert = self.forward_fn(x, expert_weights, top_experts)
+        fused_bias = self._unpermute_bias(x)
+        if fused_bias is not None:
+            x, tokens_per_expert = self._forward_once(x, expert_weights, top_experts, fused_bias)
+        else:
+            x, tokens_per_expert = self.forward_fn(x, expert_weights, top_experts)
         self.last_tokens_per_expert = tokens_per_expert      # device tensor, for load statistics in logs
         if self.training and self.args.moe_loss_weight > 0:
             save_load_balancing_loss((tokens_per_expert, scores))
         x = x.view(in_shape)
-        if self.bias is not None:
+        if self.bias is not None and fused_bias is None:
             if self.args.return_bias:
                 return x, self.bias
             return x + self.bias
         return x
+
+
+ParallelMLP._bias_base = ParallelMLP
 
 
 class MoE(torch.nn.Module):

@@ -71,16 +71,17 @@ def _gather_rows(x, indices, bin_ids, weights, bins, padded_bins, top_k, out_row
     return out
 
 
-def _scatter_rows(x, indices, bin_ids, weights, bins, padded_bins, top_k):
+def _scatter_rows(x, indices, bin_ids, weights, bins, padded_bins, top_k, bias=None):
     tokens = indices.numel() // top_k
     debug.check_routing(indices, bin_ids, bins, padded_bins, top_k, tokens, x.shape[0])
     if x.is_cuda:
-        return ext().scatter_rows(x, indices, bin_ids, weights, bins, padded_bins, top_k, tokens)
+        return ext().scatter_rows(x, indices, bin_ids, weights, bins, padded_bins, top_k, tokens, bias)
     copy_ids = indices.to(torch.int64)
     rows = _dest_rows(bin_ids, bins, padded_bins)
     tmp = x.new_zeros(tokens * top_k, x.shape[1])
     tmp[copy_ids] = _scaled(x[rows], weights, copy_ids, x.dtype)
-    return _sum_top_k(tmp, tokens, top_k)
+    out = _sum_top_k(tmp, tokens, top_k)
+    return out if bias is None else out + bias
 
 
 def _scatter_wgrad(x, grad, indices, bin_ids, bins, padded_bins, top_k):
@@ -93,6 +94,14 @@ def _scatter_wgrad(x, grad, indices, bin_ids, bins, padded_bins, top_k):
     out = torch.zeros(indices.numel(), dtype=x.dtype)
     out[copy_ids] = (x[rows].float() * grad[copy_ids // top_k].float()).sum(dim=1).to(x.dtype)
     return out
+
+
+def _bias_grad(grad: torch.Tensor) -> torch.Tensor:
+    """Column sums of ``grad[tokens, hidden]``, accumulated in fp32.  The column-sum kernel runs at memory
+    bandwidth; the library reduction takes 49 us for 32768 x 768 bf16 where it takes 12."""
+    if grad.is_cuda and (grad.shape[1] * grad.element_size()) % 16 == 0 and grad.data_ptr() % 16 == 0:
+        return ext().column_sum(grad)
+    return grad.sum(dim=0)
 
 
 def _check_routing(indices, bin_ids, bins, padded_bins=None):
@@ -132,7 +141,7 @@ class _Scatter(torch.autograd.Function):
     """Expert order -> token order with router weights and the top-k sum."""
 
     @staticmethod
-    def forward(ctx: Any, x, indices, bin_ids, weights, bins, padded_bins, top_k):
+    def forward(ctx: Any, x, indices, bin_ids, weights, bins, padded_bins, top_k, bias=None):
         x = _autocast(x)
         weights = _autocast(weights)
         need_wgrad = weights is not None and weights.requires_grad
@@ -146,7 +155,7 @@ class _Scatter(torch.autograd.Function):
         ctx.need_wgrad = need_wgrad
         ctx.top_k = top_k
         ctx.x_rows = x.shape[0]
-        return _scatter_rows(x.contiguous(), indices, bin_ids, weights, bins, padded_bins, top_k)
+        return _scatter_rows(x.contiguous(), indices, bin_ids, weights, bins, padded_bins, top_k, bias)
 
     @staticmethod
     def backward(ctx: Any, grad):
@@ -161,7 +170,8 @@ class _Scatter(torch.autograd.Function):
         if ctx.need_wgrad:
             x = saved[-1]
             dw = _scatter_wgrad(x, grad, indices, bin_ids, bins, padded_bins, ctx.top_k)
-        return dx, None, None, dw, None, None, None
+        db = _bias_grad(grad) if ctx.needs_input_grad[7] else None
+        return dx, None, None, dw, None, None, None, db
 
 
 def gather(x: torch.Tensor, indices: torch.Tensor, bin_ids: torch.Tensor, bins: torch.Tensor,
@@ -172,10 +182,13 @@ def gather(x: torch.Tensor, indices: torch.Tensor, bin_ids: torch.Tensor, bins: 
 
 
 def scatter(x: torch.Tensor, indices: torch.Tensor, bin_ids: torch.Tensor, weights: Optional[torch.Tensor],
-            bins: torch.Tensor, top_k: int) -> torch.Tensor:
-    """Inverse of :func:`gather` with optional per-copy weights; sums the ``top_k`` copies."""
+            bins: torch.Tensor, top_k: int, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Inverse of :func:`gather` with optional per-copy weights; sums the ``top_k`` copies.
+
+    ``bias`` (optional, ``[hidden]``, same type as ``x``) is added to every row of the result.
+    """
     _check_routing(indices, bin_ids, bins)
-    return _Scatter.apply(x, indices, bin_ids, weights, bins, bins, top_k)
+    return _Scatter.apply(x, indices, bin_ids, weights, bins, bins, top_k, bias)
 
 
 def padded_gather(x: torch.Tensor, indices: torch.Tensor, bin_ids: torch.Tensor, bins: torch.Tensor,
@@ -195,10 +208,10 @@ def padded_gather(x: torch.Tensor, indices: torch.Tensor, bin_ids: torch.Tensor,
 
 def padded_scatter(x: torch.Tensor, indices: torch.Tensor, bin_ids: torch.Tensor,
                    weights: Optional[torch.Tensor], bins: torch.Tensor, padded_bins: torch.Tensor,
-                   top_k: int) -> torch.Tensor:
-    """Inverse of :func:`padded_gather` with optional weights and the top-k sum."""
+                   top_k: int, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Inverse of :func:`padded_gather` with optional weights, the top-k sum and an optional bias."""
     _check_routing(indices, bin_ids, bins, padded_bins)
-    return _Scatter.apply(x, indices, bin_ids, weights, bins, padded_bins, top_k)
+    return _Scatter.apply(x, indices, bin_ids, weights, bins, padded_bins, top_k, bias)
 
 
 # ----------------------------------------------------------------------------
@@ -227,16 +240,17 @@ def _binned_gather_rows(x, indices, weights, bins, capacity, top_k):
     return out
 
 
-def _binned_scatter_rows(x, indices, weights, bins, top_k):
+def _binned_scatter_rows(x, indices, weights, bins, top_k, bias=None):
     tokens = indices.numel() // top_k
     if x.is_cuda:
-        return ext().binned_scatter_rows(x, indices, weights, bins, top_k, tokens)
+        return ext().binned_scatter_rows(x, indices, weights, bins, top_k, tokens, bias)
     capacity = x.shape[1]
     expert, slot, keep = _binned_slots(indices, bins, capacity)
     copy_ids = indices.to(torch.int64)[keep]
     tmp = x.new_zeros(tokens * top_k, x.shape[2])
     tmp[copy_ids] = _scaled(x[expert[keep], slot[keep]], weights, copy_ids, x.dtype)
-    return _sum_top_k(tmp, tokens, top_k)
+    out = _sum_top_k(tmp, tokens, top_k)
+    return out if bias is None else out + bias
 
 
 def _binned_scatter_wgrad(x, grad, indices, bins, top_k):
@@ -269,7 +283,7 @@ class _BinnedGather(torch.autograd.Function):
 class _BinnedScatter(torch.autograd.Function):
 
     @staticmethod
-    def forward(ctx: Any, x, indices, weights, bins, top_k):
+    def forward(ctx: Any, x, indices, weights, bins, top_k, bias=None):
         x = _autocast(x)
         weights = _autocast(weights)
         need_wgrad = weights is not None and weights.requires_grad
@@ -283,7 +297,7 @@ class _BinnedScatter(torch.autograd.Function):
         ctx.need_wgrad = need_wgrad
         ctx.top_k = top_k
         ctx.bin_size = x.shape[1]
-        return _binned_scatter_rows(x.contiguous(), indices, weights, bins, top_k)
+        return _binned_scatter_rows(x.contiguous(), indices, weights, bins, top_k, bias)
 
     @staticmethod
     def backward(ctx: Any, grad):
@@ -297,7 +311,8 @@ class _BinnedScatter(torch.autograd.Function):
         dw = None
         if ctx.need_wgrad:
             dw = _binned_scatter_wgrad(saved[-1], grad, indices, bins, ctx.top_k)
-        return dx, None, dw, None, None
+        db = _bias_grad(grad) if ctx.needs_input_grad[5] else None
+        return dx, None, dw, None, None, db
 
 
 def binned_gather(x: torch.Tensor, indices: torch.Tensor, bins: torch.Tensor, bin_size: int,
@@ -310,9 +325,10 @@ def binned_gather(x: torch.Tensor, indices: torch.Tensor, bins: torch.Tensor, bi
 
 
 def binned_scatter(x: torch.Tensor, indices: torch.Tensor, weights: Optional[torch.Tensor], bins: torch.Tensor,
-                   top_k: int) -> torch.Tensor:
-    """Inverse of :func:`binned_gather`; copies that were dropped contribute zero."""
+                   top_k: int, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Inverse of :func:`binned_gather`; copies that were dropped contribute zero.  ``bias`` (optional,
+    ``[hidden]``, same type as ``x``) is added to every row of the result."""
     _check_routing(indices, indices, bins)
     if x.dim() != 3 or x.shape[0] != bins.numel():
         raise ValueError('binned_scatter expects x[num_experts, bin_size, hidden]')
-    return _BinnedScatter.apply(x, indices, weights, bins, top_k)
+    return _BinnedScatter.apply(x, indices, weights, bins, top_k, bias)

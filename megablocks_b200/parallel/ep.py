@@ -267,7 +267,7 @@ class _FusedExpertParallel(torch.autograd.Function):
             if not fuse:
                 ws.return_rows(y, counts, 0, seq, done[1])
             ws.wait_return(0, seq)
-        out = ext().scatter_rows(ws.ret_y, indices, bin_ids, expert_weights, bins, bins, top_k, tokens)
+        out = ext().scatter_rows(ws.ret_y, indices, bin_ids, expert_weights, bins, bins, top_k, tokens, None)
         will_backward = torch.is_grad_enabled() and any(
             t is not None and t.requires_grad for t in (x, expert_weights, w1, w2, v1))
         if not will_backward:
@@ -329,7 +329,7 @@ class _FusedExpertParallel(torch.autograd.Function):
             ws.wait_return(1, seq)
         dx = None
         if needs[0]:
-            dx = ext().scatter_rows(ws.ret_dx, indices, bin_ids, None, bins, bins, top_k, ctx.tokens)
+            dx = ext().scatter_rows(ws.ret_dx, indices, bin_ids, None, bins, bins, top_k, ctx.tokens, None)
         return (dx, dweights, dw1, dw2, dv1) + (None,) * 11
 
 

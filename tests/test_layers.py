@@ -12,6 +12,7 @@ import torch.nn.functional as F
 from conftest import DEVICES
 
 import megablocks_b200 as mb
+from megablocks_b200 import ops
 from megablocks_b200.layers import moe as moe_mod
 from megablocks_b200.layers import router as router_mod
 from megablocks_b200.layers.arguments import from_megatron
@@ -280,3 +281,31 @@ def test_custom_activation_callable(device):
     torch.testing.assert_close(out.float(), ref, **_tol(device))
     out.float().sum().backward()
     assert layer.experts.mlp.w1.grad is not None
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize('top_k,hidden,dropped', [(1, 136, False), (3, 136, True), (1, 100, True), (2, 100, False)])
+def test_scatter_adds_the_output_bias(dtype, top_k, hidden, dropped):
+    """The bias of the un-permutation, its gradient and copies without a row, against the sum in fp32."""
+    torch.manual_seed(0)
+    tokens, experts = 77, 5
+    top = torch.randint(0, experts, (tokens * top_k,), device='cuda')
+    indices, bin_ids, bins, _, _ = ops.route_plan(top, experts)
+    bias = torch.randn(hidden, device='cuda').to(dtype).requires_grad_(True)
+    weights = torch.rand(tokens * top_k, device='cuda').to(dtype)
+    if dropped:
+        x = torch.randn(experts, 9, hidden, device='cuda').to(dtype)
+        call = lambda b: ops.binned_scatter(x, indices, weights, bins, top_k, b)
+    else:
+        x = torch.randn(tokens * top_k, hidden, device='cuda').to(dtype)
+        call = lambda b: ops.scatter(x, indices, bin_ids, weights, bins, top_k, b)
+    out = call(bias)
+    want = call(None).float() + bias.detach().float()
+    # One rounding instead of two: at most one unit of the type's last place of either term.
+    eps = torch.finfo(dtype).eps
+    assert torch.all((out.float() - want).abs() <= eps * (want.abs() + call(None).float().abs()) + 1e-6)
+    dy = torch.randn_like(out)
+    db, = torch.autograd.grad(out, bias, dy)
+    exact = dy.double().sum(0)
+    assert torch.all((db.double() - exact).abs() <= eps * exact.abs() + 1e-5 * dy.double().abs().sum(0))
