@@ -77,6 +77,40 @@ struct Config {
   static_assert(2 * kMaxGroups * 4 + kScatterBytes <= kStagingBytes, "large tables must fit the alternate staging area");
 };
 
+// Group tables of a launch, by one warp: row_end[g] = end of group g, forced to be non-decreasing and
+// inside the operand so that no tile can start or end outside it whatever `bins` holds, and (if wanted)
+// tile_end[g] = inclusive prefix sum of the groups' tiles of `tile_rows` rows.  Two shuffle scans per 32
+// groups: one thread walking 64 groups of shared memory cost each launch about 2 us.
+__device__ __forceinline__ void group_tables(const int* bins, int groups, int rows_total, int tile_rows, int* row_end,
+                                             int* tile_end, int lane) {
+  int carry_end = 0, carry_tiles = 0;
+  for (int base = 0; base < groups; base += 32) {
+    const int g = base + lane;
+    int end = g < groups ? __ldg(bins + g) : 0;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, end, d);
+      if (lane >= d) end = max(end, v);
+    }
+    end = min(max(end, carry_end), rows_total);
+    int prev = __shfl_up_sync(0xffffffffu, end, 1);
+    if (lane == 0) prev = carry_end;
+    int tiles = (end - prev + tile_rows - 1) / tile_rows;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, tiles, d);
+      if (lane >= d) tiles += v;
+    }
+    tiles += carry_tiles;
+    if (g < groups) {
+      row_end[g] = end;
+      if (tile_end != nullptr) tile_end[g] = tiles;
+    }
+    carry_end = __shfl_sync(0xffffffffu, end, 31);
+    carry_tiles = __shfl_sync(0xffffffffu, tiles, 31);
+  }
+}
+
 struct Tile {
   int group;
   int row0;        // NT / NN: first row of a and c; TN: first output row inside the group (m0)
@@ -281,13 +315,31 @@ __device__ __forceinline__ void stage_flip(Staging& st) {
   st.other = -st.other;
 }
 
-// This thread's row of the staging buffer, kept packed (16 registers for 32 values).
+// 32 values of the chunk as this thread holds them, packed (16 registers).  FRAG = false: the 32
+// columns of one row (tcgen05.ld 32x32b of an accumulator whose lanes are output rows).  FRAG = true:
+// the lanes are output COLUMNS and the accumulator is read with tcgen05.ld 16x256b; register pair w =
+// 8 h + 2 g + s then holds rows 8 g + 2 (lane % 4) + {0, 1} of column 16 h + 8 s + lane / 4, which is
+// the fragment that stmatrix / ldmatrix transpose on their way to and from the row-major staging
+// buffer.  Either way pairs of values are neighbours, so the arithmetic between is the same code.
 struct PackedRow {
   uint4 q[4];
 };
+// Address that this lane contributes to the transposing move of register group v (four 8 x 8 tiles).
+__device__ __forceinline__ uint32_t frag_offset(int lane, int v) {
+  return stage_offset(8 * ((v & 1) * 2 + (lane >> 4)) + (lane & 7), 2 * (v >> 1) + ((lane >> 3) & 1));
+}
+template <bool FRAG>
+__device__ __forceinline__ void stage_put(uint8_t* stage, int lane, int v, const uint4& w) {
+  if constexpr (FRAG) stmatrix_x4_trans(smem_u32(stage) + frag_offset(lane, v), w);
+  else *reinterpret_cast<uint4*>(stage + stage_offset(lane, v)) = w;
+}
+template <bool FRAG = false>
 __device__ __forceinline__ void stage_read_row(const uint8_t* stage, int lane, PackedRow& out) {
 #pragma unroll
-  for (int v = 0; v < 4; ++v) out.q[v] = *reinterpret_cast<const uint4*>(stage + stage_offset(lane, v));
+  for (int v = 0; v < 4; ++v) {
+    if constexpr (FRAG) out.q[v] = ldmatrix_x4_trans(smem_u32(stage) + frag_offset(lane, v));
+    else out.q[v] = *reinterpret_cast<const uint4*>(stage + stage_offset(lane, v));
+  }
 }
 // Two 16-bit values <-> one 32-bit word, without taking the address of a register.
 template <typename T>
@@ -377,7 +429,7 @@ __device__ __forceinline__ void dact_values(float acc, float z, float& dz, float
 
 // One pass over the chunk for the activation-backward epilogue: dz goes to the staging buffer as
 // it is produced, h waits packed in registers until the buffer is free again.
-template <typename T, int ACT, bool WANT_H>
+template <typename T, int ACT, bool WANT_H, bool FRAG>
 __device__ __forceinline__ void epilogue_emit_dact(const uint32_t (&raw)[32], const PackedRow& a1, Staging& stage,
                                                    T* out, T* out2, int64_t row_stride, int rows_ok, int cols,
                                                    int lane, int col, const CUtensorMap* maps, TmaOut tma) {
@@ -406,7 +458,7 @@ __device__ __forceinline__ void epilogue_emit_dact(const uint32_t (&raw)[32], co
       hw[v].x = pack2<T>(h[0], h[1]); hw[v].y = pack2<T>(h[2], h[3]);
       hw[v].z = pack2<T>(h[4], h[5]); hw[v].w = pack2<T>(h[6], h[7]);
     }
-    *reinterpret_cast<uint4*>(stage.buf + stage_offset(lane, v)) = w;
+    stage_put<FRAG>(stage.buf, lane, v, w);
   }
   if (tma.on) {
     fence_proxy_async_smem();
@@ -424,7 +476,7 @@ __device__ __forceinline__ void epilogue_emit_dact(const uint32_t (&raw)[32], co
   if constexpr (!WANT_H) return;
   if (maps != nullptr) stage_acquire(stage, lane);
 #pragma unroll
-  for (int v = 0; v < 4; ++v) *reinterpret_cast<uint4*>(stage.buf + stage_offset(lane, v)) = hw[v];
+  for (int v = 0; v < 4; ++v) stage_put<FRAG>(stage.buf, lane, v, hw[v]);
   if (tma.on) {
     fence_proxy_async_smem();
     __syncwarp();
@@ -458,7 +510,7 @@ __device__ __forceinline__ uint32_t epilogue_pair(const uint32_t (&raw)[32], con
 // Computes one output of the chunk, packs it eight columns at a time into this thread's
 // staging row and stores the chunk coalesced.  Only the accumulator row and the packed
 // auxiliary rows stay in registers.
-template <typename T, int EPI, int ACT, int WHICH>
+template <typename T, int EPI, int ACT, int WHICH, bool FRAG = false>
 __device__ __forceinline__ void epilogue_emit(const uint32_t (&raw)[32], const PackedRow& a1, const PackedRow& a2,
                                               Staging& stage, T* out, int64_t row_stride, int rows_ok, int cols,
                                               int lane, const ScatterRows<T>* scatter = nullptr, int col = 0,
@@ -471,7 +523,7 @@ __device__ __forceinline__ void epilogue_emit(const uint32_t (&raw)[32], const P
     w.y = epilogue_pair<T, EPI, ACT, WHICH>(raw, a1, a2, v * 8 + 2);
     w.z = epilogue_pair<T, EPI, ACT, WHICH>(raw, a1, a2, v * 8 + 4);
     w.w = epilogue_pair<T, EPI, ACT, WHICH>(raw, a1, a2, v * 8 + 6);
-    *reinterpret_cast<uint4*>(stage.buf + stage_offset(lane, v)) = w;
+    stage_put<FRAG>(stage.buf, lane, v, w);
   }
   if (tma.on) {
     // The staging layout is the 64-byte swizzle of a 32 x 32 box: one thread hands the chunk to
@@ -494,7 +546,7 @@ __device__ __forceinline__ void epilogue_emit(const uint32_t (&raw)[32], const P
 // Fused epilogue of one warp on a 32-row x 32-column chunk, specialised at compile time
 // on the epilogue kind and the activation.  `base_off` is the element offset of the
 // chunk's first row / first column in the output, `rows_ok` / `cols` its valid extent.
-template <typename T, int EPI, int ACT>
+template <typename T, int EPI, int ACT, bool FRAG>
 __device__ __forceinline__ void epilogue_chunk(const uint32_t (&raw)[32], const PackedRow& a1,
                                                const PackedRow& a2, Staging& stage, int64_t base_off,
                                                int64_t row_stride, int rows_ok, int cols, int lane,
@@ -505,57 +557,57 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&raw)[32], const 
     // Without the second output (the activation was kept by the forward pass) its arithmetic
     // is compiled out.
     if (p.out2)
-      epilogue_emit_dact<T, ACT, true>(raw, a1, stage, static_cast<T*>(p.c) + base_off,
+      epilogue_emit_dact<T, ACT, true, FRAG>(raw, a1, stage, static_cast<T*>(p.c) + base_off,
                                        static_cast<T*>(p.out2) + base_off, row_stride, rows_ok, cols, lane, col,
                                        maps, tma);
     else
-      epilogue_emit_dact<T, ACT, false>(raw, a1, stage, static_cast<T*>(p.c) + base_off, nullptr, row_stride,
+      epilogue_emit_dact<T, ACT, false, FRAG>(raw, a1, stage, static_cast<T*>(p.c) + base_off, nullptr, row_stride,
                                         rows_ok, cols, lane, col, maps, tma);
     return;
   }
-  epilogue_emit<T, EPI, ACT, 0>(raw, a1, a2, stage, static_cast<T*>(p.c) + base_off, row_stride, rows_ok, cols,
+  epilogue_emit<T, EPI, ACT, 0, FRAG>(raw, a1, a2, stage, static_cast<T*>(p.c) + base_off, row_stride, rows_ok, cols,
                                 lane, scatter, col, maps, tma);
   if constexpr (EPI == kEpiAct || EPI == kEpiDAct || EPI == kEpiGlu || EPI == kEpiDGlu) {
     if (p.out2)
-      epilogue_emit<T, EPI, ACT, 1>(raw, a1, a2, stage, static_cast<T*>(p.out2) + base_off, row_stride, rows_ok,
+      epilogue_emit<T, EPI, ACT, 1, FRAG>(raw, a1, a2, stage, static_cast<T*>(p.out2) + base_off, row_stride, rows_ok,
                                     cols, lane, nullptr, col, maps ? maps + 1 : nullptr, tma);
   }
   if constexpr (EPI == kEpiDGlu) {
     if (p.out3)
-      epilogue_emit<T, EPI, ACT, 2>(raw, a1, a2, stage, static_cast<T*>(p.out3) + base_off, row_stride, rows_ok,
+      epilogue_emit<T, EPI, ACT, 2, FRAG>(raw, a1, a2, stage, static_cast<T*>(p.out3) + base_off, row_stride, rows_ok,
                                     cols, lane, nullptr, col, maps ? maps + 2 : nullptr, tma);
   }
 }
 
-template <typename T, int EPI>
+template <typename T, int EPI, bool FRAG = false>
 __device__ __forceinline__ void epilogue_by_act(const uint32_t (&raw)[32], const PackedRow& a1,
                                                 const PackedRow& a2, Staging& stage, int64_t base_off,
                                                 int64_t row_stride, int rows_ok, int cols, int lane,
                                                 const GemmParams& p, const ScatterRows<T>* scatter, int col,
                                                 TmaOut tma) {
   switch (p.act) {
-    case kActGeluTanh: epilogue_chunk<T, EPI, kActGeluTanh>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
-    case kActSilu: epilogue_chunk<T, EPI, kActSilu>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
-    case kActRelu: epilogue_chunk<T, EPI, kActRelu>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
-    case kActGeluErf: epilogue_chunk<T, EPI, kActGeluErf>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
-    default: epilogue_chunk<T, EPI, kActIdentity>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
+    case kActGeluTanh: epilogue_chunk<T, EPI, kActGeluTanh, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
+    case kActSilu: epilogue_chunk<T, EPI, kActSilu, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
+    case kActRelu: epilogue_chunk<T, EPI, kActRelu, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
+    case kActGeluErf: epilogue_chunk<T, EPI, kActGeluErf, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
+    default: epilogue_chunk<T, EPI, kActIdentity, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
   }
 }
 
 // One dispatch per 32-column chunk (uniform across the warp); straight-line code inside.
-template <typename T>
+template <typename T, bool FRAG = false>
 __device__ __forceinline__ void epilogue_dispatch(const uint32_t (&raw)[32], const PackedRow& a1,
                                                   const PackedRow& a2, Staging& stage, int64_t base_off,
                                                   int64_t row_stride, int rows_ok, int cols, int lane,
                                                   const GemmParams& p, const ScatterRows<T>* scatter = nullptr,
                                                   int col = 0, TmaOut tma = TmaOut{false, 0}) {
   switch (p.epilogue) {
-    case kEpiNone: epilogue_chunk<T, kEpiNone, kActIdentity>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
-    case kEpiAdd: epilogue_chunk<T, kEpiAdd, kActIdentity>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
-    case kEpiAct: epilogue_by_act<T, kEpiAct>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
-    case kEpiDAct: epilogue_by_act<T, kEpiDAct>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
-    case kEpiGlu: epilogue_by_act<T, kEpiGlu>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
-    case kEpiDGlu: epilogue_by_act<T, kEpiDGlu>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
+    case kEpiNone: epilogue_chunk<T, kEpiNone, kActIdentity, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
+    case kEpiAdd: epilogue_chunk<T, kEpiAdd, kActIdentity, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
+    case kEpiAct: epilogue_by_act<T, kEpiAct, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
+    case kEpiDAct: epilogue_by_act<T, kEpiDAct, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
+    case kEpiGlu: epilogue_by_act<T, kEpiGlu, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
+    case kEpiDGlu: epilogue_by_act<T, kEpiDGlu, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
     default: break;
   }
 }
@@ -621,7 +673,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   const int G = p.num_groups;
 
   // ---- one-time setup ---------------------------------------------------------
-  for (int g = threadIdx.x; g < G; g += kThreads) s_row_end[g] = __ldg(p.bins + g);
+  if (warp == 0) group_tables(p.bins, G, p.rows_total, kBlockM, s_row_end, LAYOUT != kTN ? s_mblk_end : nullptr, lane);
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     // A launch that takes part in the expert-parallel exchange does nothing once a failure has
@@ -643,20 +695,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   if (warp == kMmaWarp) tmem_alloc(smem_u32(tmem_base_slot), Cfg::kTmemCols);
   __syncthreads();
   const bool dead = *dead_flag != 0;
-  if (threadIdx.x == 0) {
-    // Group ends are forced to be non-decreasing and inside the operand, so no tile can start or
-    // end outside a or c whatever `bins` holds.
-    int acc = 0, prev = 0;
-    for (int g = 0; g < G; ++g) {
-      const int end = min(max(s_row_end[g], prev), p.rows_total);
-      s_row_end[g] = end;
-      if (LAYOUT != kTN) {
-        acc += (end - prev + kBlockM - 1) / kBlockM;
-        s_mblk_end[g] = acc;
-      }
-      prev = end;
-    }
-  }
   if (scatter_on && !dead) {
     const int W = p.scatter_world, E = p.scatter_experts, epr = G;
     if (threadIdx.x == 0) {

@@ -264,6 +264,7 @@ struct GemmParams {
   int band_n;      // NT / NN: column tiles per band of the tile walk (0 = the kernel's default)
   CUtensorMap a2_map;
   CUtensorMap b2_map;
+  CUtensorMap aux_map[2];   // CTA pairs: aux1 / aux2 viewed like the outputs
   // Nullable device counter added to wait_seq and scatter_seq (see EpLayout::seq_base).
   const int* seq_base;
   // TN only, nullable: one fp32 accumulator in device memory that receives the sum of squares of

@@ -170,6 +170,30 @@ __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32])
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// 16 lanes x 32 consecutive fp32 columns in the fragment layout of an 8 x 8 matrix move: registers
+// 4 g + 2 s + e hold lane 8 s + i / 4, column 8 g + 2 (i % 4) + e of thread i.
+__device__ __forceinline__ void tmem_ld_16x256_x4(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+// Four 8 x 8 matrices of 16-bit values to / from shared memory, transposed; lane i addresses row i % 8 of
+// matrix i / 8.
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, const uint4& w) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};"
+               ::"r"(addr), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w) : "memory");
+}
+__device__ __forceinline__ uint4 ldmatrix_x4_trans(uint32_t addr) {
+  uint4 w;
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "r"(addr) : "memory");
+  return w;
+}
+
 // ---- CTA pairs (cta_group::2) -------------------------------------------------
 // Two CTAs of a cluster work on one 256-row tile: each loads its own 128 rows of A and
 // half of B, the even CTA issues the MMAs, each CTA's tensor memory receives its rows.
@@ -191,6 +215,11 @@ __device__ __forceinline__ void cluster_sync_all() {
 // Arrive on an mbarrier that lives in another CTA of the cluster.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// The same without cluster-scope release: for handing an accumulator stage back, which orders nothing
+// but tensor-memory reads (those by tcgen05.fence).  The release waits for this thread's stores.
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // Tile load whose completion bytes are counted on a barrier of either CTA of the pair
 // (`bar` is a shared::cluster address).  Every CTA fetches its own tile.
@@ -220,10 +249,11 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t a_desc, 
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Arrive on one barrier (a shared::cluster address, so it may live in either CTA of the pair)
-// once the MMAs issued so far retire.  The issuing thread calls it once per CTA to notify.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr)
+// Arrive on the barrier at this shared-memory offset in BOTH CTAs of the pair once the MMAs issued so
+// far retire.  (One commit per CTA instead costs the tensor pipe 6 to 14 % of its cycles.)
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(bar), "h"(static_cast<uint16_t>(3))
                : "memory");
 }
 

@@ -410,6 +410,7 @@ at::Tensor router_topk_backward(const at::Tensor& scores, const at::Tensor& weig
 namespace {
 
 constexpr int64_t kMaxScatterSegmentsHost = 512;   // = kMaxScatterSegments of the kernel
+constexpr int64_t kSmallGroupsHost = 224;          // = kSmallGroups of the kernels
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -560,9 +561,9 @@ std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, c
   p.alpha = float(alpha);
   p.seq_base = seq_base_ptr(seq_base);
   if (sqnorm.has_value()) {
-    TORCH_CHECK(layout == kTN && pair_mode != 1 && sqnorm->is_cuda() && sqnorm->scalar_type() == at::kFloat &&
+    TORCH_CHECK(layout == kTN && sqnorm->is_cuda() && sqnorm->scalar_type() == at::kFloat &&
                     sqnorm->numel() >= 1,
-                "sqnorm: a CUDA float32 accumulator, weight-gradient (TN) launches of the single-CTA kernel only");
+                "sqnorm: a CUDA float32 accumulator, weight-gradient (TN) launches only");
     p.sqnorm = sqnorm->data_ptr<float>();
   }
   if (epilogue == kEpiDAct || epilogue == kEpiGlu || epilogue == kEpiDGlu || epilogue == kEpiAdd) {
@@ -584,7 +585,7 @@ std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, c
   const bool dual = epilogue == kEpiGluDual;
   const bool concat = a2.has_value();
   if (dual) {
-    TORCH_CHECK(layout == kNT && b2.has_value() && !a2.has_value() && !scatter.has_value() && p.N >= 128 && pair_mode != 1,
+    TORCH_CHECK(layout == kNT && b2.has_value() && !a2.has_value() && !scatter.has_value() && p.N >= 128,
                 "the dual-B GLU epilogue needs the NT layout, a second weight tensor and at least 128 output columns");
     TORCH_CHECK(b2->is_cuda() && b2->is_contiguous() && b2->sizes() == b.sizes() && b2->scalar_type() == b.scalar_type(),
                 "b2 must match b");
@@ -662,14 +663,28 @@ std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, c
   if (out_numel == 0) return {c, out2, out3};
 
   const int block_n = (p.N >= 256 || dual) ? 256 : (p.N >= 128 ? 128 : 64);
-  // CTA pairs (cta_group::2, 256-row tiles, six 32 KB stages per CTA) pull a third less operand
-  // traffic through L2, but measured back to back against the single-CTA kernel (alternating
-  // launches, L2 flushed, medians) they are 0-8 % slower on every shape tried, from 64 ragged groups
-  // of 512 rows to 8 groups of 4096 rows with a 14336-deep contraction, in all three layouts.  They
-  // are therefore only taken on request.  pair_mode: 1 = whenever the kernel supports the problem,
-  // anything else = never.
+  // CTA pairs (cta_group::2) take every problem that fills their 256 output columns; what waits for or
+  // stores to peers, and more groups than their small tables hold, stays on the single-CTA kernel.
+  // pair_mode: 1 = whenever supported, 0 = never, anything else = the rule.
   (void)rows_hint;
-  const bool pair = pair_mode == 1 && block_n == 256 && sm_count() >= 2 && !scatter.has_value() && !dual && !concat;
+  //
+  // Rule: pairs, except where a launch only streams weights - at most 16 rows a group, and enough column
+  // tiles to give half of the SMs one.  There the single-CTA kernel keeps more weight bytes in flight per
+  // SM (128 KB against 80): 32 rows over 8 groups of 14336 x 4096, NN 159 us against 178, NT 191 against
+  // 194.  With fewer tiles the pairs' halved tile width wins: 8 rows over 64 groups of 3072 x 768, NN 34
+  // us against 26.  With more rows pairs win or draw on every shape measured (TFLOP/s sustained, single |
+  // pair): 8192 x 4096 x 14336, 8 groups, NT + GELU 1013 | 1053, GELU-bwd 988 | 1035, GLU-bwd 860 | 936,
+  // NN 985 | 1017, TN 980 | 1073; 32768 x 768 x 3072, 64 groups: 645 | 731, 535 | 658, 322 | 479,
+  // 824 | 821, 750 | 779; 10006 x 1024 x 4096, 32 groups: 625 | 692, 543 | 641, 349 | 511, 717 | 763,
+  // 588 | 635.
+  const bool streams_weights = layout != kTN && a.size(0) <= 16 * num_groups &&
+                               (1 + std::min<int64_t>(num_groups, a.size(0))) * ceil_div(p.N, 256) >= sm_count() / 2;
+  bool pair_ok = block_n == 256 && !dual && p.N >= 256 && sm_count() >= 2 && !scatter.has_value() &&
+                 !wait_flags.has_value() && num_groups <= kSmallGroupsHost &&
+                 (layout != kTN || epilogue == kEpiNone) && pair_mode != 0;
+  if (pair_ok && p.aux1) pair_ok = make_output_map(&p.aux_map[0], p.aux1, bf16, out_numel / p.N, p.N);
+  if (pair_ok && p.aux2) pair_ok = make_output_map(&p.aux_map[1], p.aux2, bf16, out_numel / p.N, p.N);
+  const bool pair = pair_ok && (pair_mode == 1 || !streams_weights);
   if (!scatter.has_value() && store_tma_enabled()) {
     // Full 32-row quarters of a tile leave through the TMA unit (one instruction per chunk).
     const int64_t out_rows = out_numel / p.N;
@@ -687,10 +702,19 @@ std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, c
       tb = make_tensor_map(b.data_ptr(), bf16, b.size(0), p.N, 64);
       tiles_bound = num_groups * ceil_div(p.M, 2 * kBlockM) * num_nb;
     } else {
-      ta = make_tensor_map(a.data_ptr(), bf16, a.size(0), p.K, kBlockM);
-      tb = layout == kNT ? make_tensor_map(b.data_ptr(), bf16, num_groups * p.N, p.K, block_n / 2)
-                         : make_tensor_map(b.data_ptr(), bf16, num_groups * p.K, p.N, 64);
-      tiles_bound = (ceil_div(a.size(0), 2 * kBlockM) + num_groups) * num_nb;
+      // Weights in 128-row (K-major) or 64-row (MN-major) boxes, tokens in 64-row boxes.
+      auto weights_map = [&](const at::Tensor& w) {
+        return layout == kNT ? make_tensor_map(w.data_ptr(), bf16, num_groups * p.N, p.K, kBlockM)
+                             : make_tensor_map(w.data_ptr(), bf16, num_groups * p.K, p.N, 64);
+      };
+      ta = make_tensor_map(a.data_ptr(), bf16, a.size(0), p.K, 64);
+      tb = weights_map(b);
+      if (concat) {
+        p.a2_map = make_tensor_map(a2->data_ptr(), bf16, a2->size(0), p.K, 64);
+        p.b2_map = weights_map(*b2);
+        p.k_concat = 1;
+      }
+      tiles_bound = (ceil_div(a.size(0), 256) + std::min<int64_t>(num_groups, a.size(0))) * num_nb;
     }
     const int pairs = int(std::max<int64_t>(1, std::min<int64_t>(tiles_bound, sm_count() / 2)));
     MB_CUDA_OK(launch(bf16, layout, block_n, ta, tb, p, 2 * pairs, stream(), true));

@@ -56,10 +56,9 @@ _ACT_NAMES = {
 }
 
 
-# CTA-pair (cta_group::2) kernel selection: 1 = whenever supported, anything else = never (the
-# default: measured against the single-CTA kernel it does not win on any shape tried).  Overridable
-# for experiments with MB200_GEMM_PAIR or per call (`pair=`).
-_PAIR_MODE = int(os.environ.get('MB200_GEMM_PAIR', '0'))
+# CTA-pair (cta_group::2) kernel selection: 1 = whenever supported, 0 = never, -1 (the default) = by the
+# rule beside the launch.  Overridable for experiments with MB200_GEMM_PAIR or per call (`pair=`).
+_PAIR_MODE = int(os.environ.get('MB200_GEMM_PAIR', '-1'))
 
 
 def activation_id(fn: Optional[Callable]) -> Optional[int]:
@@ -247,8 +246,8 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, bins: torch.Tensor, *, trans_
     ``(a b2^T, act(a b^T) * (a b2^T), a b^T)``.  ``a2`` and ``b2`` without ``trans_b``: the contraction
     runs over ``a x b`` and then ``a2 x b2`` into one accumulator, ``c = a b + a2 b2`` (the GLU input
     gradient in one launch).
-    ``pair`` overrides the kernel choice for this call: 1 = CTA pairs (``cta_group::2``, 256-row
-    tiles) whenever the problem allows, 0 = single-CTA kernel, ``None`` = the module default.
+    ``pair`` overrides the kernel choice for this call: 1 = CTA pairs (``cta_group::2``)
+    whenever the problem allows, 0 = single-CTA kernel, ``None`` = the module default.
     ``grad_norm`` (with ``trans_a``): the output is a weight gradient; if a :class:`GradNormSink` is
     installed the epilogue also adds the output's sum of squares to a slot of the sink.
     """
@@ -262,7 +261,7 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, bins: torch.Tensor, *, trans_
             scatter[2] if scatter is not None and len(scatter) > 2 else None)
         pair_mode = _PAIR_MODE if pair is None else int(pair)
         sink, slot, slot_view = _GRAD_NORM_SINK, None, None
-        if grad_norm and sink is not None and trans_a and pair_mode != 1:
+        if grad_norm and sink is not None and trans_a:
             slot, slot_view = sink._next()
         outs = ext().grouped_gemm(a, b, bins, bool(trans_a), bool(trans_b), int(epilogue), int(act), aux1, aux2,
                                   bool(want_out2), bool(want_out3), int(num_groups), c, bool(zero_tail), flags,

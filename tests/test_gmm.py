@@ -341,3 +341,68 @@ def test_weight_gradient_launch_reports_its_squared_norm(z, rows, m, n):
         want = float(out.float().square().sum())
         assert abs(float(got[slot]) - want) <= 4e-3 * want       # fp32 values before their rounding to bf16
     assert float(got[2:].abs().sum()) == 0.0
+
+
+def _pair_case(counts, k, n, trans_b, dtype, tail=0):
+    torch.manual_seed(sum(counts) + k + n)
+    z, m = len(counts), sum(counts)
+    bins = torch.cumsum(torch.tensor(counts), 0).int().cuda()
+    a = (torch.randn(m + tail, k) * 0.5).to(dtype).cuda()
+    b = (torch.randn(z, n, k) if trans_b else torch.randn(z, k, n)).mul(0.1).to(dtype).cuda()
+    return a, b, bins
+
+
+_PAIR_COUNTS = [[1], [16], [17], [31, 33], [255, 256, 257], [0, 511, 0, 513, 15, 0], [300, 1, 0, 7, 272, 1025]]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('counts', _PAIR_COUNTS)
+@pytest.mark.parametrize('k,n,trans_b', [(72, 264, True), (256, 512, True), (200, 264, False), (320, 768, False)])
+@pytest.mark.parametrize('epilogue', ['none', 'act', 'dact', 'glu', 'dglu', 'add'])
+def test_cta_pair_tiles_and_epilogues(counts, k, n, trans_b, epilogue):
+    """Token tiles of every share (1 to 256 rows, remainders of the 16 / 32 / 64-row steps), column and
+    contraction remainders, rows past the last group, and the transposed epilogue, against the CPU
+    statements of the op (fp32 products)."""
+    from megablocks_b200.utils import status
+    dtype = torch.bfloat16 if n != 512 else torch.float16
+    epi = getattr(G, 'EPI_' + epilogue.upper())
+    a, b, bins = _pair_case(counts, k, n, trans_b, dtype, tail=5)
+    aux1, aux2 = (torch.randn(a.shape[0], n).to(dtype).cuda() for _ in range(2))
+    kw = dict(trans_b=trans_b, epilogue=epi, act=G.ACT_SILU if 'glu' in epilogue else G.ACT_GELU_TANH, alpha=0.5)
+    got = G.grouped_gemm(a, b, bins, aux1=aux1, aux2=aux2, pair=1, **kw)
+    want = G.grouped_gemm(a.cpu(), b.cpu(), bins.cpu(), aux1=aux1.cpu(), aux2=aux2.cpu(), **kw)
+    status.check()
+    for g, w in zip(got, want):
+        if g is not None:
+            _close(g, w.float(), dtype)
+            assert not g[sum(counts):].any()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('counts', _PAIR_COUNTS)
+@pytest.mark.parametrize('k,n', [(72, 264), (256, 512)])
+def test_cta_pair_concatenated_contraction(counts, k, n):
+    """a x b + a2 x b2 in one accumulator, with a remainder in the first contraction."""
+    from megablocks_b200.utils import status
+    a, c, bins = _pair_case(counts, k, n, False, torch.bfloat16, tail=3)
+    a2, c2 = torch.randn_like(a), torch.randn_like(c) * 0.1
+    got, _, _ = G.grouped_gemm(a, c, bins, a2=a2, b2=c2, pair=1)
+    want, _, _ = G.grouped_gemm(a.cpu(), c.cpu(), bins.cpu(), a2=a2.cpu(), b2=c2.cpu())
+    status.check()
+    _close(got, want.float(), torch.bfloat16)
+
+
+@pytest.mark.gpu
+def test_cta_pair_gradient_norm():
+    """The squared norm taken in the weight-gradient epilogue, with a column remainder and an empty group."""
+    a, _, bins = _pair_case([100, 0, 300], 264, 264, True, torch.bfloat16)
+    dy = torch.randn(a.shape[0], 320, device='cuda').bfloat16()
+    sink = G.GradNormSink(a.device)
+    G.set_grad_norm_sink(sink)
+    try:
+        out, _, _ = G.grouped_gemm(a, dy, bins, trans_a=True, num_groups=3, grad_norm=True, pair=1)
+    finally:
+        G.set_grad_norm_sink(None)
+    # The sum is over the fp32 values before their rounding to 16 bits (2^-9 each, random sign).
+    want = float(out.double().square().sum())
+    assert abs(float(sink.slots[sink.lookup(out)]) - want) <= 1e-3 * want
