@@ -22,6 +22,9 @@ at::Tensor scatter_rows_op(const at::Tensor& x, const at::Tensor& indices, const
                         const c10::optional<at::Tensor>& weights, const at::Tensor& bins,
                         const at::Tensor& padded_bins, int64_t top_k, int64_t tokens,
                         const c10::optional<at::Tensor>& bias);
+std::vector<at::Tensor> scatter_backward_op(const at::Tensor& x, const at::Tensor& grad, const at::Tensor& indices,
+                                            const at::Tensor& weights, const at::Tensor& bins,
+                                            const c10::optional<at::Tensor>& padded_bins, int64_t top_k);
 at::Tensor scatter_wgrad_op(const at::Tensor& x, const at::Tensor& grad, const at::Tensor& indices,
                          const at::Tensor& bin_ids, const at::Tensor& bins, const at::Tensor& padded_bins,
                          int64_t top_k);
@@ -133,6 +136,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("replicate_backward", &mb::replicate_backward);
   m.def("gather_rows", &mb::gather_rows_op);
   m.def("scatter_rows", &mb::scatter_rows_op);
+  m.def("scatter_backward", &mb::scatter_backward_op);
   m.def("scatter_wgrad", &mb::scatter_wgrad_op);
   m.def("binned_gather_rows", &mb::binned_gather_rows);
   m.def("binned_scatter_rows", &mb::binned_scatter_rows);

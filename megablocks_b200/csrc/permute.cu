@@ -42,30 +42,40 @@ __device__ __forceinline__ void store_pack(T* p, const Pack<T, VEC>& in) {
   }
 }
 
-// out[r] for every row r of the expert-ordered buffer:
-//   e = group of r in padded_bins, off = r - padded_start(e);
-//   off < count(e): x[indices[start(e) + off] / top_k] (* weight), else zero.
+// Copy held by row r of the expert-ordered buffer, or -1 for a pad row: e = group of r in padded_bins
+// (capacity < 0) or r / capacity, off = r - first row of the group, indices[start(e) + off] if
+// off < count(e).
+__device__ __forceinline__ int copy_of_row(int64_t r, const int* __restrict__ indices, const int* __restrict__ bins,
+                                           const int* __restrict__ padded_bins, int num_bins, int capacity) {
+  int e, pstart = 0;
+  if (capacity >= 0) {
+    e = static_cast<int>(r / capacity);
+    pstart = e * capacity;
+  } else {
+    e = upper_bound_i32(padded_bins, num_bins, static_cast<int>(r));
+    if (e < num_bins && e > 0) pstart = __ldg(padded_bins + e - 1);
+  }
+  if (e >= num_bins) return -1;
+  const int start = e ? __ldg(bins + e - 1) : 0;
+  const int off = static_cast<int>(r) - pstart;
+  return off < __ldg(bins + e) - start ? __ldg(indices + start + off) : -1;
+}
+
+// out[r] = x[copy / top_k] (* weight[copy]) for every row r of the expert-ordered buffer, zero for pad rows.
 template <typename T, int VEC>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 gather_rows_kernel(const T* __restrict__ x, const int* __restrict__ indices, const T* __restrict__ weights, const int* __restrict__ bins,
-                   const int* __restrict__ padded_bins, int num_bins, int top_k, int64_t out_rows, int cols,
+                   const int* __restrict__ padded_bins, int num_bins, int capacity, int top_k, int64_t out_rows, int cols,
                    T* __restrict__ out) {
   const int lane = threadIdx.x & 31;
   const int64_t r = int64_t(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
   if (r >= out_rows) return;
   int src_token = -1;
   float scale = 1.f;
-  const int e = upper_bound_i32(padded_bins, num_bins, static_cast<int>(r));
-  if (e < num_bins) {
-    const int pstart = e ? __ldg(padded_bins + e - 1) : 0;
-    const int start = e ? __ldg(bins + e - 1) : 0;
-    const int count = __ldg(bins + e) - start;
-    const int off = static_cast<int>(r) - pstart;
-    if (off < count) {
-      const int copy = __ldg(indices + start + off);
-      src_token = copy / top_k;
-      if (weights != nullptr) scale = to_float(weights[copy]);
-    }
+  const int copy = copy_of_row(r, indices, bins, padded_bins, num_bins, capacity);
+  if (copy >= 0) {
+    src_token = copy / top_k;
+    if (weights != nullptr) scale = to_float(weights[copy]);
   }
   T* dst = out + r * cols;
   if (src_token < 0) {
@@ -215,6 +225,63 @@ wgrad_kernel(const T* __restrict__ x, const T* __restrict__ grad, const int* __r
   if (lane == 0) wgrad[copy] = from_float<T>(acc);
 }
 
+// Backward of the weighted un-permutation in one pass over the expert-ordered rows: for row r with
+// copy c of token t, dx[r] = weight[c] * grad[t] and dweight[c] = <x[r], grad[t]>; pad rows of dx are
+// zero.  Bound by memory: as two kernels (the gather above and wgrad_kernel) grad is read twice and an
+// inverse index map is built in between.  One warp per row, two 16-byte loads of each operand in
+// flight per lane.  dweight entries of copies without a row are cleared by the launcher.
+template <typename T, int VEC>
+__global__ void __launch_bounds__(kWarpsPerCta * 32)
+scatter_bwd_kernel(const T* __restrict__ x, const T* __restrict__ grad, const int* __restrict__ indices,
+                   const T* __restrict__ weights, const int* __restrict__ bins, const int* __restrict__ padded_bins,
+                   int num_bins, int capacity, int top_k, int64_t out_rows, int cols, T* __restrict__ dx,
+                   T* __restrict__ dweights) {
+  const int lane = threadIdx.x & 31;
+  const int64_t r = int64_t(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
+  if (r >= out_rows) return;
+  const int copy = copy_of_row(r, indices, bins, padded_bins, num_bins, capacity);
+  T* dst = dx + r * cols;
+  if (copy < 0) {
+    Pack<T, VEC> z;
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) z.v[i] = from_float<T>(0.f);
+    for (int c = lane * VEC; c < cols; c += 32 * VEC) store_pack<T, VEC>(dst + c, z);
+    return;
+  }
+  const float w = to_float(weights[copy]);
+  const T* g = grad + int64_t(copy / top_k) * cols;
+  const T* row = x + r * cols;
+  float acc[2] = {0.f, 0.f};
+  for (int c0 = lane * VEC; c0 < cols; c0 += 2 * 32 * VEC) {
+    Pack<T, VEC> pg[2], px[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int c = c0 + j * 32 * VEC;
+      if (c < cols) {
+        pg[j] = load_pack<T, VEC>(g + c);
+        px[j] = load_pack<T, VEC>(row + c);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int c = c0 + j * 32 * VEC;
+      if (c < cols) {
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) {
+          const float gv = to_float(pg[j].v[i]);
+          acc[j] = fmaf(to_float(px[j].v[i]), gv, acc[j]);
+          pg[j].v[i] = from_float<T>(gv * w);
+        }
+        store_pack<T, VEC>(dst + c, pg[j]);
+      }
+    }
+  }
+  float dot = acc[0] + acc[1];
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, d);
+  if (lane == 0) dweights[copy] = from_float<T>(dot);
+}
+
 template <typename T>
 int vec_width(int64_t cols, const void* a, const void* b) {
   constexpr int full = 16 / sizeof(T);
@@ -225,19 +292,19 @@ int vec_width(int64_t cols, const void* a, const void* b) {
 }  // namespace
 
 cudaError_t gather_rows(DType type, const void* x, const int* indices, const void* weights, const int* bins,
-                        const int* padded_bins, int num_bins, int top_k, int64_t out_rows, int cols, void* out,
-                        cudaStream_t stream) {
+                        const int* padded_bins, int num_bins, int capacity, int top_k, int64_t out_rows, int cols,
+                        void* out, cudaStream_t stream) {
   const int grid = ceil_div(out_rows, kWarpsPerCta);
   MB_SWITCH_FLOAT(type, T, {
     constexpr int kFull = 16 / sizeof(T);
     if (vec_width<T>(cols, x, out) > 1) {
       gather_rows_kernel<T, kFull><<<grid, kWarpsPerCta * 32, 0, stream>>>(
-          static_cast<const T*>(x), indices, static_cast<const T*>(weights), bins, padded_bins, num_bins, top_k,
-          out_rows, cols, static_cast<T*>(out));
+          static_cast<const T*>(x), indices, static_cast<const T*>(weights), bins, padded_bins, num_bins, capacity,
+          top_k, out_rows, cols, static_cast<T*>(out));
     } else {
       gather_rows_kernel<T, 1><<<grid, kWarpsPerCta * 32, 0, stream>>>(
-          static_cast<const T*>(x), indices, static_cast<const T*>(weights), bins, padded_bins, num_bins, top_k,
-          out_rows, cols, static_cast<T*>(out));
+          static_cast<const T*>(x), indices, static_cast<const T*>(weights), bins, padded_bins, num_bins, capacity,
+          top_k, out_rows, cols, static_cast<T*>(out));
     }
   })
   return cudaGetLastError();
@@ -265,6 +332,27 @@ cudaError_t combine_rows(DType type, const void* x, const int* inverse, const vo
           static_cast<const T*>(x), inverse, static_cast<const T*>(weights), static_cast<const T*>(bias),
           top_k, tokens, cols,
           static_cast<T*>(out));
+    }
+  })
+  return cudaGetLastError();
+}
+
+cudaError_t scatter_bwd(DType type, const void* x, const void* grad, const int* indices, const void* weights,
+                        const int* bins, const int* padded_bins, int num_bins, int capacity, int top_k, int64_t copies,
+                        int64_t out_rows, int cols, void* dx, void* dweights, cudaStream_t stream) {
+  MB_SWITCH_FLOAT(type, T, {
+    constexpr int kFull = 16 / sizeof(T);
+    const cudaError_t rc = cudaMemsetAsync(dweights, 0, size_t(copies) * sizeof(T), stream);
+    if (rc != cudaSuccess) return rc;
+    const int grid = ceil_div(out_rows, kWarpsPerCta);
+    if (vec_width<T>(cols, x, grad) > 1 && reinterpret_cast<uintptr_t>(dx) % 16 == 0) {
+      scatter_bwd_kernel<T, kFull><<<grid, kWarpsPerCta * 32, 0, stream>>>(
+          static_cast<const T*>(x), static_cast<const T*>(grad), indices, static_cast<const T*>(weights), bins,
+          padded_bins, num_bins, capacity, top_k, out_rows, cols, static_cast<T*>(dx), static_cast<T*>(dweights));
+    } else {
+      scatter_bwd_kernel<T, 1><<<grid, kWarpsPerCta * 32, 0, stream>>>(
+          static_cast<const T*>(x), static_cast<const T*>(grad), indices, static_cast<const T*>(weights), bins,
+          padded_bins, num_bins, capacity, top_k, out_rows, cols, static_cast<T*>(dx), static_cast<T*>(dweights));
     }
   })
   return cudaGetLastError();

@@ -259,8 +259,8 @@ at::Tensor gather_rows_op(const at::Tensor& x, const at::Tensor& indices, const 
   at::Tensor out = at::empty({out_rows, x.size(1)}, x.options());
   if (out.numel() == 0) return out;
   MB_CUDA_OK(gather_rows(float_code(x.scalar_type()), x.data_ptr(), indices.data_ptr<int>(), opt_ptr(weights),
-                         bins.data_ptr<int>(), padded_bins.data_ptr<int>(), int(bins.numel()), int(top_k), out_rows,
-                         int(x.size(1)), out.data_ptr(), stream()));
+                         bins.data_ptr<int>(), padded_bins.data_ptr<int>(), int(bins.numel()), -1, int(top_k),
+                         out_rows, int(x.size(1)), out.data_ptr(), stream()));
   MB_LAUNCHED(1);
   return out;
 }
@@ -290,6 +290,35 @@ at::Tensor scatter_rows_op(const at::Tensor& x, const at::Tensor& indices, const
                           opt_ptr(bias), int(top_k), tokens, int(x.size(1)), out.data_ptr(), stream()));
   MB_LAUNCHED(1);
   return out;
+}
+
+// Gradients of the weighted un-permutation, {dx, dweights}: x[rows, hidden] laid out by `padded_bins`, or
+// x[experts, capacity, hidden].
+std::vector<at::Tensor> scatter_backward_op(const at::Tensor& x, const at::Tensor& grad, const at::Tensor& indices,
+                                            const at::Tensor& weights, const at::Tensor& bins,
+                                            const c10::optional<at::Tensor>& padded_bins, int64_t top_k) {
+  MB_CHECK_CUDA(x); MB_CHECK_CONTIG(x); MB_CHECK_CUDA(grad); MB_CHECK_CONTIG(grad);
+  const bool binned = !padded_bins.has_value();
+  TORCH_CHECK(x.dim() == (binned ? 3 : 2) && grad.dim() == 2 && x.scalar_type() == grad.scalar_type() &&
+                  x.size(-1) == grad.size(1),
+              "x / grad mismatch");
+  check_index(indices, "indices"); check_index(bins, "bins");
+  if (binned) {
+    TORCH_CHECK(x.size(0) == bins.numel(), "x must hold one slice per bin");
+  } else {
+    check_index(*padded_bins, "padded_bins");
+  }
+  check_weights(weights, x, indices.numel());
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t copies = indices.numel();
+  at::Tensor dx = at::empty_like(x), dw = at::empty({copies}, x.options());
+  if (x.numel() == 0) return {dx, dw.zero_()};
+  MB_CUDA_OK(scatter_bwd(float_code(x.scalar_type()), x.data_ptr(), grad.data_ptr(), indices.data_ptr<int>(),
+                         weights.data_ptr(), bins.data_ptr<int>(), binned ? nullptr : padded_bins->data_ptr<int>(),
+                         int(bins.numel()), binned ? int(x.size(1)) : -1, int(top_k), copies,
+                         x.numel() / x.size(-1), int(x.size(-1)), dx.data_ptr(), dw.data_ptr(), stream()));
+  MB_LAUNCHED(1);
+  return {dx, dw};
 }
 
 at::Tensor scatter_wgrad_op(const at::Tensor& x, const at::Tensor& grad, const at::Tensor& indices,
@@ -322,9 +351,8 @@ at::Tensor binned_gather_rows(const at::Tensor& x, const at::Tensor& indices,
   const int64_t experts = bins.numel();
   at::Tensor out = at::empty({experts, capacity, x.size(1)}, x.options());
   if (out.numel() == 0) return out;
-  at::Tensor uniform = (at::arange(1, experts + 1, bins.options().dtype(at::kLong)) * capacity).to(at::kInt);
   MB_CUDA_OK(gather_rows(float_code(x.scalar_type()), x.data_ptr(), indices.data_ptr<int>(), opt_ptr(weights),
-                         bins.data_ptr<int>(), uniform.data_ptr<int>(), int(experts), int(top_k),
+                         bins.data_ptr<int>(), nullptr, int(experts), int(capacity), int(top_k),
                          experts * capacity, int(x.size(1)), out.data_ptr(), stream()));
   MB_LAUNCHED(1);
   return out;

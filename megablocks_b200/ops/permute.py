@@ -120,6 +120,13 @@ def _autocast(x):
     return x
 
 
+def _one_pass_backward(x, grad, weights) -> bool:
+    """Whether one kernel can give both gradients of the un-permutation (same types, saved rows as the
+    kernel reads them); the two separate kernels take everything else."""
+    return (x.is_cuda and x.is_contiguous() and x.dtype == grad.dtype == weights.dtype and weights.dim() == 1
+            and weights.is_contiguous())
+
+
 class _Gather(torch.autograd.Function):
     """Token order -> expert order; backward is the unweighted scatter."""
 
@@ -163,13 +170,15 @@ class _Scatter(torch.autograd.Function):
         saved = ctx.saved_tensors
         indices, bin_ids, bins, padded_bins = saved[:4]
         weights = saved[4] if ctx.has_weights else None
-        dx = None
-        if ctx.needs_input_grad[0]:
-            dx = _gather_rows(grad, indices, bin_ids, weights, bins, padded_bins, ctx.top_k, ctx.x_rows)
-        dw = None
-        if ctx.need_wgrad:
-            x = saved[-1]
-            dw = _scatter_wgrad(x, grad, indices, bin_ids, bins, padded_bins, ctx.top_k)
+        dx = dw = None
+        if ctx.need_wgrad and ctx.needs_input_grad[0] and _one_pass_backward(saved[-1], grad, weights):
+            debug.check_routing(indices, bin_ids, bins, padded_bins, ctx.top_k, grad.shape[0], ctx.x_rows)
+            dx, dw = ext().scatter_backward(saved[-1], grad, indices, weights, bins, padded_bins, ctx.top_k)
+        else:
+            if ctx.needs_input_grad[0]:
+                dx = _gather_rows(grad, indices, bin_ids, weights, bins, padded_bins, ctx.top_k, ctx.x_rows)
+            if ctx.need_wgrad:
+                dw = _scatter_wgrad(saved[-1], grad, indices, bin_ids, bins, padded_bins, ctx.top_k)
         db = _bias_grad(grad) if ctx.needs_input_grad[7] else None
         return dx, None, None, dw, None, None, None, db
 
@@ -305,12 +314,14 @@ class _BinnedScatter(torch.autograd.Function):
         saved = ctx.saved_tensors
         indices, bins = saved[:2]
         weights = saved[2] if ctx.has_weights else None
-        dx = None
-        if ctx.needs_input_grad[0]:
-            dx = _binned_gather_rows(grad, indices, weights, bins, ctx.bin_size, ctx.top_k)
-        dw = None
-        if ctx.need_wgrad:
-            dw = _binned_scatter_wgrad(saved[-1], grad, indices, bins, ctx.top_k)
+        dx = dw = None
+        if ctx.need_wgrad and ctx.needs_input_grad[0] and _one_pass_backward(saved[-1], grad, weights):
+            dx, dw = ext().scatter_backward(saved[-1], grad, indices, weights, bins, None, ctx.top_k)
+        else:
+            if ctx.needs_input_grad[0]:
+                dx = _binned_gather_rows(grad, indices, weights, bins, ctx.bin_size, ctx.top_k)
+            if ctx.need_wgrad:
+                dw = _binned_scatter_wgrad(saved[-1], grad, indices, bins, ctx.top_k)
         db = _bias_grad(grad) if ctx.needs_input_grad[5] else None
         return dx, None, dw, None, None, db
 

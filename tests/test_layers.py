@@ -309,3 +309,36 @@ def test_scatter_adds_the_output_bias(dtype, top_k, hidden, dropped):
     db, = torch.autograd.grad(out, bias, dy)
     exact = dy.double().sum(0)
     assert torch.all((db.double() - exact).abs() <= eps * exact.abs() + 1e-5 * dy.double().abs().sum(0))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize('layout', ['ragged', 'padded', 'capacity'])
+@pytest.mark.parametrize('top_k,hidden', [(1, 136), (2, 1032), (3, 100)])
+def test_unpermutation_backward_in_one_pass(dtype, layout, top_k, hidden):
+    """Both gradients of the weighted un-permutation against the CPU statements, with pad rows, dropped
+    copies, an empty expert and row lengths around the vector width."""
+    torch.manual_seed(1)
+    tokens, experts, capacity = 61, 6, 12
+    top = torch.randint(0, experts - 1, (tokens * top_k,))
+    indices, bin_ids, bins, padded, _ = ops.route_plan(top, experts)
+    rows = {'ragged': tokens * top_k, 'padded': int(padded[-1]) + 7, 'capacity': experts * capacity}[layout]
+    x = torch.randn(rows, hidden).to(dtype)
+    weights = torch.rand(tokens * top_k).to(dtype)
+    dy = torch.randn(tokens, hidden).to(dtype)
+
+    def grads(dev):
+        args = [t.to(dev) for t in (indices, bin_ids, bins, padded)]
+        xx, ww = x.to(dev).requires_grad_(True), weights.to(dev).requires_grad_(True)
+        if layout == 'capacity':
+            y = ops.binned_scatter(xx.view(experts, capacity, hidden), args[0], ww, args[2], top_k)
+        elif layout == 'padded':
+            y = ops.padded_scatter(xx, args[0], args[1], ww, args[2], args[3], top_k)
+        else:
+            y = ops.scatter(xx, args[0], args[1], ww, args[2], top_k)
+        return torch.autograd.grad(y, [xx, ww], dy.to(dev))
+
+    eps = torch.finfo(dtype).eps
+    for got, want in zip(grads('cuda'), grads('cpu')):
+        # Sums of `hidden` fp32 products in another order, then one rounding.
+        torch.testing.assert_close(got.cpu().float(), want.float(), rtol=2 * eps, atol=1e-5 * hidden ** 0.5 + eps)
