@@ -23,7 +23,7 @@ import torch
 
 from megablocks_b200.layers import common, mpu
 from megablocks_b200.layers.arguments import Arguments, InitFn
-from megablocks_b200.layers.fused_mlp import expert_mlp
+from megablocks_b200.layers.fused_mlp import capacity_mlp, capacity_mlp_fused, expert_mlp
 from megablocks_b200.ops import gg as G
 from megablocks_b200.ops import sparse
 
@@ -140,9 +140,16 @@ class MLP(_ExpertWeights):
         return self._bins_cache[key]
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        experts, capacity, hidden = x.shape
+        if capacity > 0:
+            w1, w2 = resolve_dtensor(self.w1), resolve_dtensor(self.w2)
+            if capacity_mlp_fused(x, w1, w2, self.args.activation_fn):
+                y = capacity_mlp(x.reshape(experts * capacity, hidden), w1, w2,
+                                 self._uniform_bins(experts, capacity, x.device), self.args.activation_fn,
+                                 self.wgrad_scale())
+                return y.view(experts, capacity, -1)
         w1 = resolve_dtensor(self.scale_grad(self.w1))
         w2 = resolve_dtensor(self.scale_grad(self.w2))
-        experts, capacity, hidden = x.shape
         if capacity == 0:
             return x.new_zeros(experts, 0, w2.shape[-1])
         bins = self._uniform_bins(experts, capacity, x.device)

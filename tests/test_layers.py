@@ -342,3 +342,25 @@ def test_unpermutation_backward_in_one_pass(dtype, layout, top_k, hidden):
     for got, want in zip(grads('cuda'), grads('cpu')):
         # Sums of `hidden` fp32 products in another order, then one rounding.
         torch.testing.assert_close(got.cpu().float(), want.float(), rtol=2 * eps, atol=1e-5 * hidden ** 0.5 + eps)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('act', [partial(F.gelu, approximate='tanh'), F.silu, F.gelu])
+@pytest.mark.parametrize('tokens,hidden,ffn', [(40, 64, 72), (333, 136, 256)])
+def test_token_dropping_experts_in_gemm_epilogues(act, tokens, hidden, ffn):
+    """Experts of the token-dropping layer with the activation in the GEMM epilogues, against the same
+    layer with a callable the kernel does not know (elementwise passes)."""
+    torch.manual_seed(0)
+    grads = []
+    for fn in (act, lambda z: act(z)):
+        torch.manual_seed(0)
+        layer = mb.MoE(mb.Arguments(hidden_size=hidden, ffn_hidden_size=ffn, moe_num_experts=4, moe_top_k=2,
+                                    moe_capacity_factor=1, activation_fn=fn, bias=False, return_bias=False, fp16=False,
+                                    bf16=True, device=torch.device('cuda')))
+        x = torch.randn(tokens, 1, hidden, device='cuda').bfloat16().requires_grad_(True)
+        y = layer(x)
+        moe_mod.clear_load_balancing_loss()
+        grads.append([y] + list(torch.autograd.grad(y, [x] + list(layer.parameters()), torch.ones_like(y))))
+    for got, want in zip(*grads):
+        # bf16 intermediates are rounded alike on both sides; sums differ in order and in the last place.
+        torch.testing.assert_close(got, want, rtol=3e-2, atol=2e-2 * float(want.detach().float().abs().max()) + 1e-6)
