@@ -63,9 +63,13 @@ struct SortScratch {
   int chunk, num_chunks;
 };
 
-SortScratch make_scratch(int64_t n, int nbins, const at::TensorOptions& opts) {
+// The route plan allocates its scratch, so its chunks can stay short (the serial walk of a chunk is what
+// a placement takes: 39 us for 131072 copies in chunks of 2048).
+int route_warp_chunk(int64_t n) { return n <= (1 << 16) ? 128 : (n <= (1 << 20) ? 512 : sort_warp_chunk(n)); }
+
+SortScratch make_scratch(int64_t n, int nbins, const at::TensorOptions& opts, int chunk = 0) {
   SortScratch s;
-  s.chunk = sort_warp_chunk(n);
+  s.chunk = chunk > 0 ? chunk : sort_warp_chunk(n);
   s.num_chunks = std::max<int>(1, int(ceil_div(n, s.chunk)));
   s.partial = at::empty({int64_t(nbins) * s.num_chunks}, opts.dtype(at::kInt));
   s.totals = at::empty({nbins}, opts.dtype(at::kInt));
@@ -160,7 +164,26 @@ std::vector<at::Tensor> route_plan(const at::Tensor& top_experts, int64_t num_ex
   // The scan kernel of the sort writes all three per-expert arrays in full.
   at::Tensor bins = at::empty({num_experts}, iopts), padded_bins = at::empty({num_experts}, iopts);
   at::Tensor tpe = at::empty({num_experts}, iopts);
-  // torch.topk yields int64 ids: narrow once, then a single counting-sort pass.
+  const bool ids64 = top_experts.scalar_type() == at::kLong;      // what top-k yields: read as they are
+  if (n <= kPlanMaxCopies && (1 << bits_for(num_experts)) <= kPlanMaxBins &&
+      (ids64 || top_experts.scalar_type() == at::kInt)) {
+    MB_CUDA_OK(route_plan_small(ids64, top_experts.data_ptr(), int(n), bits_for(num_experts), int(num_experts),
+                                int(block), indices.data_ptr<int>(), bin_ids.data_ptr<int>(), bins.data_ptr<int>(),
+                                padded_bins.data_ptr<int>(), tpe.data_ptr<int>(), stream()));
+    MB_LAUNCHED(1);
+    return {indices, bin_ids, bins, padded_bins, tpe};
+  }
+  if (ids64 && num_experts <= kMaxSortBins) {
+    const int bits = bits_for(num_experts);
+    SortScratch s = make_scratch(n, 1 << bits, top_experts.options(), route_warp_chunk(n));
+    MB_CUDA_OK(route_sort64(top_experts.data_ptr<int64_t>(), n, bits, s.chunk, s.num_chunks, s.partial.data_ptr<int>(),
+                            s.totals.data_ptr<int>(), bin_ids.data_ptr<int>(), indices.data_ptr<int>(),
+                            tpe.data_ptr<int>(), bins.data_ptr<int>(), padded_bins.data_ptr<int>(), int(num_experts),
+                            int(block), stream()));
+    MB_LAUNCHED(3);
+    return {indices, bin_ids, bins, padded_bins, tpe};
+  }
+  // Other id types are narrowed once; then a single counting-sort pass.
   at::Tensor e32 = top_experts.scalar_type() == at::kInt ? top_experts : top_experts.to(at::kInt);
   if (num_experts <= kMaxSortBins) {
     const int bits = bits_for(num_experts);

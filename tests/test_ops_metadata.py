@@ -153,3 +153,16 @@ def test_micro_benchmark_scripts_run_on_the_host():
     assert [r['bins'] for r in rows] == [2, 4, 8, 16, 32, 64, 128, 256]
     rows = padded_scatter_benchmark.run(cpu, iters=1, cases=((512, 64, 8, 4), (2048, 64, 8, 1)))
     assert len(rows) == 2 and all(r['forward_us'] > 0 and r['backward_us'] > 0 for r in rows)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('dtype', [torch.int32, torch.int64])
+@pytest.mark.parametrize('copies', [1, 31, 1025, 4096, 4097, 16385, 131073, 65537])
+@pytest.mark.parametrize('experts', [1, 5, 256, 257, 1000])
+def test_route_plan_paths_agree_with_cpu(dtype, copies, experts):
+    """One-launch plan (up to 4096 copies and 256 experts) and the three-launch sort, both id types, against
+    the composed CPU ops; the sort is stable and whole, so everything is equal."""
+    torch.manual_seed(copies + experts)
+    top = (torch.rand(copies) ** 2 * experts).to(dtype)          # uneven, some experts empty
+    for got, want in zip(ops.route_plan(top.cuda(), experts, 128), ops.route_plan(top, experts, 128)):
+        assert got.dtype == torch.int32 and torch.equal(got.cpu(), want.to(torch.int32))
