@@ -730,12 +730,23 @@ std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, c
   // 588 | 635.
   const bool streams_weights = layout != kTN && a.size(0) <= 16 * num_groups &&
                                (1 + std::min<int64_t>(num_groups, a.size(0))) * ceil_div(p.N, 256) >= sm_count() / 2;
+  // A long contraction over few waves of tiles: a pair's tiles are twice as large, and the last wave can
+  // cost it more than its loop gains.  Compared by waves x cycles of a K step (256 for the weights' load
+  // and one per token of a tile; the single-CTA loop runs 7 % longer), with half a tile per group for the
+  // raggedness.  4094 rows over 8 groups, 14336 -> 4096: single 447 us, pair 502.
+  auto few_waves_lose = [&] {
+    if (layout == kTN || p.K < 2048 || (epilogue != kEpiNone && epilogue != kEpiAct)) return false;
+    const double rows = double(a.size(0)), groups = double(num_groups), nb = double(ceil_div(p.N, 256));
+    const double tiles2 = rows / 256 + 0.5 * groups, tiles1 = rows / 128 + 0.5 * groups;
+    const double waves2 = std::ceil(tiles2 * nb / (sm_count() / 2)), waves1 = std::ceil(tiles1 * nb / sm_count());
+    return waves2 <= 6 && waves1 * 512 * 1.07 < waves2 * (256 + rows / tiles2);
+  };
   bool pair_ok = block_n == 256 && !dual && p.N >= 256 && sm_count() >= 2 && !scatter.has_value() &&
                  !wait_flags.has_value() && num_groups <= kSmallGroupsHost &&
                  (layout != kTN || epilogue == kEpiNone) && pair_mode != 0;
   if (pair_ok && p.aux1) pair_ok = make_output_map(&p.aux_map[0], p.aux1, bf16, out_numel / p.N, p.N);
   if (pair_ok && p.aux2) pair_ok = make_output_map(&p.aux_map[1], p.aux2, bf16, out_numel / p.N, p.N);
-  const bool pair = pair_ok && (pair_mode == 1 || !streams_weights);
+  const bool pair = pair_ok && (pair_mode == 1 || !(streams_weights || few_waves_lose()));
   if (!scatter.has_value() && store_tma_enabled()) {
     // Full 32-row quarters of a tile leave through the TMA unit (one instruction per chunk).
     const int64_t out_rows = out_numel / p.N;
