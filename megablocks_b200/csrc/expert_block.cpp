@@ -1,0 +1,164 @@
+// The routed expert computation of one device - plan, permute, expert GEMMs, weighted un-permute - as one
+// native call forward and one backward.  The kernels are those behind the separate ops; what this saves
+// is the host's time between them: some 20 us of Python per op (an autograd node, argument checks and
+// conversions), which bounds small calls (a decode step of 8 tokens has 60 us of kernels, a 256-token
+// training pass 110).
+//
+// Two layouts, as in the layers (megablocks/layers/dmoe.py:196-249, moe.py:185-245 of the reference):
+//   capacity < 0   dropless: ragged row groups, weights [E, f, h], groups given by the plan's `bins`;
+//   capacity > 0   token-dropping: [E, capacity, h] slots, w1 [E, h, f], groups given by `gemm_bins`.
+#include <torch/extension.h>
+
+#include "kernels.h"
+
+namespace mb {
+
+using OptTensor = c10::optional<at::Tensor>;
+
+std::vector<at::Tensor> route_plan(const at::Tensor& top_experts, int64_t num_experts, int64_t block);
+at::Tensor gather_rows_op(const at::Tensor& x, const at::Tensor& indices, const at::Tensor& bin_ids,
+                          const OptTensor& weights, const at::Tensor& bins, const at::Tensor& padded_bins,
+                          int64_t top_k, int64_t out_rows);
+at::Tensor binned_gather_rows(const at::Tensor& x, const at::Tensor& indices, const OptTensor& weights,
+                              const at::Tensor& bins, int64_t capacity, int64_t top_k);
+at::Tensor scatter_rows_op(const at::Tensor& x, const at::Tensor& indices, const at::Tensor& bin_ids,
+                           const OptTensor& weights, const at::Tensor& bins, const at::Tensor& padded_bins,
+                           int64_t top_k, int64_t tokens, const OptTensor& bias);
+at::Tensor binned_scatter_rows(const at::Tensor& x, const at::Tensor& indices, const OptTensor& weights,
+                               const at::Tensor& bins, int64_t top_k, int64_t tokens, const OptTensor& bias);
+std::vector<at::Tensor> scatter_backward_op(const at::Tensor& x, const at::Tensor& grad, const at::Tensor& indices,
+                                            const at::Tensor& weights, const at::Tensor& bins,
+                                            const OptTensor& padded_bins, int64_t top_k);
+at::Tensor column_sum_op(const at::Tensor& x);
+std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, const at::Tensor& bins, bool trans_a,
+                                     bool trans_b, int64_t epilogue, int64_t act, const OptTensor& aux1,
+                                     const OptTensor& aux2, bool want_out2, bool want_out3, int64_t num_groups,
+                                     const OptTensor& c_in, bool zero_tail, const OptTensor& wait_flags,
+                                     int64_t wait_count, int64_t wait_stride, int64_t wait_seq, int64_t rows_hint,
+                                     int64_t pair_mode, const c10::optional<std::vector<at::Tensor>>& scatter,
+                                     const std::vector<int64_t>& scatter_args, double alpha, const OptTensor& a2,
+                                     const OptTensor& b2, const OptTensor& sqnorm, const OptTensor& seq_base);
+
+namespace {
+
+struct Gemm {
+  bool trans_a = false, trans_b = false;
+  int64_t epilogue = gemm::kEpiNone, act = 0;
+  OptTensor aux1, aux2, a2, b2, sqnorm;
+  bool want_out2 = true, want_out3 = true;
+  double alpha = 1.0;
+
+  std::vector<at::Tensor> run(const at::Tensor& a, const at::Tensor& b, const at::Tensor& bins, int64_t pair) const {
+    return grouped_gemm(a, b, bins, trans_a, trans_b, epilogue, act, aux1, aux2, want_out2, want_out3, bins.numel(), {},
+                        true, {}, 0, 0, 0, 0, pair, {}, {}, alpha, a2, b2, sqnorm, {});
+  }
+};
+
+at::Tensor rows_of(const at::Tensor& t) { return t.dim() == 3 ? t.view({-1, t.size(2)}) : t; }
+
+}  // namespace
+
+// {out, tokens_per_expert} or, with `save`, also {indices, bin_ids, bins, x rows, y rows, z1, z2, h}
+// (z2 undefined for the MLP).
+std::vector<at::Tensor> expert_block_forward(const at::Tensor& x, const at::Tensor& top_experts,
+                                             const at::Tensor& weights, const at::Tensor& w1, const at::Tensor& w2,
+                                             const OptTensor& v1, const OptTensor& bias, const OptTensor& gemm_bins,
+                                             int64_t num_experts, int64_t top_k, int64_t act, int64_t capacity, bool save,
+                                             int64_t pair) {
+  const auto plan = route_plan(top_experts, num_experts, 128);
+  const at::Tensor &indices = plan[0], &bin_ids = plan[1], &bins = plan[2];
+  const bool binned = capacity > 0;
+  TORCH_CHECK(!binned || (gemm_bins.has_value() && !v1.has_value()), "capacity layout: uniform bins, no gate weight");
+  const int64_t tokens = x.size(0);
+  at::Tensor rows = binned ? rows_of(binned_gather_rows(x, indices, {}, bins, capacity, top_k))
+                           : gather_rows_op(x, indices, bin_ids, {}, bins, bins, top_k, indices.numel());
+  const at::Tensor& groups = binned ? *gemm_bins : bins;
+  at::Tensor z1, z2, h;
+  Gemm up;
+  up.trans_b = !binned;
+  up.act = act;
+  if (v1.has_value()) {
+    up.epilogue = gemm::kEpiGluDual;
+    up.b2 = v1;
+    auto o = up.run(rows, w1, groups, pair);
+    z2 = o[0]; h = o[1]; z1 = o[2];
+  } else {
+    up.epilogue = gemm::kEpiAct;
+    auto o = up.run(rows, w1, groups, pair);
+    z1 = o[0]; h = o[1];
+  }
+  at::Tensor y = Gemm{}.run(h, w2, groups, pair)[0];
+  at::Tensor out;
+  if (binned) {
+    y = y.view({num_experts, capacity, -1});
+    out = binned_scatter_rows(y, indices, weights, bins, top_k, tokens, bias);
+  } else {
+    out = scatter_rows_op(y, indices, bin_ids, weights, bins, bins, top_k, tokens, bias);
+  }
+  if (!save) return {out, plan[4]};
+  return {out, plan[4], indices, bin_ids, bins, rows, y, z1, z2, h};
+}
+
+// {dx, dweights, dw1, dw2, dv1, dbias}, undefined where `needs` says so.  `slots`: per weight gradient
+// (w1, w2, v1) an optional accumulator of its squared norm.
+std::vector<at::Tensor> expert_block_backward(const at::Tensor& dout, const at::Tensor& indices,
+                                              const at::Tensor& bin_ids, const at::Tensor& bins,
+                                              const OptTensor& gemm_bins, const at::Tensor& rows, const at::Tensor& y,
+                                              const at::Tensor& z1, const OptTensor& z2, const OptTensor& h_in,
+                                              const at::Tensor& weights, const at::Tensor& w1, const at::Tensor& w2,
+                                              const OptTensor& v1, const std::vector<bool>& needs,
+                                              const std::vector<OptTensor>& slots, int64_t top_k, int64_t act,
+                                              double wgrad_scale, int64_t capacity, int64_t pair) {
+  const bool binned = capacity > 0;
+  const at::Tensor& groups = binned ? *gemm_bins : bins;
+  const int64_t tokens = dout.size(0);
+  at::Tensor dx, dweights, dw1, dw2, dv1, dbias;
+  if (needs[5]) dbias = column_sum_op(dout);
+  auto un = scatter_backward_op(y, dout, indices, weights, bins, binned ? OptTensor() : OptTensor(bins), top_k);
+  if (needs[1]) dweights = un[1];
+  if (!(needs[0] || needs[2] || needs[3] || needs[4])) return {dx, dweights, dw1, dw2, dv1, dbias};
+  const at::Tensor dy = rows_of(un[0]);
+  Gemm down;
+  down.trans_b = true;
+  down.act = act;
+  down.aux1 = z1;
+  at::Tensor dz1, dz2, h = h_in.has_value() ? *h_in : at::Tensor();
+  if (v1.has_value()) {
+    down.epilogue = gemm::kEpiDGlu;
+    down.aux2 = z2;
+    down.want_out3 = !h.defined();
+    auto o = down.run(dy, w2, groups, pair);
+    dz1 = o[0]; dz2 = o[1];
+    if (!h.defined()) h = o[2];
+  } else {
+    down.epilogue = gemm::kEpiDAct;
+    down.want_out2 = !h.defined();
+    auto o = down.run(dy, w2, groups, pair);
+    dz1 = o[0];
+    if (!h.defined()) h = o[1];
+  }
+  auto wgrad = [&](const at::Tensor& a, const at::Tensor& b, const OptTensor& slot) {
+    Gemm g;
+    g.trans_a = true;
+    g.alpha = wgrad_scale;
+    g.sqnorm = slot;
+    return g.run(a, b, groups, pair)[0];
+  };
+  if (needs[3]) dw2 = wgrad(h, dy, slots[1]);
+  if (needs[2]) dw1 = binned ? wgrad(rows, dz1, slots[0]) : wgrad(dz1, rows, slots[0]);
+  if (v1.has_value() && needs[4]) dv1 = wgrad(dz2, rows, slots[2]);
+  if (needs[0]) {
+    Gemm in;
+    in.trans_b = binned;
+    if (v1.has_value()) {       // dx = dz1 w1 + dz2 v1 as one contraction over both pairs
+      in.a2 = dz2;
+      in.b2 = v1;
+    }
+    at::Tensor d = in.run(dz1, w1, groups, pair)[0];
+    dx = binned ? binned_scatter_rows(d.view({groups.numel(), capacity, -1}), indices, {}, bins, top_k, tokens, {})
+                : scatter_rows_op(d, indices, bin_ids, {}, bins, bins, top_k, tokens, {});
+  }
+  return {dx, dweights, dw1, dw2, dv1, dbias};
+}
+
+}  // namespace mb

@@ -17,7 +17,7 @@ row-blocks past the last expert are zero and cost no FLOPs.
 import torch
 
 from megablocks_b200 import ops
-from megablocks_b200.layers import common, dmlp_registry, moe, mpu
+from megablocks_b200.layers import common, dmlp_registry, glu, mlp, moe, mpu
 from megablocks_b200.layers.arguments import Arguments
 from megablocks_b200.ops import sparse
 
@@ -147,6 +147,20 @@ class ParallelDroplessMLP(moe.ParallelMLP):
                                                 mlp._grouped_view(w2), v1, w1_kn=False, expert_capacity=0)
 
     # -- dispatch --------------------------------------------------------------
+    _block_steps = ('forward', 'indices_and_bins', 'forward_once', '_forward_once', 'grouped_forward_once',
+                    'grouped_permute_and_compute')
+
+    def _block_experts(self, tokens: int):
+        m = self.mlp
+        if self.args.mlp_impl != 'grouped' or type(m) not in (mlp.GroupedMLP, glu.GroupedGLU):
+            return None
+        v1 = m.v1 if type(m) is glu.GroupedGLU else None
+        if any(hasattr(w, 'to_local') for w in (m.w1, m.w2)):
+            return None
+        view = m._grouped_view
+        return (view(m.w1), view(m.w2), None if v1 is None else view(v1), None, -1,
+                bool(self.args.memory_optimized_mlp))
+
     _bias_steps = ('forward_once', '_forward_once', 'sparse_forward_once', 'grouped_forward_once',
                    'grouped_permute_and_compute')
 

@@ -24,9 +24,10 @@ import torch
 import torch.distributed as dist
 
 from megablocks_b200 import ops
-from megablocks_b200.layers import common, mlp, mpu, router, sharedexpert_registry
+from megablocks_b200.layers import common, expert_block, mlp, mpu, router, sharedexpert_registry
 from megablocks_b200.layers.all_to_all import all_to_all
 from megablocks_b200.layers.arguments import Arguments
+from megablocks_b200.layers.fused_mlp import capacity_mlp_fused
 from megablocks_b200.utils.metrics import comm_timer, nvtx_range
 
 _LOAD_BALANCING_LOSS = []
@@ -158,6 +159,40 @@ class ParallelMLP(torch.nn.Module):
 
     def forward_once(self, x: torch.Tensor, expert_weights: torch.Tensor, top_experts: torch.Tensor):
         return self._forward_once(x, expert_weights, top_experts, None)
+
+    _block_steps = ('forward', 'indices_and_bins', 'expert_capacity') + _bias_steps
+
+    def _block_call(self, x: torch.Tensor, expert_weights: torch.Tensor, top_experts: torch.Tensor):
+        """``(out, tokens_per_expert, whether the bias is in it)`` from the single native call, or ``None``
+        where the layer has to run step by step."""
+        base, cls = self._bias_base, type(self)
+        if (getattr(self.forward_fn, '__func__', None) is not base.forward_once
+                or any(getattr(cls, name) is not getattr(base, name) for name in base._block_steps)):
+            return None
+        experts = self._block_experts(x.numel() // x.shape[-1])
+        if experts is None:
+            return None
+        w1, w2, v1, gemm_bins, capacity, memory_optimized = experts
+        bias = self.bias if self.bias is not None and not self.args.return_bias else None
+        top_experts, expert_weights = top_experts.flatten(), expert_weights.flatten()
+        args = self.args
+        if torch.is_grad_enabled() and not expert_weights.requires_grad and (x.requires_grad or w1.requires_grad):
+            return None         # a frozen router: the step-by-step path keeps less for the backward pass
+        if not expert_block.route(x, expert_weights, top_experts, self.mlp, w1, w2, v1, bias, args.activation_fn):
+            return None
+        out, counts = expert_block.expert_block(x, expert_weights, top_experts, w1, w2, v1, bias, gemm_bins,
+                                                self.num_experts, self.top_k, args.activation_fn, capacity,
+                                                memory_optimized, self.mlp.wgrad_scale())
+        return out, counts, bias is not None
+
+    def _block_experts(self, tokens: int):
+        """Expert tensors of the single native call: ``(w1, w2, v1, gemm_bins, capacity, memory_optimized)``."""
+        m = self.mlp
+        capacity = self.expert_capacity(tokens)
+        if type(m) is not mlp.MLP or capacity <= 0 or not m.w1.is_cuda or not capacity_mlp_fused(
+                m.w1, m.w1, m.w2, self.args.activation_fn):
+            return None
+        return m.w1, m.w2, None, m._uniform_bins(self.num_experts, capacity, m.w1.device), capacity, False
 
     def _forward_once(self, x, expert_weights, top_experts, bias):
         expert_weights = expert_weights.flatten()
@@ -319,8 +354,12 @@ class ParallelMLP(torch.nn.Module):
     def forward(self, x: torch.Tensor, scores: torch.Tensor, expert_weights: torch.Tensor,
                 top_experts: torch.Tensor):
         in_shape = x.size()
-        fused_bias = self._unpermute_bias(x)
-        if fused_bias is not None:
+        block = self._block_call(x, expert_weights, top_experts)
+        fused_bias = None
+        if block is not None:
+            x, tokens_per_expert, with_bias = block
+            fused_bias = self.bias if with_bias else None
+        elif (fused_bias := self._unpermute_bias(x)) is not None:
             x, tokens_per_expert = self._forward_once(x, expert_weights, top_experts, fused_bias)
         else:
             x, tokens_per_expert = self.forward_fn(x, expert_weights, top_experts)

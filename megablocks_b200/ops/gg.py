@@ -200,6 +200,13 @@ class GradNormSink:
         i = len(self._by_address)
         return (i, self.slots[i:i + 1]) if i < self.slots.numel() else (None, None)
 
+    def reserve(self, count: int):
+        """``count`` consecutive ``(slot, view)`` pairs (``(None, None)`` past the last), to be recorded in
+        this order before any other launch takes one."""
+        first = len(self._by_address)
+        return [(i, self.slots[i:i + 1]) if i < self.slots.numel() else (None, None)
+                for i in range(first, first + count)]
+
     def _record(self, out: torch.Tensor, slot: int) -> None:
         self._by_address[out.data_ptr()] = (slot, out.numel())
 

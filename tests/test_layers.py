@@ -364,3 +364,75 @@ def test_token_dropping_experts_in_gemm_epilogues(act, tokens, hidden, ffn):
     for got, want in zip(*grads):
         # bf16 intermediates are rounded alike on both sides; sums differ in order and in the last place.
         torch.testing.assert_close(got, want, rtol=3e-2, atol=2e-2 * float(want.detach().float().abs().max()) + 1e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('kind', ['mlp', 'glu', 'dropping'])
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize('tokens,top_k,bias,memory_optimized', [(1, 1, True, False), (37, 2, False, True), (300, 1, True, True)])
+def test_native_expert_block_equals_the_separate_ops(kind, dtype, tokens, top_k, bias, memory_optimized):
+    """One native call against the same kernels launched op by op (a hook on the expert module sends the
+    layer there): outputs and every gradient are equal, with and without autograd."""
+    torch.manual_seed(0)
+    args = mb.Arguments(hidden_size=72, ffn_hidden_size=264, moe_num_experts=5, moe_top_k=top_k, moe_capacity_factor=1,
+                        mlp_type='glu' if kind == 'glu' else 'mlp', mlp_impl='grouped', activation_fn=F.silu, bias=bias,
+                        return_bias=False, memory_optimized_mlp=memory_optimized, fp16=dtype == torch.float16,
+                        bf16=dtype == torch.bfloat16, device=torch.device('cuda'))
+    layer = (mb.MoE if kind == 'dropping' else mb.dMoE)(args)
+    if bias:
+        torch.nn.init.normal_(layer.experts.bias)
+    x = torch.randn(tokens, 1, 72, device='cuda').to(dtype).requires_grad_(True)
+    dy = torch.randn_like(x)
+
+    def run():
+        y = layer(x)
+        moe_mod.clear_load_balancing_loss()
+        with torch.no_grad():
+            plain = layer(x)
+        moe_mod.clear_load_balancing_loss()
+        return [y, plain] + list(torch.autograd.grad(y, [x] + list(layer.parameters()), dy))
+
+    assert layer.experts._block_call(x, *layer.router(x)[1:]) is not None or tokens * top_k < 5
+    moe_mod.clear_load_balancing_loss()
+    fast = run()
+    hook = layer.experts.mlp.register_forward_hook(lambda *a: None)
+    assert layer.experts._block_call(x, *layer.router(x)[1:]) is None
+    slow = run()
+    hook.remove()
+    for got, want in zip(fast, slow):
+        assert torch.equal(got, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize('experts', [4, 8, 24, 32, 64, 128, 256, 320])
+@pytest.mark.parametrize('top_k,norm_p', [(1, 0), (2, 1), (4, 2), (8, 0)])
+def test_router_selection_over_expert_counts(dtype, experts, top_k, norm_p):
+    """Vector and warp-per-token router kernels, forward and backward, around their size limits, with equal
+    logits (ties go to the lowest id) and an infinite one."""
+    if top_k > experts:
+        return
+    torch.manual_seed(experts)
+    logits = torch.randn(37, experts).to(dtype)
+    logits[3] = 0.5
+    logits[5, 1] = -float('inf')
+    got = router_mod._FusedTopK.apply(logits.cuda().requires_grad_(True), top_k, float(norm_p))
+    scores = logits.float().softmax(-1).to(dtype)
+    # An fp32 exponential and sum: within one unit of the last place after rounding.
+    torch.testing.assert_close(got[0].detach().cpu().float(), scores.float(), rtol=2 * torch.finfo(dtype).eps + 1e-5, atol=1e-7)
+    own = got[0].detach().cpu()
+    order = torch.sort(own.float(), dim=-1, descending=True, stable=True)[1][:, :top_k]
+    assert torch.equal(got[2].cpu(), order)
+    x = own.double().requires_grad_(True)       # d logits = s (g - <g, s>) for the scores that were selected from
+    w = x.gather(1, order)
+    if norm_p:
+        w = w / w.norm(p=norm_p, dim=-1, keepdim=True)
+    torch.testing.assert_close(got[1].detach().cpu().double(), w.detach(), rtol=3 * torch.finfo(dtype).eps, atol=1e-7)
+    ds, dw = torch.randn_like(own), torch.randn(37, top_k).to(dtype)
+    g, = torch.autograd.grad([x, w], x, [ds.double(), dw.double()])
+    want = own.double() * (g - (g * own.double()).sum(-1, keepdim=True))
+    leaf = logits.cuda().requires_grad_(True)
+    out = router_mod._FusedTopK.apply(leaf, top_k, float(norm_p))
+    dl, = torch.autograd.grad([out[0], out[1]], leaf, [ds.cuda(), dw.cuda()])
+    torch.testing.assert_close(dl.cpu().double(), want, rtol=4 * torch.finfo(dtype).eps + 1e-5,
+                               atol=1e-5 + torch.finfo(dtype).eps * float(want.abs().max()))
