@@ -21,6 +21,10 @@
 // transposed topology), described to the MMA by the matching descriptors, so no transposed copy
 // of a dense matrix or of the block values is made.
 //
+// The dense output columns of a dsd tile are 128 or 256 (BN): with 256 every block of values is loaded
+// for twice as many columns, 48 KB per 512 tensor-pipe cycles instead of 32 KB per 256, which is what the
+// products are bound by.  sdd and dds tiles are one block wide.
+//
 // Roles per CTA (320 threads, one CTA per SM, tiles taken round-robin): warp 8 TMA producer,
 // warp 9 tensor-memory owner and MMA issuer, warps 0-7 epilogue (tcgen05.ld, convert, coalesced
 // stores through a swizzled staging buffer).  Two accumulator stages overlap the epilogue of a
@@ -44,11 +48,19 @@ using gemm::kThreads;
 using gemm::kUmmaK;
 using gemm::kWaitLimitNs;
 
-constexpr int kStages = 6;
-constexpr int kBBytes = kBlock * kBlockK * 2;
-constexpr int kTileBytes = kStages * (kABytes + kBBytes);
-constexpr int kSmemBytes = kTileBytes + kEpilogueWarps * 2048 + 256 + 1024;
-constexpr int kTmemCols = 2 * kBlock;
+template <int BN>
+struct Config {
+  static constexpr int kStages = BN == 256 ? 4 : 6;
+  static constexpr int kBBytes = BN * kBlockK * 2;
+  static constexpr int kTileBytes = kStages * (kABytes + kBBytes);
+  static constexpr int kSmemBytes = kTileBytes + kEpilogueWarps * 2048 + 256 + 1024;
+  static constexpr int kTmemCols = 2 * BN;
+};
+
+// Block indices come as int32 or, as the topology stores them, int16.
+__device__ __forceinline__ int load_index(const int* base, int i, int idx16) {
+  return idx16 ? static_cast<int>(__ldg(reinterpret_cast<const int16_t*>(base) + i)) : __ldg(base + i);
+}
 
 struct Work {
   int out_row;      // first row of the output tile
@@ -59,10 +71,13 @@ struct Work {
   int seg_end;
 };
 
-template <typename T, bool A_MN, bool B_MN>
+template <typename T, bool A_MN, bool B_MN, int BN>
 __global__ void __launch_bounds__(kThreads, 1)
 bsmm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
             const __grid_constant__ BsmmParams p) {
+  using Cfg = Config<BN>;
+  constexpr int kStages = Cfg::kStages, kBBytes = Cfg::kBBytes, kTileBytes = Cfg::kTileBytes;
+  constexpr int kTmemCols = Cfg::kTmemCols;
   constexpr bool kIsBf16 = std::is_same<T, __nv_bfloat16>::value;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -105,8 +120,8 @@ bsmm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   auto decode = [&](int t) {
     Work w;
     if (p.mode == kSdd) {
-      w.a_block = __ldg(p.row_indices + t);
-      w.b_block = __ldg(p.column_indices + t);
+      w.a_block = load_index(p.row_indices, t, p.idx16);
+      w.b_block = load_index(p.column_indices, t, p.idx16);
       w.out_row = t * kBlock;
       w.out_col = 0;
       w.seg_begin = 0;
@@ -114,7 +129,7 @@ bsmm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     } else if (p.mode == kDsd) {
       const int i = t / p.tiles_inner, nb = t - i * p.tiles_inner;   // inner: column tiles of the output
       w.out_row = i * kBlock;
-      w.out_col = nb * kBlock;
+      w.out_col = nb * BN;
       w.a_block = 0;
       w.b_block = nb;
       w.seg_begin = __ldg(p.seg_offsets + i);
@@ -165,7 +180,7 @@ bsmm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             if ((ks & 1) == 0) {
               const int idx = w.seg_begin + (ks >> 1);
               blk = p.seg_block != nullptr ? __ldg(p.seg_block + idx) : idx;
-              kblk = __ldg(p.seg_k + idx);
+              kblk = load_index(p.seg_k, idx, p.idx16);
             }
             const int half = (ks & 1) * kBlockK;
             if (p.mode == kDsd) {       // A = block values, B = dense
@@ -188,7 +203,7 @@ bsmm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           }
           if constexpr (B_MN) {
 #pragma unroll
-            for (int j = 0; j < kBlock / 64; ++j) tma_load_2d(b_dst + j * kBoxBytes, &tmap_b, bar, bn + 64 * j, bk);
+            for (int j = 0; j < BN / 64; ++j) tma_load_2d(b_dst + j * kBoxBytes, &tmap_b, bar, bn + 64 * j, bk);
           } else {
             tma_load_2d(b_dst, &tmap_b, bar, bk, bn);
           }
@@ -198,27 +213,26 @@ bsmm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     }
   } else if (warp == kMmaWarp) {
     // ======================= MMA issuer ==========================================
-    constexpr uint32_t idesc = instr_desc_f16(kIsBf16, A_MN, B_MN, kBlockM, kBlock);
+    constexpr uint32_t idesc = instr_desc_f16(kIsBf16, A_MN, B_MN, kBlockM, BN);
     int stage = 0;
     uint32_t phase = 0;
     int acc_stage = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-      const Work w = decode(t);
-      const int steps = k_steps(w);
-      ok = mbar_wait(smem_u32(&tmem_empty_bar[acc_stage]), acc_phase ^ 1u, abort_flag, p.status, gemm::kErrMmaTmem,
-                     kWaitLimitNs);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      tcgen05_fence_after();
-      const uint32_t d_tmem = tmem_base + acc_stage * kBlock;
-      for (int ks = 0; ks < steps; ++ks) {
-        ok = mbar_wait(smem_u32(&full_bar[stage]), phase, abort_flag, p.status, gemm::kErrMmaFull, kWaitLimitNs);
-        ok = __all_sync(0xffffffffu, ok);
+    // One thread issues: a warp-synchronous loop costs the tensor pipe about 4 % of its cycles.
+    if (lane == 0) {
+      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+        const Work w = decode(t);
+        const int steps = k_steps(w);
+        ok = mbar_wait(smem_u32(&tmem_empty_bar[acc_stage]), acc_phase ^ 1u, abort_flag, p.status, gemm::kErrMmaTmem,
+                       kWaitLimitNs);
         if (!ok) break;
         tcgen05_fence_after();
-        if (lane == 0) {
+        const uint32_t d_tmem = tmem_base + acc_stage * BN;
+        for (int ks = 0; ks < steps; ++ks) {
+          ok = mbar_wait(smem_u32(&full_bar[stage]), phase, abort_flag, p.status, gemm::kErrMmaFull, kWaitLimitNs);
+          if (!ok) break;
+          tcgen05_fence_after();
           const uint32_t a_base = smem_u32(smem_a + stage * kABytes);
           const uint32_t b_base = smem_u32(smem_b + stage * kBBytes);
 #pragma unroll
@@ -230,18 +244,15 @@ bsmm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             umma_f16(d_tmem, a_desc, b_desc, idesc, (ks | k) != 0 ? 1u : 0u);
           }
           umma_commit(smem_u32(&empty_bar[stage]));
+          if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
-        __syncwarp();
-        if (++stage == kStages) { stage = 0; phase ^= 1u; }
-      }
-      if (!ok) break;
-      if (lane == 0) {
+        if (!ok) break;
         if (steps > 0) umma_commit(smem_u32(&tmem_full_bar[acc_stage]));
         else mbar_arrive(smem_u32(&tmem_full_bar[acc_stage]));   // a row / column without blocks: zeros
+        if (++acc_stage == 2) { acc_stage = 0; acc_phase ^= 1u; }
       }
-      __syncwarp();
-      if (++acc_stage == 2) { acc_stage = 0; acc_phase ^= 1u; }
     }
+    __syncwarp();
   } else if (warp < kEpilogueWarps) {
     // ======================= epilogue warps ======================================
     const int quarter = warp & 3;
@@ -261,10 +272,10 @@ bsmm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tcgen05_fence_after();
-      const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + acc_stage * kBlock;
+      const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + acc_stage * BN;
       if (rows_ok > 0) {
 #pragma unroll 1
-        for (int ci = half; ci < kBlock / 32; ci += 2) {
+        for (int ci = half; ci < BN / 32; ci += 2) {
           const int col = w.out_col + ci * 32;
           if (col >= p.out_cols) break;
           uint32_t raw[32];
@@ -310,10 +321,11 @@ bsmm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   }
 }
 
-template <typename T, bool A_MN, bool B_MN>
+template <typename T, bool A_MN, bool B_MN, int BN>
 cudaError_t launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const BsmmParams& p, int grid,
                        cudaStream_t stream) {
-  auto kernel = bsmm_kernel<T, A_MN, B_MN>;
+  constexpr int kSmemBytes = Config<BN>::kSmemBytes;
+  auto kernel = bsmm_kernel<T, A_MN, B_MN, BN>;
   static bool configured[64] = {false};
   int dev = 0;
   cudaError_t rc = cudaGetDevice(&dev);

@@ -311,6 +311,8 @@ struct BsmmParams {
   int mode;
   int num_tiles;
   int tiles_inner;             // dsd: column tiles per block row; dds: row tiles per block column
+  int tile_cols;               // columns of an output tile: 128, dsd also 256
+  int idx16;                   // row_indices, column_indices and seg_k point to int16 values
   int K;                       // sdd: dense contraction length
   const int* row_indices;      // sdd: block row of every stored block
   const int* column_indices;   // sdd: block column of every stored block

@@ -835,7 +835,12 @@ at::Tensor bsmm_op(int64_t mode, const at::Tensor& a, bool a_mn, const at::Tenso
   auto check_idx = [](const at::Tensor& t, const char* name) {
     TORCH_CHECK(t.is_cuda() && t.is_contiguous() && t.scalar_type() == at::kInt, name, " must be a contiguous CUDA int32 tensor");
   };
-  check_idx(idx0, "bsmm index 0");
+  // Block indices are read in the type that the topology stores them in.
+  auto check_block_idx = [](const at::Tensor& t, const char* name) {
+    TORCH_CHECK(t.is_cuda() && t.is_contiguous() && (t.scalar_type() == at::kInt || t.scalar_type() == at::kShort), name,
+                " must be a contiguous CUDA int32 or int16 tensor");
+    return t.scalar_type() == at::kShort ? 1 : 0;
+  };
   c10::cuda::CUDAGuard guard(a.device());
   const bool bf16 = a.scalar_type() == at::kBFloat16;
   auto as2d = [](const at::Tensor& t) { return t.dim() == 3 ? t.view({t.size(0) * t.size(1), t.size(2)}) : t; };
@@ -844,11 +849,13 @@ at::Tensor bsmm_op(int64_t mode, const at::Tensor& a, bool a_mn, const at::Tenso
 
   BsmmParams p{};
   p.mode = int(mode);
+  p.tile_cols = int(kBlock);
   p.status = status_word(a.device()).data_ptr<int>();
   at::Tensor out;
   if (mode == kSdd) {
     TORCH_CHECK(idx1.has_value(), "sdd needs row and column indices");
-    check_idx(*idx1, "bsmm index 1");
+    p.idx16 = check_block_idx(idx0, "bsmm index 0");
+    TORCH_CHECK(check_block_idx(*idx1, "bsmm index 1") == p.idx16, "sdd: row and column indices differ in type");
     const int64_t nnz = idx0.numel();
     TORCH_CHECK(idx1->numel() == nnz, "sdd: row and column index arrays differ in length");
     const int64_t ka = a_mn ? a2.size(0) : a2.size(1), kb = b_mn ? b2.size(0) : b2.size(1);
@@ -857,8 +864,8 @@ at::Tensor bsmm_op(int64_t mode, const at::Tensor& a, bool a_mn, const at::Tenso
     TORCH_CHECK(m % kBlock == 0 && n % kBlock == 0, "sdd: output dimensions must be multiples of 128");
     out = at::empty({nnz, kBlock, kBlock}, a.options());
     p.K = int(ka);
-    p.row_indices = idx0.data_ptr<int>();
-    p.column_indices = idx1->data_ptr<int>();
+    p.row_indices = static_cast<const int*>(idx0.data_ptr());
+    p.column_indices = static_cast<const int*>(idx1->data_ptr());
     p.num_tiles = int(nnz);
     p.tiles_inner = 1;
     p.out_ld = kBlock;
@@ -867,7 +874,8 @@ at::Tensor bsmm_op(int64_t mode, const at::Tensor& a, bool a_mn, const at::Tenso
   } else {
     TORCH_CHECK(mode == kDsd || mode == kDds, "bsmm: unknown mode");
     TORCH_CHECK(idx2.has_value(), "dsd / dds need the segment list");
-    check_idx(*idx2, "bsmm index 2");
+    check_idx(idx0, "bsmm index 0");
+    p.idx16 = check_block_idx(*idx2, "bsmm index 2");
     if (idx1.has_value()) check_idx(*idx1, "bsmm index 1");
     const at::Tensor& values = mode == kDsd ? a2 : b2;
     TORCH_CHECK(values.size(1) == kBlock && values.size(0) % kBlock == 0, "bsmm: block values must be [nnz, 128, 128]");
@@ -877,11 +885,16 @@ at::Tensor bsmm_op(int64_t mode, const at::Tensor& a, bool a_mn, const at::Tenso
     const int64_t lists = idx0.numel() - 1;
     p.seg_offsets = idx0.data_ptr<int>();
     p.seg_block = idx1.has_value() ? idx1->data_ptr<int>() : nullptr;
-    p.seg_k = idx2->data_ptr<int>();
+    p.seg_k = static_cast<const int*>(idx2->data_ptr());
     if (mode == kDsd) {
       TORCH_CHECK(lists * kBlock == out_rows, "dsd: one segment list per 128 output rows expected");
       TORCH_CHECK((b_mn ? b2.size(1) : b2.size(0)) == out_cols, "dsd: dense operand does not match the output width");
-      p.tiles_inner = int(ceil_div(out_cols, kBlock));
+      // 256 columns a tile unless that leaves SMs without one: a K step of such a tile loads 48 KB, of two
+      // narrow ones 64, so a wave of wide tiles costs about 1.5 narrow ones.
+      const int64_t narrow = ceil_div(lists * ceil_div(out_cols, kBlock), sm_count());
+      const int64_t wide = ceil_div(lists * ceil_div(out_cols, 256), sm_count());
+      if (out_cols >= 256 && wide * 3 <= narrow * 2) p.tile_cols = 256;
+      p.tiles_inner = int(ceil_div(out_cols, p.tile_cols));
     } else {
       TORCH_CHECK(lists * kBlock == out_cols, "dds: one segment list per 128 output columns expected");
       TORCH_CHECK((a_mn ? a2.size(1) : a2.size(0)) == out_rows, "dds: dense operand does not match the output height");
@@ -895,7 +908,7 @@ at::Tensor bsmm_op(int64_t mode, const at::Tensor& a, bool a_mn, const at::Tenso
   p.out = out.data_ptr();
   if (out.numel() == 0 || p.num_tiles == 0) return out;
   const CUtensorMap ta = make_tensor_map(a2.data_ptr(), bf16, a2.size(0), a2.size(1), a_mn ? 64 : 128);
-  const CUtensorMap tb = make_tensor_map(b2.data_ptr(), bf16, b2.size(0), b2.size(1), b_mn ? 64 : 128);
+  const CUtensorMap tb = make_tensor_map(b2.data_ptr(), bf16, b2.size(0), b2.size(1), b_mn ? 64 : p.tile_cols);
   const int grid = std::max(1, std::min(p.num_tiles, sm_count()));
   MB_CUDA_OK(launch(bf16, a_mn, b_mn, ta, tb, p, grid, stream()));
   MB_LAUNCHED(1);

@@ -194,11 +194,16 @@ def _i32(t: torch.Tensor) -> torch.Tensor:
     return t if t.dtype == torch.int32 and t.is_contiguous() else t.to(torch.int32).contiguous()
 
 
+def _block_index(t: torch.Tensor) -> torch.Tensor:
+    """Block indices as the kernel reads them: int16 or int32, as stored."""
+    return t if t.dtype in (torch.int16, torch.int32) and t.is_contiguous() else _i32(t)
+
+
 def _segments(s: Matrix, transposed_list: bool):
     """Segment list ``(offsets, block position or None, k-block)`` of the rows of ``s`` or of ``s^T``."""
     if transposed_list:
-        return _i32(s.offsets_t), _i32(s.block_offsets_t), _i32(s.column_indices_t)
-    return _i32(s.offsets), None, _i32(s.column_indices)
+        return _i32(s.offsets_t), _i32(s.block_offsets_t), _block_index(s.column_indices_t)
+    return _i32(s.offsets), None, _block_index(s.column_indices)
 
 
 def _sdd_kernel(a: torch.Tensor, b: torch.Tensor, topo: Matrix) -> torch.Tensor:
@@ -206,7 +211,10 @@ def _sdd_kernel(a: torch.Tensor, b: torch.Tensor, topo: Matrix) -> torch.Tensor:
     sa, a_t = _stored(a)
     sb, b_t = _stored(b)
     # a is [M, K]: stored transposed = MN-major.  b is [K, N]: stored as given = MN-major.
-    return ext().bsmm(_MODE_SDD, sa, a_t, sb, not b_t, _i32(topo.row_indices), _i32(topo.column_indices), None, 0, 0)
+    rows, cols = _block_index(topo.row_indices), _block_index(topo.column_indices)
+    if rows.dtype != cols.dtype:
+        rows, cols = _i32(rows), _i32(cols)
+    return ext().bsmm(_MODE_SDD, sa, a_t, sb, not b_t, rows, cols, None, 0, 0)
 
 
 def _dsd_kernel(s: Matrix, data: torch.Tensor, b: torch.Tensor) -> torch.Tensor:

@@ -177,3 +177,23 @@ def test_tensor_core_products_match_fp32(m, k, n, sparsity, dtype):
     close(sparse.to_dense(sparse.with_data(topo, data.grad)), d4.grad * mask)
     from megablocks_b200.utils import status
     status.check()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('cols', [128, 248, 256, 520, 1024])
+@pytest.mark.parametrize('rows', [256, 2560])
+@pytest.mark.parametrize('index', [torch.int16, torch.int32])
+def test_dsd_tile_widths_and_index_types(rows, cols, index):
+    """Wide and narrow dense tiles (whole, ragged and single), empty block rows and both index types, plain
+    and transposed, against the fp32 products of the dense matrices."""
+    torch.manual_seed(rows + cols)
+    topo = sparse.random_mask(rows, 1280, 0.7, 128, device='cuda', dtype=torch.bfloat16)
+    topo = sparse.Matrix(topo._size, torch.randn_like(topo.data) * 0.1, topo.row_indices.to(index),
+                         topo.column_indices.to(index), topo.offsets)
+    dense = topo.to_dense().float()
+    for m, d in ((topo, dense), (topo.t(), dense.t())):
+        b = torch.randn(d.shape[1], cols, device='cuda').bfloat16()
+        for rhs in (b, b.t().contiguous().t()):
+            got, want = sparse.dsd(m, rhs).float(), d @ b.float()
+            # One rounding of the result and fp32 sums in another order.
+            torch.testing.assert_close(got, want, rtol=2 ** -8, atol=2 ** -8 * float(want.abs().max()))
