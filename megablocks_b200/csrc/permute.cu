@@ -128,22 +128,33 @@ __global__ void inverse_map_kernel(const int* __restrict__ indices, const int* _
 }
 
 // out[t] = sum_s weight[t*k+s] * x[inverse[t*k+s]] [+ bias]  (fp32 accumulate, one rounding).
-// Bound by memory (k rows read, one written per token).  The layer's output bias rides along here: as
-// an elementwise add of its own it read and wrote the whole output again with a broadcast operand that
-// the library does not vectorise (56 us for 32768 x 768 bf16, 80 us for 65536 x 512 fp16; this kernel
-// itself takes 15 / 21 us either way).
-template <typename T, int VEC>
+// Bound by memory: k rows read, one written per token.
+//   SINGLE (top-1): a plain loop over the row at full occupancy is at the bandwidth (32768 x 768 bf16 in
+//   14.4 us, 100 MB); four pieces in flight per lane cost it 96 registers and twice the time.  Rows are
+//   cut into slices only while there are too few tokens to fill the SMs.
+//   Otherwise a warp takes one slice of kCombineChunks x 32 lanes x 16 bytes and loads it of two copies
+//   before it uses either: a whole row per warp, one load at a time, took 13.6 us for 16 tokens x 4096 x
+//   top-2 and 24.8 for 2047, a slice 2.7 and 12.6.
+// The layer's output bias rides along here: as an elementwise add of its own it read and wrote the whole
+// output again with a broadcast operand that the library does not vectorise (56 us for 32768 x 768 bf16,
+// 80 us for 65536 x 512 fp16).
+constexpr int kCombineChunks = 2;
+
+template <typename T, int VEC, bool SINGLE>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 combine_rows_kernel(const T* __restrict__ x, const int* __restrict__ inverse, const T* __restrict__ weights,
-                    const T* __restrict__ bias, int top_k, int64_t tokens, int cols, T* __restrict__ out) {
+                    const T* __restrict__ bias, int top_k, int64_t tokens, int cols, int slice_cols,
+                    T* __restrict__ out) {
   const int lane = threadIdx.x & 31;
   const int64_t t = int64_t(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
   if (t >= tokens) return;
+  const int begin = blockIdx.y * slice_cols;
+  const int end = min(cols, begin + slice_cols);
   T* dst = out + t * cols;
-  if (top_k == 1) {
+  if constexpr (SINGLE) {
     const int row = __ldg(inverse + t);
     const float w = (weights != nullptr) ? to_float(weights[t]) : 1.f;
-    for (int c = lane * VEC; c < cols; c += 32 * VEC) {
+    for (int c = begin + lane * VEC; c < end; c += 32 * VEC) {
       Pack<T, VEC> p;
       if (row >= 0) {
         p = load_pack<T, VEC>(x + int64_t(row) * cols + c);
@@ -162,32 +173,56 @@ combine_rows_kernel(const T* __restrict__ x, const int* __restrict__ inverse, co
       }
       store_pack<T, VEC>(dst + c, p);
     }
-    return;
-  }
-  for (int c = lane * VEC; c < cols; c += 32 * VEC) {
-    float acc[VEC];
+  } else {
+    for (int c0 = begin + lane * VEC; c0 < end; c0 += kCombineChunks * 32 * VEC) {
+      float acc[kCombineChunks][VEC];
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) acc[i] = 0.f;
-    for (int s = 0; s < top_k; ++s) {
-      const int64_t copy = t * top_k + s;
-      const int row = __ldg(inverse + copy);
-      if (row < 0) continue;
-      const float w = (weights != nullptr) ? to_float(weights[copy]) : 1.f;
-      Pack<T, VEC> p = load_pack<T, VEC>(x + int64_t(row) * cols + c);
-      // Each product is rounded to T before the sum, as when the k scaled copies
-      // are first stored and then added.
+      for (int j = 0; j < kCombineChunks; ++j)
 #pragma unroll
-      for (int i = 0; i < VEC; ++i) acc[i] += to_float(from_float<T>(to_float(p.v[i]) * w));
+        for (int i = 0; i < VEC; ++i) acc[j][i] = 0.f;
+      for (int s = 0; s < top_k; s += 2) {
+        int row[2];
+        float w[2];
+        Pack<T, VEC> p[2][kCombineChunks];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int64_t copy = t * top_k + s + u;
+          row[u] = s + u < top_k ? __ldg(inverse + copy) : -1;
+          w[u] = (weights != nullptr && s + u < top_k) ? to_float(weights[copy]) : 1.f;
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int j = 0; j < kCombineChunks; ++j) {
+            const int c = c0 + j * 32 * VEC;
+            if (row[u] >= 0 && c < end) p[u][j] = load_pack<T, VEC>(x + int64_t(row[u]) * cols + c);
+          }
+        // Each product is rounded to T before the sum, as when the k scaled copies are first stored and
+        // then added.
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int j = 0; j < kCombineChunks; ++j) {
+            if (row[u] < 0 || c0 + j * 32 * VEC >= end) continue;
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) acc[j][i] += to_float(from_float<T>(to_float(p[u][j].v[i]) * w[u]));
+          }
+      }
+#pragma unroll
+      for (int j = 0; j < kCombineChunks; ++j) {
+        const int c = c0 + j * 32 * VEC;
+        if (c >= end) break;
+        if (bias != nullptr) {
+          const Pack<T, VEC> b = load_pack<T, VEC>(bias + c);
+#pragma unroll
+          for (int i = 0; i < VEC; ++i) acc[j][i] += to_float(b.v[i]);
+        }
+        Pack<T, VEC> o;
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) o.v[i] = from_float<T>(acc[j][i]);
+        store_pack<T, VEC>(dst + c, o);
+      }
     }
-    if (bias != nullptr) {
-      const Pack<T, VEC> b = load_pack<T, VEC>(bias + c);
-#pragma unroll
-      for (int i = 0; i < VEC; ++i) acc[i] += to_float(b.v[i]);
-    }
-    Pack<T, VEC> o;
-#pragma unroll
-    for (int i = 0; i < VEC; ++i) o.v[i] = from_float<T>(acc[i]);
-    store_pack<T, VEC>(dst + c, o);
   }
 }
 
@@ -319,20 +354,28 @@ cudaError_t inverse_map(const int* indices, const int* bins, const int* padded_b
 
 cudaError_t combine_rows(DType type, const void* x, const int* inverse, const void* weights, const void* bias,
                          int top_k, int64_t tokens, int cols, void* out, cudaStream_t stream) {
-  const int grid = ceil_div(tokens, kWarpsPerCta);
+  if (tokens == 0 || cols == 0) return cudaSuccess;
   MB_SWITCH_FLOAT(type, T, {
     constexpr int kFull = 16 / sizeof(T);
-    if (vec_width<T>(cols, x, out) > 1 && reinterpret_cast<uintptr_t>(bias) % 16 == 0) {
-      combine_rows_kernel<T, kFull><<<grid, kWarpsPerCta * 32, 0, stream>>>(
-          static_cast<const T*>(x), inverse, static_cast<const T*>(weights), static_cast<const T*>(bias),
-          top_k, tokens, cols,
-          static_cast<T*>(out));
-    } else {
-      combine_rows_kernel<T, 1><<<grid, kWarpsPerCta * 32, 0, stream>>>(
-          static_cast<const T*>(x), inverse, static_cast<const T*>(weights), static_cast<const T*>(bias),
-          top_k, tokens, cols,
-          static_cast<T*>(out));
-    }
+    const bool wide = vec_width<T>(cols, x, out) > 1 && reinterpret_cast<uintptr_t>(bias) % 16 == 0;
+    const bool single = top_k == 1;
+    const int step = (single ? 1 : kCombineChunks) * 32 * (wide ? kFull : 1);
+    const int steps = ceil_div(cols, step);
+    // Top-1: slices enough for 64 warps on each of 148 SMs.  Otherwise one step a warp.
+    const int64_t wanted = (148 * 64 + tokens - 1) / tokens;
+    int per_slice = single ? ceil_div(steps, wanted < steps ? static_cast<int>(wanted) : steps) : 1;
+    per_slice = max(per_slice, ceil_div(steps, 65535));       // the grid's limit
+    const int slices = ceil_div(steps, per_slice);
+    const dim3 grid(ceil_div(tokens, kWarpsPerCta), slices);
+    auto run = [&](auto kernel) {
+      kernel<<<grid, kWarpsPerCta * 32, 0, stream>>>(
+          static_cast<const T*>(x), inverse, static_cast<const T*>(weights), static_cast<const T*>(bias), top_k, tokens,
+          cols, per_slice * step, static_cast<T*>(out));
+    };
+    if (wide && single) run(combine_rows_kernel<T, kFull, true>);
+    else if (wide) run(combine_rows_kernel<T, kFull, false>);
+    else if (single) run(combine_rows_kernel<T, 1, true>);
+    else run(combine_rows_kernel<T, 1, false>);
   })
   return cudaGetLastError();
 }
