@@ -57,6 +57,9 @@ std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, c
                                      const c10::optional<at::Tensor>& a2, const c10::optional<at::Tensor>& b2,
                                      const c10::optional<at::Tensor>& sqnorm,
                                      const c10::optional<at::Tensor>& seq_base);
+std::vector<at::Tensor> route_plan_rows(const at::Tensor& top_experts, int64_t num_experts, int64_t block,
+                                        int64_t capacity);
+
 // expert_block.cpp
 std::vector<at::Tensor> expert_block_forward(const at::Tensor& x, const at::Tensor& top_experts,
                                              const at::Tensor& weights, const at::Tensor& w1, const at::Tensor& w2,
@@ -64,7 +67,7 @@ std::vector<at::Tensor> expert_block_forward(const at::Tensor& x, const at::Tens
                                              const c10::optional<at::Tensor>& gemm_bins, int64_t num_experts,
                                              int64_t top_k, int64_t act, int64_t capacity, bool save, int64_t pair);
 std::vector<at::Tensor> expert_block_backward(
-    const at::Tensor& dout, const at::Tensor& indices, const at::Tensor& bin_ids, const at::Tensor& bins,
+    const at::Tensor& dout, const at::Tensor& indices, const at::Tensor& inverse, const at::Tensor& bins,
     const c10::optional<at::Tensor>& gemm_bins, const at::Tensor& rows, const at::Tensor& y, const at::Tensor& z1,
     const c10::optional<at::Tensor>& z2, const c10::optional<at::Tensor>& h_in, const at::Tensor& weights,
     const at::Tensor& w1, const at::Tensor& w2, const c10::optional<at::Tensor>& v1, const std::vector<bool>& needs,
@@ -142,6 +145,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.doc() = "megablocks_b200 sm_100a kernels";
   m.def("sort_pairs", &mb::sort_pairs);
   m.def("route_plan", &mb::route_plan);
+  m.def("route_plan_rows", &mb::route_plan_rows);
   m.def("histogram", &mb::histogram_op);
   m.def("cumsum", &mb::cumsum_op);
   m.def("topology", &mb::topology_op);

@@ -15,17 +15,15 @@ namespace mb {
 
 using OptTensor = c10::optional<at::Tensor>;
 
-std::vector<at::Tensor> route_plan(const at::Tensor& top_experts, int64_t num_experts, int64_t block);
+std::vector<at::Tensor> route_plan_rows(const at::Tensor& top_experts, int64_t num_experts, int64_t block,
+                                        int64_t capacity);
+at::Tensor combine_rows_op(const at::Tensor& x, const at::Tensor& inverse, const OptTensor& weights, int64_t top_k,
+                           int64_t tokens, const OptTensor& bias);
 at::Tensor gather_rows_op(const at::Tensor& x, const at::Tensor& indices, const at::Tensor& bin_ids,
                           const OptTensor& weights, const at::Tensor& bins, const at::Tensor& padded_bins,
                           int64_t top_k, int64_t out_rows);
 at::Tensor binned_gather_rows(const at::Tensor& x, const at::Tensor& indices, const OptTensor& weights,
                               const at::Tensor& bins, int64_t capacity, int64_t top_k);
-at::Tensor scatter_rows_op(const at::Tensor& x, const at::Tensor& indices, const at::Tensor& bin_ids,
-                           const OptTensor& weights, const at::Tensor& bins, const at::Tensor& padded_bins,
-                           int64_t top_k, int64_t tokens, const OptTensor& bias);
-at::Tensor binned_scatter_rows(const at::Tensor& x, const at::Tensor& indices, const OptTensor& weights,
-                               const at::Tensor& bins, int64_t top_k, int64_t tokens, const OptTensor& bias);
 std::vector<at::Tensor> scatter_backward_op(const at::Tensor& x, const at::Tensor& grad, const at::Tensor& indices,
                                             const at::Tensor& weights, const at::Tensor& bins,
                                             const OptTensor& padded_bins, int64_t top_k);
@@ -58,15 +56,15 @@ at::Tensor rows_of(const at::Tensor& t) { return t.dim() == 3 ? t.view({-1, t.si
 
 }  // namespace
 
-// {out, tokens_per_expert} or, with `save`, also {indices, bin_ids, bins, x rows, y rows, z1, z2, h}
+// {out, tokens_per_expert} or, with `save`, also {indices, inverse, bins, x rows, y rows, z1, z2, h}
 // (z2 undefined for the MLP).
 std::vector<at::Tensor> expert_block_forward(const at::Tensor& x, const at::Tensor& top_experts,
                                              const at::Tensor& weights, const at::Tensor& w1, const at::Tensor& w2,
                                              const OptTensor& v1, const OptTensor& bias, const OptTensor& gemm_bins,
                                              int64_t num_experts, int64_t top_k, int64_t act, int64_t capacity, bool save,
                                              int64_t pair) {
-  const auto plan = route_plan(top_experts, num_experts, 128);
-  const at::Tensor &indices = plan[0], &bin_ids = plan[1], &bins = plan[2];
+  const auto plan = route_plan_rows(top_experts, num_experts, 128, capacity);
+  const at::Tensor &indices = plan[0], &bin_ids = plan[1], &bins = plan[2], &inverse = plan[5];
   const bool binned = capacity > 0;
   TORCH_CHECK(!binned || (gemm_bins.has_value() && !v1.has_value()), "capacity layout: uniform bins, no gate weight");
   const int64_t tokens = x.size(0);
@@ -88,21 +86,16 @@ std::vector<at::Tensor> expert_block_forward(const at::Tensor& x, const at::Tens
     z1 = o[0]; h = o[1];
   }
   at::Tensor y = Gemm{}.run(h, w2, groups, pair)[0];
-  at::Tensor out;
-  if (binned) {
-    y = y.view({num_experts, capacity, -1});
-    out = binned_scatter_rows(y, indices, weights, bins, top_k, tokens, bias);
-  } else {
-    out = scatter_rows_op(y, indices, bin_ids, weights, bins, bins, top_k, tokens, bias);
-  }
+  at::Tensor out = combine_rows_op(y, inverse, weights, top_k, tokens, bias);
   if (!save) return {out, plan[4]};
-  return {out, plan[4], indices, bin_ids, bins, rows, y, z1, z2, h};
+  if (binned) y = y.view({num_experts, capacity, -1});
+  return {out, plan[4], indices, inverse, bins, rows, y, z1, z2, h};
 }
 
 // {dx, dweights, dw1, dw2, dv1, dbias}, undefined where `needs` says so.  `slots`: per weight gradient
 // (w1, w2, v1) an optional accumulator of its squared norm.
 std::vector<at::Tensor> expert_block_backward(const at::Tensor& dout, const at::Tensor& indices,
-                                              const at::Tensor& bin_ids, const at::Tensor& bins,
+                                              const at::Tensor& inverse, const at::Tensor& bins,
                                               const OptTensor& gemm_bins, const at::Tensor& rows, const at::Tensor& y,
                                               const at::Tensor& z1, const OptTensor& z2, const OptTensor& h_in,
                                               const at::Tensor& weights, const at::Tensor& w1, const at::Tensor& w2,
@@ -155,8 +148,7 @@ std::vector<at::Tensor> expert_block_backward(const at::Tensor& dout, const at::
       in.b2 = v1;
     }
     at::Tensor d = in.run(dz1, w1, groups, pair)[0];
-    dx = binned ? binned_scatter_rows(d.view({groups.numel(), capacity, -1}), indices, {}, bins, top_k, tokens, {})
-                : scatter_rows_op(d, indices, bin_ids, {}, bins, bins, top_k, tokens, {});
+    dx = combine_rows_op(d, inverse, {}, top_k, tokens, {});
   }
   return {dx, dweights, dw1, dw2, dv1, dbias};
 }

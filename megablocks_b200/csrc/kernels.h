@@ -27,14 +27,16 @@ cudaError_t sort_pass(DType key_type, const void* keys, const void* vals_in, int
                       void* vals_out, int* tpe, int* bins, int* padded_bins, int num_real_bins, int block,
                       cudaStream_t stream);
 // Route plan of at most kPlanMaxCopies copies over at most kPlanMaxBins experts in one launch; ids are
-// int64 (`keys64`) or int32.
+// int64 (`keys64`) or int32.  `inverse` (nullable): row of every copy, in expert order (capacity <= 0)
+// or among [experts, capacity] slots, -1 when dropped.
 constexpr int kPlanMaxBins = 256;
 constexpr int kPlanMaxCopies = 4096;
 cudaError_t route_plan_small(bool keys64, const void* keys, int n, int bits, int num_experts, int block, int* indices,
-                             int* bin_ids, int* bins, int* padded_bins, int* tpe, cudaStream_t stream);
+                             int* bin_ids, int* bins, int* padded_bins, int* tpe, int* inverse, int capacity,
+                             cudaStream_t stream);
 cudaError_t route_sort64(const int64_t* keys, int64_t n, int bits, int chunk, int num_chunks, int* partial, int* totals,
                          int* bin_ids, int* indices, int* tpe, int* bins, int* padded_bins, int num_experts, int block,
-                         cudaStream_t stream);
+                         int* inverse, int capacity, cudaStream_t stream);
 cudaError_t histogram(DType type, const void* x, int64_t batch, int64_t n, int num_bins, int* out_zeroed,
                       int sms, cudaStream_t stream);
 cudaError_t cumsum(DType type, const void* x, void* out, int64_t rows, int64_t cols, bool exclusive,

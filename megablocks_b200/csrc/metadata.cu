@@ -125,6 +125,15 @@ __device__ void block_scan_totals(const int* __restrict__ totals, int nbins, int
   __syncthreads();
 }
 
+// Row of the copy at sorted position `pos` of bin d: the position itself, or (capacity > 0) its slot of the
+// bin's `capacity` slots, -1 past them.  The plan knows it where it places the copy; the un-permutation
+// would otherwise search it again with a launch of its own, forward and backward.
+__device__ __forceinline__ int row_of_copy(int pos, int bin_start, int d, int capacity) {
+  if (capacity <= 0) return pos;
+  const int off = pos - bin_start;
+  return off < capacity ? d * capacity + off : -1;
+}
+
 // Pass 3: stable placement.  Optionally (route plan) CTA 0 also writes the
 // per-bin totals, their inclusive prefix sums and the block-padded prefix sums.
 template <typename K, typename KO, typename V>
@@ -133,7 +142,7 @@ sort_place_kernel(const K* __restrict__ keys, const V* __restrict__ vals_in, int
                   bool flip_sign, int chunk, int num_chunks, const int* __restrict__ partial,
                   const int* __restrict__ totals, KO* __restrict__ keys_out, V* __restrict__ vals_out,
                   int* __restrict__ tpe_out, int* __restrict__ bins_out, int* __restrict__ padded_bins_out,
-                  int num_real_bins, int block) {
+                  int num_real_bins, int block, int* __restrict__ inverse, int capacity) {
   extern __shared__ int smem[];
   const int nbins = 1 << bits;
   int* bin_base = smem;                       // [nbins]
@@ -175,6 +184,7 @@ sort_place_kernel(const K* __restrict__ keys, const V* __restrict__ vals_in, int
     if (valid) {
       keys_out[pos] = static_cast<KO>(key);
       vals_out[pos] = vals_in != nullptr ? vals_in[i] : static_cast<V>(i);
+      if (inverse != nullptr) inverse[i] = row_of_copy(pos, bin_base[d], d, capacity);
     }
   }
 }
@@ -194,7 +204,8 @@ template <typename K>
 __global__ void __launch_bounds__(kPlanThreads)
 route_plan_small_kernel(const K* __restrict__ keys, int n, int bits, int num_experts, int block,
                         int* __restrict__ indices, int* __restrict__ bin_ids, int* __restrict__ bins,
-                        int* __restrict__ padded_bins, int* __restrict__ tpe) {
+                        int* __restrict__ padded_bins, int* __restrict__ tpe, int* __restrict__ inverse, int capacity) {
+  __shared__ int bin_start[kPlanMaxBins];
   __shared__ int cursor[kPlanWarps * kPlanMaxBins];     // [warp][bin]
   __shared__ int warp_sums[2 * kPlanWarps];
   const int nbins = 1 << bits;                          // <= kPlanMaxBins <= kPlanThreads
@@ -228,6 +239,7 @@ route_plan_small_kernel(const K* __restrict__ keys, int n, int bits, int num_exp
       padded_bins[b] = incl_p;
     }
     int at = incl - total;                              // first position of (warp, bin)
+    bin_start[b] = at;
     for (int w = 0; w < kPlanWarps; ++w) {
       const int count = cursor[w * kPlanMaxBins + b];
       cursor[w * kPlanMaxBins + b] = at;
@@ -250,6 +262,7 @@ route_plan_small_kernel(const K* __restrict__ keys, int n, int bits, int num_exp
     if (valid) {
       bin_ids[pos] = key;
       indices[pos] = i;
+      if (inverse != nullptr) inverse[i] = row_of_copy(pos, bin_start[d], d, capacity);
     }
   }
 }
@@ -257,15 +270,17 @@ route_plan_small_kernel(const K* __restrict__ keys, int n, int bits, int num_exp
 }  // namespace
 
 cudaError_t route_plan_small(bool keys64, const void* keys, int n, int bits, int num_experts, int block, int* indices,
-                             int* bin_ids, int* bins, int* padded_bins, int* tpe, cudaStream_t stream) {
+                             int* bin_ids, int* bins, int* padded_bins, int* tpe, int* inverse, int capacity,
+                             cudaStream_t stream) {
   if (n < 1 || bits < 1 || (1 << bits) > kPlanMaxBins || num_experts > (1 << bits)) return cudaErrorInvalidValue;
   if (keys64)
     route_plan_small_kernel<int64_t><<<1, kPlanThreads, 0, stream>>>(static_cast<const int64_t*>(keys), n, bits,
                                                                      num_experts, block, indices, bin_ids, bins,
-                                                                     padded_bins, tpe);
+                                                                     padded_bins, tpe, inverse, capacity);
   else
     route_plan_small_kernel<int><<<1, kPlanThreads, 0, stream>>>(static_cast<const int*>(keys), n, bits, num_experts,
-                                                                 block, indices, bin_ids, bins, padded_bins, tpe);
+                                                                 block, indices, bin_ids, bins, padded_bins, tpe,
+                                                                 inverse, capacity);
   return cudaGetLastError();
 }
 
@@ -287,7 +302,7 @@ cudaError_t sort_pass(DType key_type, const void* keys, const void* vals_in, int
     sort_place_kernel<K, K, K><<<grid, kSortThreads, place_smem, stream>>>(
         static_cast<const K*>(keys), static_cast<const K*>(vals_in), n, shift, bits, flip_sign, chunk, num_chunks,
         partial, totals, static_cast<K*>(keys_out), static_cast<K*>(vals_out), tpe, bins, padded_bins,
-        num_real_bins, block);
+        num_real_bins, block, nullptr, 0);
   })
   return cudaGetLastError();
 }
@@ -296,7 +311,7 @@ cudaError_t sort_pass(DType key_type, const void* keys, const void* vals_in, int
 // narrowed copy of the ids is made first.
 cudaError_t route_sort64(const int64_t* keys, int64_t n, int bits, int chunk, int num_chunks, int* partial, int* totals,
                          int* bin_ids, int* indices, int* tpe, int* bins, int* padded_bins, int num_experts, int block,
-                         cudaStream_t stream) {
+                         int* inverse, int capacity, cudaStream_t stream) {
   const int nbins = 1 << bits;
   const int grid = ceil_div(num_chunks, kSortWarps);
   sort_hist_kernel<int64_t><<<grid, kSortThreads, size_t(kSortWarps) * nbins * sizeof(int), stream>>>(
@@ -305,7 +320,7 @@ cudaError_t route_sort64(const int64_t* keys, int64_t n, int bits, int chunk, in
   sort_place_kernel<int64_t, int, int>
       <<<grid, kSortThreads, size_t(nbins + 8 + kSortWarps * nbins) * sizeof(int), stream>>>(
           keys, nullptr, n, 0, bits, false, chunk, num_chunks, partial, totals, bin_ids, indices, tpe, bins, padded_bins,
-          num_experts, block);
+          num_experts, block, inverse, capacity);
   return cudaGetLastError();
 }
 

@@ -149,12 +149,16 @@ std::vector<at::Tensor> sort_pairs(const at::Tensor& x, int64_t end_bit) {
   return {keys_a, vals_a};
 }
 
-std::vector<at::Tensor> route_plan(const at::Tensor& top_experts, int64_t num_experts, int64_t block) {
+// With `inverse` given, it becomes the copies' rows (see route_plan_small) where the path can give them,
+// and stays undefined otherwise.
+static std::vector<at::Tensor> route_plan_impl(const at::Tensor& top_experts, int64_t num_experts, int64_t block,
+                                               at::Tensor* inverse, int64_t capacity) {
   MB_CHECK_CUDA(top_experts); MB_CHECK_CONTIG(top_experts);
   TORCH_CHECK(top_experts.dim() == 1, "route_plan expects flattened expert ids");
   TORCH_CHECK(num_experts >= 1 && block >= 1, "bad route_plan arguments");
   c10::cuda::CUDAGuard guard(top_experts.device());
   const int64_t n = top_experts.numel();
+  TORCH_CHECK(capacity <= 0 || num_experts * capacity <= 0x7fffffff, "route_plan: too many slots");
   auto iopts = top_experts.options().dtype(at::kInt);
   at::Tensor indices = at::empty({n}, iopts), bin_ids = at::empty({n}, iopts);
   if (n == 0) {
@@ -164,22 +168,30 @@ std::vector<at::Tensor> route_plan(const at::Tensor& top_experts, int64_t num_ex
   // The scan kernel of the sort writes all three per-expert arrays in full.
   at::Tensor bins = at::empty({num_experts}, iopts), padded_bins = at::empty({num_experts}, iopts);
   at::Tensor tpe = at::empty({num_experts}, iopts);
+  int* rows = nullptr;
+  auto want_rows = [&] {
+    if (inverse == nullptr) return;
+    *inverse = at::empty({n}, iopts);
+    rows = inverse->data_ptr<int>();
+  };
   const bool ids64 = top_experts.scalar_type() == at::kLong;      // what top-k yields: read as they are
   if (n <= kPlanMaxCopies && (1 << bits_for(num_experts)) <= kPlanMaxBins &&
       (ids64 || top_experts.scalar_type() == at::kInt)) {
+    want_rows();
     MB_CUDA_OK(route_plan_small(ids64, top_experts.data_ptr(), int(n), bits_for(num_experts), int(num_experts),
                                 int(block), indices.data_ptr<int>(), bin_ids.data_ptr<int>(), bins.data_ptr<int>(),
-                                padded_bins.data_ptr<int>(), tpe.data_ptr<int>(), stream()));
+                                padded_bins.data_ptr<int>(), tpe.data_ptr<int>(), rows, int(capacity), stream()));
     MB_LAUNCHED(1);
     return {indices, bin_ids, bins, padded_bins, tpe};
   }
   if (ids64 && num_experts <= kMaxSortBins) {
     const int bits = bits_for(num_experts);
     SortScratch s = make_scratch(n, 1 << bits, top_experts.options(), route_warp_chunk(n));
+    want_rows();
     MB_CUDA_OK(route_sort64(top_experts.data_ptr<int64_t>(), n, bits, s.chunk, s.num_chunks, s.partial.data_ptr<int>(),
                             s.totals.data_ptr<int>(), bin_ids.data_ptr<int>(), indices.data_ptr<int>(),
                             tpe.data_ptr<int>(), bins.data_ptr<int>(), padded_bins.data_ptr<int>(), int(num_experts),
-                            int(block), stream()));
+                            int(block), rows, int(capacity), stream()));
     MB_LAUNCHED(3);
     return {indices, bin_ids, bins, padded_bins, tpe};
   }
@@ -200,6 +212,38 @@ std::vector<at::Tensor> route_plan(const at::Tensor& top_experts, int64_t num_ex
   at::Tensor counts = at::bincount(e32, {}, num_experts).to(at::kInt);
   at::Tensor padded = at::floor_divide(counts + (block - 1), block) * block;
   return {sorted[1], sorted[0], at::cumsum(counts, 0).to(at::kInt), at::cumsum(padded, 0).to(at::kInt), counts};
+}
+
+std::vector<at::Tensor> route_plan(const at::Tensor& top_experts, int64_t num_experts, int64_t block) {
+  return route_plan_impl(top_experts, num_experts, block, nullptr, 0);
+}
+
+// The plan and, as a sixth tensor, the row of every copy: in expert order (capacity <= 0) or among
+// [experts, capacity] slots, -1 for a dropped copy.
+std::vector<at::Tensor> route_plan_rows(const at::Tensor& top_experts, int64_t num_experts, int64_t block,
+                                        int64_t capacity) {
+  at::Tensor inverse;
+  auto plan = route_plan_impl(top_experts, num_experts, block, &inverse, capacity);
+  if (!inverse.defined()) inverse = build_inverse(plan[0], plan[2], plan[2], capacity > 0 ? int(capacity) : -1);
+  plan.push_back(inverse);
+  return plan;
+}
+
+// out[t] = sum of the rows of token t's copies (weighted, plus bias); `inverse` as above.
+at::Tensor combine_rows_op(const at::Tensor& x, const at::Tensor& inverse, const c10::optional<at::Tensor>& weights,
+                           int64_t top_k, int64_t tokens, const c10::optional<at::Tensor>& bias) {
+  MB_CHECK_CUDA(x); MB_CHECK_CONTIG(x);
+  TORCH_CHECK(x.dim() == 2, "combine expects x[rows, hidden]");
+  check_index(inverse, "inverse");
+  TORCH_CHECK(inverse.numel() == tokens * top_k, "one row per copy expected");
+  check_weights(weights, x, inverse.numel());
+  c10::cuda::CUDAGuard guard(x.device());
+  at::Tensor out = at::empty({tokens, x.size(1)}, x.options());
+  if (out.numel() == 0) return out;
+  MB_CUDA_OK(combine_rows(float_code(x.scalar_type()), x.data_ptr(), inverse.data_ptr<int>(), opt_ptr(weights),
+                          opt_ptr(bias), int(top_k), tokens, int(x.size(1)), out.data_ptr(), stream()));
+  MB_LAUNCHED(1);
+  return out;
 }
 
 // ---------------------------------------------------------------------------

@@ -27,17 +27,20 @@ class _ExpertBlock(torch.autograd.Function):
     @staticmethod
     def forward(ctx: Any, x, weights, top_experts, w1, w2, v1, bias, gemm_bins, num_experts, top_k, act, capacity,
                 memory_optimized, wgrad_scale):
-        out, counts, indices, bin_ids, bins, rows, y, z1, z2, h = ext().expert_block_forward(
+        out, counts, indices, inverse, bins, rows, y, z1, z2, h = ext().expert_block_forward(
             x, top_experts, weights, w1, w2, v1, bias, gemm_bins, num_experts, top_k, act, capacity, True, G._PAIR_MODE)
-        ctx.save_for_backward(weights, w1, w2, v1, gemm_bins, indices, bin_ids, bins, rows, y, z1,
+        ctx.save_for_backward(weights, w1, w2, v1, gemm_bins, indices, inverse, bins, rows, y, z1,
                               z2 if v1 is not None else None, None if memory_optimized else h)
         ctx.top_k, ctx.act, ctx.capacity, ctx.wgrad_scale = top_k, act, capacity, wgrad_scale
         ctx.mark_non_differentiable(counts)
+        ctx.set_materialize_grads(False)        # no zero tensor for the counts
         return out, counts
 
     @staticmethod
     def backward(ctx: Any, dout, _dcounts):
-        weights, w1, w2, v1, gemm_bins, indices, bin_ids, bins, rows, y, z1, z2, h = ctx.saved_tensors
+        weights, w1, w2, v1, gemm_bins, indices, inverse, bins, rows, y, z1, z2, h = ctx.saved_tensors
+        if dout is None:
+            return (None,) * 14
         need = ctx.needs_input_grad
         needs = [need[0], need[1], need[3], need[4], need[5], need[6]]
         sink = G._GRAD_NORM_SINK
@@ -47,7 +50,7 @@ class _ExpertBlock(torch.autograd.Function):
             for k, (slot, view) in zip(wanted, sink.reserve(len(wanted))):
                 slots[k], views[k] = slot, view
         dx, dweights, *dw, dbias = ext().expert_block_backward(
-            dout.contiguous(), indices, bin_ids, bins, gemm_bins, rows, y, z1, z2, h, weights, w1, w2, v1, needs, views,
+            dout.contiguous(), indices, inverse, bins, gemm_bins, rows, y, z1, z2, h, weights, w1, w2, v1, needs, views,
             ctx.top_k, ctx.act, ctx.wgrad_scale, ctx.capacity, G._PAIR_MODE)
         for k in (1, 0, 2):
             if slots[k] is not None:
@@ -60,7 +63,7 @@ def _hooked(module: torch.nn.Module) -> bool:
                 or module._backward_pre_hooks or 'forward' in module.__dict__)
 
 
-def _special_mode() -> bool:
+def special_mode() -> bool:
     """A mode in which calling the kernels without (or with another) autograd node would change a result."""
     return (torch.is_autocast_enabled('cuda') or torch.jit.is_tracing() or forward_ad._current_level >= 0
             or torch._C._functorch.peek_interpreter_stack() is not None or debug.enabled()
@@ -82,7 +85,7 @@ def route(x, expert_weights, top_experts, mlp, w1, w2, v1, bias, activation_fn) 
             or hidden != x.shape[-1] or top_experts.numel() != expert_weights.numel()
             or (bias is not None and bias.data_ptr() % 16)):
         return False
-    return G.activation_id(activation_fn) is not None and not _hooked(mlp) and not _special_mode()
+    return G.activation_id(activation_fn) is not None and not _hooked(mlp) and not special_mode()
 
 
 def expert_block(x, expert_weights, top_experts, w1, w2, v1, bias, gemm_bins, num_experts, top_k, activation_fn,

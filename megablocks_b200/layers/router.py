@@ -17,7 +17,8 @@ from typing import Any
 
 import torch
 
-from megablocks_b200.layers import common
+from megablocks_b200._ext import ext
+from megablocks_b200.layers import common, expert_block
 from megablocks_b200.layers.arguments import Arguments
 
 _ROUTER_LOGITS = []
@@ -62,23 +63,31 @@ class _UniformExpertAssignment(torch.autograd.Function):
 _uniform_expert_assignment = _UniformExpertAssignment.apply
 
 
+def _fused_top_k(logits: torch.Tensor, top_k: int, norm_p: float):
+    """The fused selection; without its autograd node where nothing is differentiated (a decode step)."""
+    if torch.is_grad_enabled() and logits.requires_grad or expert_block.special_mode():
+        return _FusedTopK.apply(logits, top_k, norm_p)
+    return tuple(ext().router_topk_forward(logits.contiguous(), top_k, norm_p))
+
+
 class _FusedTopK(torch.autograd.Function):
     """softmax -> top-k -> optional p-norm normalisation, one CUDA kernel each way."""
 
     @staticmethod
     def forward(ctx: Any, logits: torch.Tensor, top_k: int, norm_p: float):
-        from megablocks_b200._ext import ext
         scores, weights, experts = ext().router_topk_forward(logits.contiguous(), top_k, float(norm_p))
         ctx.save_for_backward(scores, weights, experts)
         ctx.norm_p = float(norm_p)
         ctx.mark_non_differentiable(experts)
+        ctx.set_materialize_grads(False)        # no zero tensor for the expert ids
         return scores, weights, experts
 
     @staticmethod
     def backward(ctx: Any, dscores, dweights, _dexperts):
-        from megablocks_b200._ext import ext
         scores, weights, experts = ctx.saved_tensors
         if dscores is None:
+            if dweights is None:
+                return None, None, None
             dscores = torch.zeros_like(scores)
         if dweights is None:
             dweights = torch.zeros_like(weights)
@@ -121,7 +130,7 @@ class LearnedRouter(torch.nn.Module):
                     and args.moe_num_experts <= 1024 and args.moe_top_k <= 8
                     and (not norm_p or float(norm_p) in (1.0, 2.0)))
         if fused_ok:
-            return _FusedTopK.apply(logits, args.moe_top_k, float(norm_p) if norm_p else 0.0)
+            return _fused_top_k(logits, args.moe_top_k, float(norm_p) if norm_p else 0.0)
         scores = logits.softmax(dim=-1)
         weights, experts = self._top_k(scores)
         if norm_p:

@@ -436,3 +436,40 @@ def test_router_selection_over_expert_counts(dtype, experts, top_k, norm_p):
     dl, = torch.autograd.grad([out[0], out[1]], leaf, [ds.cuda(), dw.cuda()])
     torch.testing.assert_close(dl.cpu().double(), want, rtol=4 * torch.finfo(dtype).eps + 1e-5,
                                atol=1e-5 + torch.finfo(dtype).eps * float(want.abs().max()))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('experts,copies', [(5, 1), (64, 4096), (64, 5000), (1000, 300), (1200, 50)])
+@pytest.mark.parametrize('capacity', [0, 3])
+def test_plan_gives_the_rows_of_the_copies(experts, copies, capacity):
+    """Rows of the copies from the plan (both its paths, and the search that serves the rest) against the
+    sorted order; dropped copies are -1."""
+    from megablocks_b200._ext import ext
+    torch.manual_seed(copies)
+    top = torch.randint(0, experts, (copies,), device='cuda')
+    indices, bin_ids, bins, _, _, rows = ext().route_plan_rows(top, experts, 128, capacity)
+    want = torch.empty_like(indices)
+    place = torch.arange(copies, device='cuda', dtype=torch.int32)
+    if capacity:
+        first = torch.cat([bins.new_zeros(1), bins[:-1]])[bin_ids.long()]
+        place = torch.where(place - first < capacity, bin_ids * capacity + place - first, -1)
+    want[indices.long()] = place.to(torch.int32)
+    assert torch.equal(rows, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize('top_k', [1, 2, 3, 5])
+@pytest.mark.parametrize('hidden', [8, 100, 512, 520, 1032])
+def test_combine_slices_and_copy_pairs(dtype, top_k, hidden):
+    """Un-permutation over row lengths around a warp's slice and odd numbers of copies, some dropped."""
+    torch.manual_seed(hidden)
+    tokens, experts, capacity = 19, 4, 9
+    top = torch.randint(0, experts, (tokens * top_k,))
+    indices, _, bins, _, _ = ops.route_plan(top, experts)
+    x = torch.randn(experts, capacity, hidden).to(dtype)
+    w = torch.rand(tokens * top_k).to(dtype)
+    got = ops.binned_scatter(x.cuda(), indices.cuda(), w.cuda(), bins.cuda(), top_k)
+    want = ops.binned_scatter(x, indices, w, bins, top_k)
+    # The same products and the same order of the sum: one rounding at most apart.
+    torch.testing.assert_close(got.cpu().float(), want.float(), rtol=torch.finfo(dtype).eps, atol=1e-6)
