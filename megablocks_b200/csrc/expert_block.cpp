@@ -28,14 +28,14 @@ std::vector<at::Tensor> scatter_backward_op(const at::Tensor& x, const at::Tenso
                                             const at::Tensor& weights, const at::Tensor& bins,
                                             const OptTensor& padded_bins, int64_t top_k);
 at::Tensor column_sum_op(const at::Tensor& x);
-std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, const at::Tensor& bins, bool trans_a,
+std::vector<at::Tensor> grouped_gemm_outputs(const at::Tensor& a, const at::Tensor& b, const at::Tensor& bins, bool trans_a,
                                      bool trans_b, int64_t epilogue, int64_t act, const OptTensor& aux1,
                                      const OptTensor& aux2, bool want_out2, bool want_out3, int64_t num_groups,
                                      const OptTensor& c_in, bool zero_tail, const OptTensor& wait_flags,
                                      int64_t wait_count, int64_t wait_stride, int64_t wait_seq, int64_t rows_hint,
                                      int64_t pair_mode, const c10::optional<std::vector<at::Tensor>>& scatter,
                                      const std::vector<int64_t>& scatter_args, double alpha, const OptTensor& a2,
-                                     const OptTensor& b2, const OptTensor& sqnorm, const OptTensor& seq_base);
+                                     const OptTensor& b2, const OptTensor& sqnorm, const OptTensor& seq_base, bool only_out2);
 
 namespace {
 
@@ -43,12 +43,12 @@ struct Gemm {
   bool trans_a = false, trans_b = false;
   int64_t epilogue = gemm::kEpiNone, act = 0;
   OptTensor aux1, aux2, a2, b2, sqnorm;
-  bool want_out2 = true, want_out3 = true;
+  bool want_out2 = true, want_out3 = true, only_out2 = false;
   double alpha = 1.0;
 
   std::vector<at::Tensor> run(const at::Tensor& a, const at::Tensor& b, const at::Tensor& bins, int64_t pair) const {
-    return grouped_gemm(a, b, bins, trans_a, trans_b, epilogue, act, aux1, aux2, want_out2, want_out3, bins.numel(), {},
-                        true, {}, 0, 0, 0, 0, pair, {}, {}, alpha, a2, b2, sqnorm, {});
+    return grouped_gemm_outputs(a, b, bins, trans_a, trans_b, epilogue, act, aux1, aux2, want_out2, want_out3, bins.numel(), {},
+                        true, {}, 0, 0, 0, 0, pair, {}, {}, alpha, a2, b2, sqnorm, {}, only_out2);
   }
 };
 
@@ -75,6 +75,7 @@ std::vector<at::Tensor> expert_block_forward(const at::Tensor& x, const at::Tens
   Gemm up;
   up.trans_b = !binned;
   up.act = act;
+  up.only_out2 = !save;         // the pre-activations are for the backward pass
   if (v1.has_value()) {
     up.epilogue = gemm::kEpiGluDual;
     up.b2 = v1;

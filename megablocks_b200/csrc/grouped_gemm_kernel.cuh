@@ -565,8 +565,10 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&raw)[32], const 
                                         rows_ok, cols, lane, col, maps, tma);
     return;
   }
-  epilogue_emit<T, EPI, ACT, 0, FRAG>(raw, a1, a2, stage, static_cast<T*>(p.c) + base_off, row_stride, rows_ok, cols,
-                                lane, scatter, col, maps, tma);
+  // Without a main output (inference keeps no pre-activations) only the activation is stored.
+  if ((EPI != kEpiAct && EPI != kEpiGlu) || p.c)
+    epilogue_emit<T, EPI, ACT, 0, FRAG>(raw, a1, a2, stage, static_cast<T*>(p.c) + base_off, row_stride, rows_ok, cols,
+                                        lane, scatter, col, maps, tma);
   if constexpr (EPI == kEpiAct || EPI == kEpiDAct || EPI == kEpiGlu || EPI == kEpiDGlu) {
     if (p.out2)
       epilogue_emit<T, EPI, ACT, 1, FRAG>(raw, a1, a2, stage, static_cast<T*>(p.out2) + base_off, row_stride, rows_ok,
@@ -1045,9 +1047,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           if (rows_ok > 0) {
             const int cols = min(32, p.N - col);
             const CUtensorMap* maps = p.store_tma ? p.out_map : nullptr;
-            epilogue_emit<T, kEpiNone, kActIdentity, 0>(raw, z1, unused, stage, static_cast<T*>(p.out3) + row_off + col,
-                                                        p.N, rows_ok, cols, lane, nullptr, col,
-                                                        maps ? maps + 2 : nullptr, tma);
+            if (p.out3)
+              epilogue_emit<T, kEpiNone, kActIdentity, 0>(raw, z1, unused, stage, static_cast<T*>(p.out3) + row_off + col,
+                                                          p.N, rows_ok, cols, lane, nullptr, col,
+                                                          maps ? maps + 2 : nullptr, tma);
             tmem_ld_32x32(taddr + BLOCK_N / 2 + c0, raw);
             tmem_ld_wait();
             epilogue_by_act<T, kEpiGlu>(raw, z1, unused, stage, row_off + col, p.N, rows_ok, cols, lane, p, nullptr, col,
@@ -1184,7 +1187,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       const int64_t stride = int64_t(gridDim.x) * (kEpilogueWarps * 32);
       for (int64_t i = begin + tid * 8; i < end; i += stride * 8) {
         const uint4 z = make_uint4(0, 0, 0, 0);
-        *reinterpret_cast<uint4*>(static_cast<T*>(p.c) + i) = z;
+        if (p.c) *reinterpret_cast<uint4*>(static_cast<T*>(p.c) + i) = z;
         if (p.out2) *reinterpret_cast<uint4*>(static_cast<T*>(p.out2) + i) = z;
         if (p.out3) *reinterpret_cast<uint4*>(static_cast<T*>(p.out3) + i) = z;
       }

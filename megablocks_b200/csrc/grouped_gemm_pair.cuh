@@ -628,7 +628,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       const int64_t stride = int64_t(gridDim.x) * (kPairEpilogueWarps * 32);
       for (int64_t i = begin + tid * 8; i < end; i += stride * 8) {
         const uint4 z = make_uint4(0, 0, 0, 0);
-        *reinterpret_cast<uint4*>(static_cast<T*>(p.c) + i) = z;
+        if (p.c) *reinterpret_cast<uint4*>(static_cast<T*>(p.c) + i) = z;
         if (p.out2) *reinterpret_cast<uint4*>(static_cast<T*>(p.out2) + i) = z;
         if (p.out3) *reinterpret_cast<uint4*>(static_cast<T*>(p.out3) + i) = z;
       }

@@ -603,7 +603,9 @@ bool grouped_gemm_supported(const at::Tensor& a, const at::Tensor& b, bool trans
   return K == Kb && K % 8 == 0 && N % 8 == 0 && N >= 64 && K >= 8;
 }
 
-std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, const at::Tensor& bins, bool trans_a,
+// `only_out2`: the activation epilogues (kEpiAct, kEpiGluDual) store nothing but the activation; c and
+// out3 come back undefined.
+std::vector<at::Tensor> grouped_gemm_outputs(const at::Tensor& a, const at::Tensor& b, const at::Tensor& bins, bool trans_a,
                                      bool trans_b, int64_t epilogue, int64_t act,
                                      const c10::optional<at::Tensor>& aux1, const c10::optional<at::Tensor>& aux2,
                                      bool want_out2, bool want_out3, int64_t num_groups,
@@ -614,7 +616,7 @@ std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, c
                                      const std::vector<int64_t>& scatter_args, double alpha,
                                      const c10::optional<at::Tensor>& a2, const c10::optional<at::Tensor>& b2,
                                      const c10::optional<at::Tensor>& sqnorm,
-                                     const c10::optional<at::Tensor>& seq_base) {
+                                     const c10::optional<at::Tensor>& seq_base, bool only_out2) {
   using namespace gemm;
   MB_CHECK_CUDA(a); MB_CHECK_CUDA(b); MB_CHECK_CUDA(bins);
   MB_CHECK_CONTIG(a); MB_CHECK_CONTIG(b); MB_CHECK_CONTIG(bins);
@@ -641,10 +643,13 @@ std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, c
     p.M = 0;
     // With the fused combine the rows go to the peers' return buffers: no local output exists.
     if (scatter.has_value()) c = at::empty({0, p.N}, a.options());
-    else c = c_in.has_value() ? *c_in : at::empty({a.size(0), p.N}, a.options());
+    else if (!only_out2) c = c_in.has_value() ? *c_in : at::empty({a.size(0), p.N}, a.options());
   }
-  TORCH_CHECK(c.is_contiguous() && c.scalar_type() == a.scalar_type(), "bad output buffer");
-  const int64_t out_numel = scatter.has_value() ? a.size(0) * int64_t(p.N) : c.numel();
+  TORCH_CHECK(!only_out2 || (layout != kTN && !c_in.has_value() && !scatter.has_value() && want_out2 &&
+                             (epilogue == kEpiAct || epilogue == kEpiGluDual)),
+              "an activation alone: activation epilogues of the NT / NN layouts only");
+  TORCH_CHECK(only_out2 || (c.is_contiguous() && c.scalar_type() == a.scalar_type()), "bad output buffer");
+  const int64_t out_numel = scatter.has_value() || only_out2 ? a.size(0) * int64_t(p.N) : c.numel();
   auto check_aux = [&](const c10::optional<at::Tensor>& t, const char* name) {
     TORCH_CHECK(t.has_value() && t->is_cuda() && t->is_contiguous() && t->numel() == out_numel &&
                     t->scalar_type() == a.scalar_type(),
@@ -670,10 +675,10 @@ std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, c
     p.aux2 = aux2->data_ptr();
   }
   if (epilogue != kEpiNone && epilogue != kEpiAdd && want_out2) {
-    out2 = at::empty_like(c);
+    out2 = only_out2 ? at::empty({a.size(0), p.N}, a.options()) : at::empty_like(c);
     p.out2 = out2.data_ptr();
   }
-  if ((epilogue == kEpiDGlu && want_out3) || epilogue == kEpiGluDual) {
+  if ((epilogue == kEpiDGlu && want_out3) || (epilogue == kEpiGluDual && !only_out2)) {
     out3 = at::empty_like(c);
     p.out3 = out3.data_ptr();
   }
@@ -692,7 +697,7 @@ std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, c
                     b2->is_cuda() && b2->is_contiguous() && b2->sizes() == b.sizes() && b2->scalar_type() == b.scalar_type(),
                 "a2 / b2 must match a / b");
   }
-  p.c = c.data_ptr();
+  p.c = only_out2 ? nullptr : c.data_ptr();
   p.status = status_word(a.device()).data_ptr<int>();
 #ifdef MB_GEMM_TIMING
   p.timing = reinterpret_cast<long long*>(timing_words(a.device()).data_ptr<int64_t>());
@@ -794,7 +799,7 @@ std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, c
   if (!scatter.has_value() && store_tma_enabled()) {
     // Full 32-row quarters of a tile leave through the TMA unit (one instruction per chunk).
     const int64_t out_rows = out_numel / p.N;
-    bool ok = make_output_map(&p.out_map[0], p.c, bf16, out_rows, p.N);
+    bool ok = p.c == nullptr || make_output_map(&p.out_map[0], p.c, bf16, out_rows, p.N);
     if (ok && p.out2) ok = make_output_map(&p.out_map[1], p.out2, bf16, out_rows, p.N);
     if (ok && p.out3) ok = make_output_map(&p.out_map[2], p.out3, bf16, out_rows, p.N);
     p.store_tma = ok ? 1 : 0;
@@ -856,6 +861,23 @@ std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, c
   MB_CUDA_OK(launch(bf16, layout, block_n, ta, tb, p, grid, stream()));
   MB_LAUNCHED(1);
   return {c, out2, out3};
+}
+
+std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, const at::Tensor& bins, bool trans_a,
+                                     bool trans_b, int64_t epilogue, int64_t act,
+                                     const c10::optional<at::Tensor>& aux1, const c10::optional<at::Tensor>& aux2,
+                                     bool want_out2, bool want_out3, int64_t num_groups,
+                                     const c10::optional<at::Tensor>& c_in, bool zero_tail,
+                                     const c10::optional<at::Tensor>& wait_flags, int64_t wait_count,
+                                     int64_t wait_stride, int64_t wait_seq, int64_t rows_hint, int64_t pair_mode,
+                                     const c10::optional<std::vector<at::Tensor>>& scatter,
+                                     const std::vector<int64_t>& scatter_args, double alpha,
+                                     const c10::optional<at::Tensor>& a2, const c10::optional<at::Tensor>& b2,
+                                     const c10::optional<at::Tensor>& sqnorm,
+                                     const c10::optional<at::Tensor>& seq_base) {
+  return grouped_gemm_outputs(a, b, bins, trans_a, trans_b, epilogue, act, aux1, aux2, want_out2, want_out3, num_groups, c_in, zero_tail,
+                              wait_flags, wait_count, wait_stride, wait_seq, rows_hint, pair_mode, scatter, scatter_args, alpha, a2,
+                              b2, sqnorm, seq_base, false);
 }
 
 // ---------------------------------------------------------------------------
