@@ -126,9 +126,10 @@ __device__ void block_scan_totals(const int* __restrict__ totals, int nbins, int
 }
 
 // Row of the copy at sorted position `pos` of bin d: the position itself, or (capacity > 0) its slot of the
-// bin's `capacity` slots, -1 past them.  The plan knows it where it places the copy; the un-permutation
+// bin's `capacity` slots, -1 past them.  An id beyond the experts belongs to none: -1.  The plan knows it where it places the copy; the un-permutation
 // would otherwise search it again with a launch of its own, forward and backward.
-__device__ __forceinline__ int row_of_copy(int pos, int bin_start, int d, int capacity) {
+__device__ __forceinline__ int row_of_copy(int pos, int bin_start, int d, int num_experts, int capacity) {
+  if (d >= num_experts) return -1;
   if (capacity <= 0) return pos;
   const int off = pos - bin_start;
   return off < capacity ? d * capacity + off : -1;
@@ -184,7 +185,7 @@ sort_place_kernel(const K* __restrict__ keys, const V* __restrict__ vals_in, int
     if (valid) {
       keys_out[pos] = static_cast<KO>(key);
       vals_out[pos] = vals_in != nullptr ? vals_in[i] : static_cast<V>(i);
-      if (inverse != nullptr) inverse[i] = row_of_copy(pos, bin_base[d], d, capacity);
+      if (inverse != nullptr) inverse[i] = row_of_copy(pos, bin_base[d], d, num_real_bins, capacity);
     }
   }
 }
@@ -262,7 +263,7 @@ route_plan_small_kernel(const K* __restrict__ keys, int n, int bits, int num_exp
     if (valid) {
       bin_ids[pos] = key;
       indices[pos] = i;
-      if (inverse != nullptr) inverse[i] = row_of_copy(pos, bin_start[d], d, capacity);
+      if (inverse != nullptr) inverse[i] = row_of_copy(pos, bin_start[d], d, num_experts, capacity);
     }
   }
 }

@@ -458,6 +458,20 @@ def test_plan_gives_the_rows_of_the_copies(experts, copies, capacity):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize('copies', [100, 5000])
+@pytest.mark.parametrize('capacity', [0, 4])
+def test_plan_drops_copies_of_no_expert(copies, capacity):
+    """An id past the last expert (but inside the sort's key bits) has no row on either path."""
+    from megablocks_b200._ext import ext
+    top = torch.arange(copies, device='cuda') % 8
+    rows = ext().route_plan_rows(top, 5, 128, capacity)[5]
+    assert torch.all((rows == -1) | (top < 5))
+    assert int(rows.max()) < (5 * capacity if capacity else copies)
+    if not capacity:
+        assert torch.equal(rows == -1, top >= 5)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize('top_k', [1, 2, 3, 5])
 @pytest.mark.parametrize('hidden', [8, 100, 512, 520, 1032])
