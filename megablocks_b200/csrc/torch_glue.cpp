@@ -1243,6 +1243,9 @@ at::Tensor column_sum_op(const at::Tensor& x) {
   MB_CHECK_CUDA(x); MB_CHECK_CONTIG(x);
   TORCH_CHECK(x.dim() == 2 && (x.size(1) * x.element_size()) % 16 == 0,
               "column_sum expects x[rows, cols] with rows of a multiple of 16 bytes");
+  // The kernel reads 16 bytes at a time.  A contiguous gradient may still start at any element (a slice of
+  // a flat buffer, the backward of a flattened cat): the library reduction takes those.
+  if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0) return at::sum(x, {0});
   c10::cuda::CUDAGuard guard(x.device());
   at::Tensor out = at::empty({x.size(1)}, x.options());
   const int slices = colsum_slices(x.size(0), int(x.size(1)), int(x.element_size()), sm_count());

@@ -403,6 +403,53 @@ def test_native_expert_block_equals_the_separate_ops(kind, dtype, tokens, top_k,
         assert torch.equal(got, want)
 
 
+def _stock_layer(kind, dtype=torch.bfloat16, hidden=72, ffn=264, experts=5, top_k=2, **kw):
+    """A layer whose calls take the native expert block (kind 'sparse': only its output-bias rule)."""
+    args = dict(hidden_size=hidden, ffn_hidden_size=ffn, moe_num_experts=experts, moe_top_k=top_k, moe_capacity_factor=1,
+                mlp_type='glu' if kind == 'glu' else 'mlp', mlp_impl='sparse' if kind == 'sparse' else 'grouped',
+                activation_fn=F.silu, bias=True, return_bias=False, fp16=dtype == torch.float16,
+                bf16=dtype == torch.bfloat16, device=torch.device('cuda'))
+    args.update(kw)
+    layer = (mb.MoE if kind == 'dropping' else mb.dMoE)(mb.Arguments(**args))
+    if layer.experts.bias is not None:
+        torch.nn.init.normal_(layer.experts.bias)
+    return layer
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('kind', ['mlp', 'glu', 'dropping'])
+@pytest.mark.parametrize('offset', [0, 1, 3])
+def test_output_gradient_at_any_address(kind, offset):
+    """A contiguous output gradient may start at any element of a flat buffer; the kernels that read 16 bytes
+    at a time must not be handed one that does not start on 16 bytes."""
+    layer = _stock_layer(kind)
+    x = torch.randn(37, 1, 72, device='cuda').bfloat16().requires_grad_(True)
+    flat = torch.randn(37 * 72 + 8, device='cuda').bfloat16()
+    dy = flat[offset:offset + 37 * 72].view(37, 1, 72)
+    assert dy.is_contiguous() and (dy.data_ptr() % 16 == 0) == (offset == 0)
+    y = layer(x)
+    moe_mod.clear_load_balancing_loss()
+    leaves = [x] + list(layer.parameters())
+    got = torch.autograd.grad(y, leaves, dy, retain_graph=True)
+    want = torch.autograd.grad(y, leaves, dy.clone())
+    for leaf, g, w in zip(leaves, got, want):
+        if leaf is layer.experts.bias:      # fp32 sums in another order, rounded once
+            torch.testing.assert_close(g, w, rtol=2 ** -7, atol=1e-5 * 37)
+        else:
+            torch.testing.assert_close(g, w, rtol=2 ** -7, atol=2 ** -8 * float(w.float().abs().max()))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
+def test_column_sum_of_rows_at_any_address(dtype):
+    from megablocks_b200._ext import ext
+    flat = torch.randn(100 * 72 + 8, device='cuda').to(dtype)
+    for offset in (0, 1, 2, 7):
+        x = flat[offset:offset + 100 * 72].view(100, 72)
+        want = x.double().sum(0)
+        assert torch.all((ext().column_sum(x).double() - want).abs() <= torch.finfo(dtype).eps * want.abs() + 1e-5 * x.double().abs().sum(0))
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize('experts', [4, 8, 24, 32, 64, 128, 256, 320])
