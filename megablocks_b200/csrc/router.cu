@@ -17,6 +17,18 @@ namespace {
 constexpr int kMaxPerLane = kRouterMaxExperts / 32;
 constexpr int kMaxTopK = kRouterMaxTopK;
 
+// A token with a NaN or +inf logit has NaN scores.  They are selected like the largest ones, so every
+// token gets top_k distinct ids of [0, experts) (scores lie in [0, 1], taken ones count as -1), and its
+// weights are NaN: an overflow is seen in the loss and not read as an address.
+__device__ __forceinline__ float selection_key(float score) { return score != score ? INFINITY : score; }
+__device__ __forceinline__ float selected_score(float key) { return key == INFINITY ? NAN : key; }
+
+// Score of a selected id in the backward kernels; an id of no expert has none.
+template <typename T>
+__device__ __forceinline__ float score_of(const T* scores, int e, int num_experts) {
+  return static_cast<unsigned>(e) < static_cast<unsigned>(num_experts) ? to_float(scores[e]) : NAN;
+}
+
 template <typename T, int PL>
 __global__ void __launch_bounds__(128)
 router_topk_fwd_kernel(const T* __restrict__ logits, int64_t tokens, int num_experts, int top_k, float norm_p,
@@ -52,7 +64,7 @@ router_topk_fwd_kernel(const T* __restrict__ logits, int64_t tokens, int num_exp
     if (e < num_experts) {
       const T r = from_float<T>(v[j] * inv);
       srow[e] = r;
-      v[j] = to_float(r);          // selection runs on the rounded scores
+      v[j] = selection_key(to_float(r));          // selection runs on the rounded scores
     } else {
       v[j] = -1.f;
     }
@@ -73,7 +85,7 @@ router_topk_fwd_kernel(const T* __restrict__ logits, int64_t tokens, int num_exp
       const int oe = __shfl_xor_sync(0xffffffffu, best_e, d);
       if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; }
     }
-    chosen_w[s] = best;
+    chosen_w[s] = selected_score(best);
     chosen_e[s] = best_e;
     if ((best_e & 31) == lane) {
 #pragma unroll
@@ -139,7 +151,7 @@ router_topk_fwd_vec_kernel(const T* __restrict__ logits, int64_t tokens, int top
 #pragma unroll
   for (int j = 0; j < VEC; ++j) {
     raw.v[j] = from_float<T>(v[j] * inv);
-    v[j] = to_float(raw.v[j]);                    // selection runs on the rounded scores
+    v[j] = selection_key(to_float(raw.v[j]));     // selection runs on the rounded scores
   }
   if (live) *reinterpret_cast<uint4*>(scores + t * E + l * VEC) = *reinterpret_cast<const uint4*>(&raw);
   float chosen[kMaxTopK];
@@ -158,8 +170,8 @@ router_topk_fwd_vec_kernel(const T* __restrict__ logits, int64_t tokens, int top
       const int oe = __shfl_xor_sync(0xffffffffu, best_e, d);
       if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; }
     }
-    chosen[s] = best;
-    norm += norm_p == 1.f ? fabsf(best) : best * best;
+    chosen[s] = selected_score(best);
+    norm += norm_p == 1.f ? fabsf(chosen[s]) : chosen[s] * chosen[s];
 #pragma unroll
     for (int j = 0; j < VEC; ++j)
       if (best_e == l * VEC + j) v[j] = -1.f;
@@ -198,7 +210,7 @@ router_topk_bwd_vec_kernel(const T* __restrict__ scores, const int64_t* __restri
   for (int s = 0; s < kMaxTopK; ++s) {
     if (s >= top_k) break;
     sel[s] = static_cast<int>(experts[t * top_k + s]);
-    raw[s] = to_float(scores[t * E + sel[s]]);
+    raw[s] = score_of(scores + t * E, sel[s], E);
     dsel[s] = to_float(dweights[t * top_k + s]);
     norm_acc += (norm_p == 1.f) ? fabsf(raw[s]) : raw[s] * raw[s];
     dot += dsel[s] * raw[s];
@@ -269,7 +281,7 @@ router_topk_bwd_kernel(const T* __restrict__ scores, const int64_t* __restrict__
   float norm_acc = 0.f, dot = 0.f;
   for (int s = 0; s < top_k; ++s) {
     sel[s] = static_cast<int>(experts[t * top_k + s]);
-    raw[s] = to_float(srow[sel[s]]);
+    raw[s] = score_of(srow, sel[s], num_experts);
     dsel[s] = to_float(dweights[t * top_k + s]);
     norm_acc += (norm_p == 1.f) ? fabsf(raw[s]) : raw[s] * raw[s];
     dot += dsel[s] * raw[s];

@@ -486,6 +486,42 @@ def test_router_selection_over_expert_counts(dtype, experts, top_k, norm_p):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize('experts', [4, 24, 64, 256, 320])
+@pytest.mark.parametrize('top_k,norm_p', [(1, 0), (2, 1), (4, 2)])
+def test_router_selection_of_non_finite_logits(dtype, experts, top_k, norm_p):
+    """Tokens with NaN or infinite logits (an fp16 overflow) get distinct ids of real experts and NaN scores,
+    weights and gradients, like the library's softmax and top-k; their neighbours are untouched."""
+    torch.manual_seed(experts)
+    clean = torch.randn(37, experts).to(dtype)
+    logits, bad = clean.clone(), [3, 4, 9, 20, 36]
+    logits[3, 1] = float('nan')
+    logits[4, 2] = float('inf')
+    logits[9] = float('nan')
+    logits[20] = float('inf')
+    logits[36] = -float('inf')
+    run = lambda t: router_mod._FusedTopK.apply(t, top_k, float(norm_p))
+    leaf = logits.cuda().requires_grad_(True)
+    scores, weights, ids = run(leaf)
+    with torch.no_grad():
+        plain = router_mod._fused_top_k(leaf, top_k, float(norm_p))
+    assert torch.equal(plain[2], ids)
+    assert int(ids.min()) >= 0 and int(ids.max()) < experts
+    assert all(len(set(row)) == top_k for row in ids.tolist())
+    assert scores[bad].isnan().all() and weights[bad].isnan().all()
+    assert torch.equal(logits.float().softmax(-1).isnan(), scores.detach().cpu().isnan())
+    own = clean.cuda().requires_grad_(True)
+    want = run(own)
+    rest = [t for t in range(37) if t not in bad]
+    for got, ref in zip((scores, weights, ids), want):
+        assert torch.equal(got[rest], ref[rest])
+    ds, dw = torch.randn(37, experts, device='cuda').to(dtype), torch.randn(37, top_k, device='cuda').to(dtype)
+    got, = torch.autograd.grad([scores, weights], leaf, [ds, dw])
+    ref, = torch.autograd.grad(want[:2], own, [ds, dw])
+    assert got[bad].isnan().all() and torch.equal(got[rest], ref[rest])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize('experts,copies', [(5, 1), (64, 4096), (64, 5000), (1000, 300), (1200, 50)])
 @pytest.mark.parametrize('capacity', [0, 3])
 def test_plan_gives_the_rows_of_the_copies(experts, copies, capacity):
