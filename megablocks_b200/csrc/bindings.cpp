@@ -60,17 +60,27 @@ std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, c
 std::vector<at::Tensor> route_plan_rows(const at::Tensor& top_experts, int64_t num_experts, int64_t block,
                                         int64_t capacity);
 
+at::Tensor combine_rows_op(const at::Tensor& x, const at::Tensor& inverse, const c10::optional<at::Tensor>& weights,
+                           int64_t top_k, int64_t tokens, const c10::optional<at::Tensor>& bias);
+
 // expert_block.cpp
+std::vector<at::Tensor> expert_rows_forward(const at::Tensor& x, const at::Tensor& top_experts, const at::Tensor& w1,
+                                            const at::Tensor& w2, const c10::optional<at::Tensor>& v1,
+                                            const c10::optional<at::Tensor>& gemm_bins, int64_t num_experts,
+                                            int64_t top_k, int64_t act, int64_t capacity, bool save, int64_t pair);
 std::vector<at::Tensor> expert_block_forward(const at::Tensor& x, const at::Tensor& top_experts,
                                              const at::Tensor& weights, const at::Tensor& w1, const at::Tensor& w2,
                                              const c10::optional<at::Tensor>& v1, const c10::optional<at::Tensor>& bias,
                                              const c10::optional<at::Tensor>& gemm_bins, int64_t num_experts,
-                                             int64_t top_k, int64_t act, int64_t capacity, bool save, int64_t pair);
-std::vector<at::Tensor> expert_block_backward(
-    const at::Tensor& dout, const at::Tensor& indices, const at::Tensor& inverse, const at::Tensor& bins,
-    const c10::optional<at::Tensor>& gemm_bins, const at::Tensor& rows, const at::Tensor& y, const at::Tensor& z1,
-    const c10::optional<at::Tensor>& z2, const c10::optional<at::Tensor>& h_in, const at::Tensor& weights,
-    const at::Tensor& w1, const at::Tensor& w2, const c10::optional<at::Tensor>& v1, const std::vector<bool>& needs,
+                                             int64_t top_k, int64_t act, int64_t capacity, int64_t pair);
+std::vector<at::Tensor> expert_combine_backward(const at::Tensor& dout, const at::Tensor& indices, const at::Tensor& bins,
+                                                const at::Tensor& y, const at::Tensor& weights,
+                                                const std::vector<bool>& needs, int64_t top_k, int64_t capacity);
+std::vector<at::Tensor> expert_rows_backward(
+    const at::Tensor& dy, const at::Tensor& inverse, const at::Tensor& bins, const c10::optional<at::Tensor>& gemm_bins,
+    const at::Tensor& rows, const at::Tensor& z1, const c10::optional<at::Tensor>& z2,
+    const c10::optional<at::Tensor>& h_in, const at::Tensor& w1, const at::Tensor& w2,
+    const c10::optional<at::Tensor>& v1, const std::vector<bool>& needs,
     const std::vector<c10::optional<at::Tensor>>& slots, int64_t top_k, int64_t act, double wgrad_scale,
     int64_t capacity, int64_t pair);
 int64_t read_status(bool clear);
@@ -162,8 +172,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("router_topk_backward", &mb::router_topk_backward);
   m.def("grouped_gemm_supported", &mb::grouped_gemm_supported);
   m.def("grouped_gemm", &mb::grouped_gemm);
+  m.def("combine_rows", &mb::combine_rows_op);
   m.def("expert_block_forward", &mb::expert_block_forward);
-  m.def("expert_block_backward", &mb::expert_block_backward);
+  m.def("expert_rows_forward", &mb::expert_rows_forward);
+  m.def("expert_rows_backward", &mb::expert_rows_backward);
+  m.def("expert_combine_backward", &mb::expert_combine_backward);
   m.def("read_status", &mb::read_status);
   m.def("launch_count", &mb::launch_count);
   m.def("count_launches", &mb::count_launches);

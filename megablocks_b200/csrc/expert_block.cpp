@@ -1,8 +1,10 @@
 // The routed expert computation of one device - plan, permute, expert GEMMs, weighted un-permute - as one
-// native call forward and one backward.  The kernels are those behind the separate ops; what this saves
-// is the host's time between them: some 20 us of Python per op (an autograd node, argument checks and
+// native call where nothing is differentiated, else as two each way (the experts, the un-permutation),
+// each behind an autograd node.  The kernels are those behind the separate ops; what this saves is the
+// host's time between them: some 20 us of Python per op (an autograd node, argument checks and
 // conversions), which bounds small calls (a decode step of 8 tokens has 60 us of kernels, a 256-token
-// training pass 110).
+// training pass 110).  Two nodes and not one, because y, which only the un-permutation's backward reads,
+// has to be free before the experts' backward allocates.
 //
 // Two layouts, as in the layers (megablocks/layers/dmoe.py:196-249, moe.py:185-245 of the reference):
 //   capacity < 0   dropless: ragged row groups, weights [E, f, h], groups given by the plan's `bins`;
@@ -27,6 +29,11 @@ at::Tensor binned_gather_rows(const at::Tensor& x, const at::Tensor& indices, co
 std::vector<at::Tensor> scatter_backward_op(const at::Tensor& x, const at::Tensor& grad, const at::Tensor& indices,
                                             const at::Tensor& weights, const at::Tensor& bins,
                                             const OptTensor& padded_bins, int64_t top_k);
+at::Tensor scatter_wgrad_op(const at::Tensor& x, const at::Tensor& grad, const at::Tensor& indices,
+                            const at::Tensor& bin_ids, const at::Tensor& bins, const at::Tensor& padded_bins,
+                            int64_t top_k);
+at::Tensor binned_scatter_wgrad(const at::Tensor& x, const at::Tensor& grad, const at::Tensor& indices,
+                                const at::Tensor& bins, int64_t top_k);
 at::Tensor column_sum_op(const at::Tensor& x);
 std::vector<at::Tensor> grouped_gemm_outputs(const at::Tensor& a, const at::Tensor& b, const at::Tensor& bins, bool trans_a,
                                      bool trans_b, int64_t epilogue, int64_t act, const OptTensor& aux1,
@@ -56,18 +63,16 @@ at::Tensor rows_of(const at::Tensor& t) { return t.dim() == 3 ? t.view({-1, t.si
 
 }  // namespace
 
-// {out, tokens_per_expert} or, with `save`, also {indices, inverse, bins, x rows, y rows, z1, z2, h}
-// (z2 undefined for the MLP).
-std::vector<at::Tensor> expert_block_forward(const at::Tensor& x, const at::Tensor& top_experts,
-                                             const at::Tensor& weights, const at::Tensor& w1, const at::Tensor& w2,
-                                             const OptTensor& v1, const OptTensor& bias, const OptTensor& gemm_bins,
-                                             int64_t num_experts, int64_t top_k, int64_t act, int64_t capacity, bool save,
-                                             int64_t pair) {
+// {y, tokens_per_expert, indices, inverse, bins} and, with `save`, {x rows, z1, z2, h} (z2 undefined for the
+// MLP): plan, permutation and expert GEMMs; y[rows, hidden] is in expert order.
+std::vector<at::Tensor> expert_rows_forward(const at::Tensor& x, const at::Tensor& top_experts, const at::Tensor& w1,
+                                            const at::Tensor& w2, const OptTensor& v1, const OptTensor& gemm_bins,
+                                            int64_t num_experts, int64_t top_k, int64_t act, int64_t capacity, bool save,
+                                            int64_t pair) {
   const auto plan = route_plan_rows(top_experts, num_experts, 128, capacity);
   const at::Tensor &indices = plan[0], &bin_ids = plan[1], &bins = plan[2], &inverse = plan[5];
   const bool binned = capacity > 0;
   TORCH_CHECK(!binned || (gemm_bins.has_value() && !v1.has_value()), "capacity layout: uniform bins, no gate weight");
-  const int64_t tokens = x.size(0);
   at::Tensor rows = binned ? rows_of(binned_gather_rows(x, indices, {}, bins, capacity, top_k))
                            : gather_rows_op(x, indices, bin_ids, {}, bins, bins, top_k, indices.numel());
   const at::Tensor& groups = binned ? *gemm_bins : bins;
@@ -87,49 +92,70 @@ std::vector<at::Tensor> expert_block_forward(const at::Tensor& x, const at::Tens
     z1 = o[0]; h = o[1];
   }
   at::Tensor y = Gemm{}.run(h, w2, groups, pair)[0];
-  at::Tensor out = combine_rows_op(y, inverse, weights, top_k, tokens, bias);
-  if (!save) return {out, plan[4]};
-  if (binned) y = y.view({num_experts, capacity, -1});
-  return {out, plan[4], indices, inverse, bins, rows, y, z1, z2, h};
+  if (!save) return {y, plan[4], indices, inverse, bins};
+  return {y, plan[4], indices, inverse, bins, rows, z1, z2, h};
 }
 
-// {dx, dweights, dw1, dw2, dv1, dbias}, undefined where `needs` says so.  `slots`: per weight gradient
+// {out, tokens_per_expert}: the whole block where nothing is differentiated.
+std::vector<at::Tensor> expert_block_forward(const at::Tensor& x, const at::Tensor& top_experts,
+                                             const at::Tensor& weights, const at::Tensor& w1, const at::Tensor& w2,
+                                             const OptTensor& v1, const OptTensor& bias, const OptTensor& gemm_bins,
+                                             int64_t num_experts, int64_t top_k, int64_t act, int64_t capacity,
+                                             int64_t pair) {
+  auto o = expert_rows_forward(x, top_experts, w1, w2, v1, gemm_bins, num_experts, top_k, act, capacity, false, pair);
+  return {combine_rows_op(o[0], o[3], weights, top_k, x.size(0), bias), o[1]};
+}
+
+// {dy, dweights, dbias} of the un-permutation, undefined where `needs` says so.
+std::vector<at::Tensor> expert_combine_backward(const at::Tensor& dout, const at::Tensor& indices, const at::Tensor& bins,
+                                                const at::Tensor& y, const at::Tensor& weights,
+                                                const std::vector<bool>& needs, int64_t top_k, int64_t capacity) {
+  const bool binned = capacity > 0;
+  const at::Tensor slots = binned ? y.view({bins.numel(), capacity, y.size(1)}) : y;
+  at::Tensor dy, dweights, dbias;
+  if (needs[2]) dbias = column_sum_op(dout);
+  if (needs[0]) {
+    auto un = scatter_backward_op(slots, dout, indices, weights, bins, binned ? OptTensor() : OptTensor(bins), top_k);
+    dy = rows_of(un[0]);
+    if (needs[1]) dweights = un[1];
+  } else if (needs[1]) {
+    dweights = binned ? binned_scatter_wgrad(slots, dout, indices, bins, top_k)
+                      : scatter_wgrad_op(slots, dout, indices, indices, bins, bins, top_k);
+  }
+  return {dy, dweights, dbias};
+}
+
+// {dx, dw1, dw2, dv1} from the gradient of y, undefined where `needs` says so.  `slots`: per weight gradient
 // (w1, w2, v1) an optional accumulator of its squared norm.
-std::vector<at::Tensor> expert_block_backward(const at::Tensor& dout, const at::Tensor& indices,
-                                              const at::Tensor& inverse, const at::Tensor& bins,
-                                              const OptTensor& gemm_bins, const at::Tensor& rows, const at::Tensor& y,
-                                              const at::Tensor& z1, const OptTensor& z2, const OptTensor& h_in,
-                                              const at::Tensor& weights, const at::Tensor& w1, const at::Tensor& w2,
-                                              const OptTensor& v1, const std::vector<bool>& needs,
-                                              const std::vector<OptTensor>& slots, int64_t top_k, int64_t act,
-                                              double wgrad_scale, int64_t capacity, int64_t pair) {
+std::vector<at::Tensor> expert_rows_backward(const at::Tensor& dy, const at::Tensor& inverse, const at::Tensor& bins,
+                                             const OptTensor& gemm_bins, const at::Tensor& rows, const at::Tensor& z1,
+                                             const OptTensor& z2, const OptTensor& h_in, const at::Tensor& w1,
+                                             const at::Tensor& w2, const OptTensor& v1, const std::vector<bool>& needs,
+                                             const std::vector<OptTensor>& slots, int64_t top_k, int64_t act,
+                                             double wgrad_scale, int64_t capacity, int64_t pair) {
   const bool binned = capacity > 0;
   const at::Tensor& groups = binned ? *gemm_bins : bins;
-  const int64_t tokens = dout.size(0);
-  at::Tensor dx, dweights, dw1, dw2, dv1, dbias;
-  if (needs[5]) dbias = column_sum_op(dout);
-  auto un = scatter_backward_op(y, dout, indices, weights, bins, binned ? OptTensor() : OptTensor(bins), top_k);
-  if (needs[1]) dweights = un[1];
-  if (!(needs[0] || needs[2] || needs[3] || needs[4])) return {dx, dweights, dw1, dw2, dv1, dbias};
-  const at::Tensor dy = rows_of(un[0]);
-  Gemm down;
-  down.trans_b = true;
-  down.act = act;
-  down.aux1 = z1;
+  at::Tensor dx, dw1, dw2, dv1;
   at::Tensor dz1, dz2, h = h_in.has_value() ? *h_in : at::Tensor();
-  if (v1.has_value()) {
-    down.epilogue = gemm::kEpiDGlu;
-    down.aux2 = z2;
-    down.want_out3 = !h.defined();
-    auto o = down.run(dy, w2, groups, pair);
-    dz1 = o[0]; dz2 = o[1];
-    if (!h.defined()) h = o[2];
-  } else {
-    down.epilogue = gemm::kEpiDAct;
-    down.want_out2 = !h.defined();
-    auto o = down.run(dy, w2, groups, pair);
-    dz1 = o[0];
-    if (!h.defined()) h = o[1];
+  {
+    Gemm down;
+    down.trans_b = true;
+    down.act = act;
+    down.aux1 = z1;
+    if (v1.has_value()) {
+      down.epilogue = gemm::kEpiDGlu;
+      down.aux2 = z2;
+      down.want_out3 = !h.defined();
+      auto o = down.run(dy, w2, groups, pair);
+      dz1 = o[0]; dz2 = o[1];
+      if (!h.defined()) h = o[2];
+    } else {
+      down.epilogue = gemm::kEpiDAct;
+      down.want_out2 = !h.defined();
+      auto o = down.run(dy, w2, groups, pair);
+      dz1 = o[0];
+      if (!h.defined()) h = o[1];
+    }
   }
   auto wgrad = [&](const at::Tensor& a, const at::Tensor& b, const OptTensor& slot) {
     Gemm g;
@@ -138,20 +164,26 @@ std::vector<at::Tensor> expert_block_backward(const at::Tensor& dout, const at::
     g.sqnorm = slot;
     return g.run(a, b, groups, pair)[0];
   };
-  if (needs[3]) dw2 = wgrad(h, dy, slots[1]);
-  if (needs[2]) dw1 = binned ? wgrad(rows, dz1, slots[0]) : wgrad(dz1, rows, slots[0]);
-  if (v1.has_value() && needs[4]) dv1 = wgrad(dz2, rows, slots[2]);
+  if (needs[2]) dw2 = wgrad(h, dy, slots[1]);
+  if (needs[1]) dw1 = binned ? wgrad(rows, dz1, slots[0]) : wgrad(dz1, rows, slots[0]);
+  if (v1.has_value() && needs[3]) dv1 = wgrad(dz2, rows, slots[2]);
   if (needs[0]) {
-    Gemm in;
-    in.trans_b = binned;
-    if (v1.has_value()) {       // dx = dz1 w1 + dz2 v1 as one contraction over both pairs
-      in.a2 = dz2;
-      in.b2 = v1;
+    at::Tensor d;
+    {
+      Gemm in;
+      in.trans_b = binned;
+      if (v1.has_value()) {       // dx = dz1 w1 + dz2 v1 as one contraction over both pairs
+        in.a2 = dz2;
+        in.b2 = v1;
+      }
+      d = in.run(dz1, w1, groups, pair)[0];
     }
-    at::Tensor d = in.run(dz1, w1, groups, pair)[0];
-    dx = combine_rows_op(d, inverse, {}, top_k, tokens, {});
+    dz1.reset();                  // free before dx is allocated
+    dz2.reset();
+    h.reset();
+    dx = combine_rows_op(d, inverse, {}, top_k, inverse.numel() / top_k, {});
   }
-  return {dx, dweights, dw1, dw2, dv1, dbias};
+  return {dx, dw1, dw2, dv1};
 }
 
 }  // namespace mb

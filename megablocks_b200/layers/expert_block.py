@@ -1,10 +1,10 @@
-"""The routed expert computation of one device as a single native call.
+"""The routed expert computation of one device as one native call, or two where it is differentiated.
 
 Plan, permutation, expert GEMMs and weighted un-permutation are the kernels that the ops of
-``megablocks_b200.ops`` launch one by one; ``csrc/expert_block.cpp`` launches them back to back, and one
-autograd node stands for what are otherwise three.  That takes the Python between the launches out,
-which is what small calls are made of: a decode step (8 tokens, 64 experts) has 60 us of kernels in 205
-us, a 256-token training pass 110 in 730.
+``megablocks_b200.ops`` launch one by one; ``csrc/expert_block.cpp`` launches them back to back, and two
+autograd nodes (the experts, the un-permutation) stand for what are otherwise three.  That takes the
+Python between the launches out, which is what small calls are made of: a decode step (8 tokens, 64
+experts) has 60 us of kernels in 205 us, a 256-token training pass 110 in 730.
 
 :func:`route` says whether a layer's call may take this path: stock steps and expert modules without
 hooks, 16-bit CUDA tensors that the kernels take, an activation they know, none of the modes that give an
@@ -22,40 +22,66 @@ from megablocks_b200.ops import gg as G
 from megablocks_b200.utils import debug
 
 
-class _ExpertBlock(torch.autograd.Function):
+class _Experts(torch.autograd.Function):
+    """Plan, permutation and expert GEMMs: the copies' results in expert order, and the plan."""
 
     @staticmethod
-    def forward(ctx: Any, x, weights, top_experts, w1, w2, v1, bias, gemm_bins, num_experts, top_k, act, capacity,
-                memory_optimized, wgrad_scale):
-        out, counts, indices, inverse, bins, rows, y, z1, z2, h = ext().expert_block_forward(
-            x, top_experts, weights, w1, w2, v1, bias, gemm_bins, num_experts, top_k, act, capacity, True, G._PAIR_MODE)
-        ctx.save_for_backward(weights, w1, w2, v1, gemm_bins, indices, inverse, bins, rows, y, z1,
-                              z2 if v1 is not None else None, None if memory_optimized else h)
-        ctx.top_k, ctx.act, ctx.capacity, ctx.wgrad_scale = top_k, act, capacity, wgrad_scale
-        ctx.mark_non_differentiable(counts)
-        ctx.set_materialize_grads(False)        # no zero tensor for the counts
-        return out, counts
-
-    @staticmethod
-    def backward(ctx: Any, dout, _dcounts):
-        weights, w1, w2, v1, gemm_bins, indices, inverse, bins, rows, y, z1, z2, h = ctx.saved_tensors
-        if dout is None:
-            return (None,) * 14
+    def forward(ctx: Any, x, top_experts, w1, w2, v1, gemm_bins, num_experts, top_k, act, capacity, memory_optimized,
+                wgrad_scale):
         need = ctx.needs_input_grad
-        needs = [need[0], need[1], need[3], need[4], need[5], need[6]]
+        keep = need[0] or need[2] or need[3] or need[4]
+        y, counts, indices, inverse, bins, *kept = ext().expert_rows_forward(
+            x, top_experts, w1, w2, v1, gemm_bins, num_experts, top_k, act, capacity, keep, G._PAIR_MODE)
+        if keep:
+            rows, z1, z2, h = kept
+            ctx.save_for_backward(w1, w2, v1, gemm_bins, inverse, bins, rows, z1, z2 if v1 is not None else None,
+                                  None if memory_optimized else h)
+        ctx.top_k, ctx.act, ctx.capacity, ctx.wgrad_scale = top_k, act, capacity, wgrad_scale
+        ctx.mark_non_differentiable(counts, indices, inverse, bins)
+        ctx.set_materialize_grads(False)        # no zero tensors for the plan
+        return y, counts, indices, inverse, bins
+
+    @staticmethod
+    def backward(ctx: Any, dy, *_plan):
+        if dy is None:
+            return (None,) * 12
+        w1, w2, v1, gemm_bins, inverse, bins, rows, z1, z2, h = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        needs = [need[0], need[2], need[3], need[4]]
         sink = G._GRAD_NORM_SINK
         views, slots = [None, None, None], [None, None, None]
         if sink is not None:
-            wanted = [k for k in (1, 0, 2) if needs[2 + k] and (k < 2 or v1 is not None)]     # launch order
+            wanted = [k for k in (1, 0, 2) if needs[1 + k] and (k < 2 or v1 is not None)]     # launch order
             for k, (slot, view) in zip(wanted, sink.reserve(len(wanted))):
                 slots[k], views[k] = slot, view
-        dx, dweights, *dw, dbias = ext().expert_block_backward(
-            dout.contiguous(), indices, inverse, bins, gemm_bins, rows, y, z1, z2, h, weights, w1, w2, v1, needs, views,
-            ctx.top_k, ctx.act, ctx.wgrad_scale, ctx.capacity, G._PAIR_MODE)
+        dx, *dw = ext().expert_rows_backward(dy.contiguous(), inverse, bins, gemm_bins, rows, z1, z2, h, w1, w2, v1,
+                                             needs, views, ctx.top_k, ctx.act, ctx.wgrad_scale, ctx.capacity,
+                                             G._PAIR_MODE)
         for k in (1, 0, 2):
             if slots[k] is not None:
                 sink._record(dw[k], slots[k])
-        return (dx, dweights, None, *dw, dbias, None, None, None, None, None, None, None)
+        return (dx, None, *dw) + (None,) * 7
+
+
+class _Combine(torch.autograd.Function):
+    """Weighted un-permutation and output bias.  A node of its own: it alone keeps ``y``, and frees it before
+    the experts' backward starts."""
+
+    @staticmethod
+    def forward(ctx: Any, y, weights, bias, indices, inverse, bins, top_k, capacity):
+        ctx.save_for_backward(y, weights, indices, bins)
+        ctx.top_k, ctx.capacity = top_k, capacity
+        ctx.set_materialize_grads(False)
+        return ext().combine_rows(y, inverse, weights, top_k, inverse.numel() // top_k, bias)
+
+    @staticmethod
+    def backward(ctx: Any, dout):
+        if dout is None:
+            return (None,) * 8
+        y, weights, indices, bins = ctx.saved_tensors
+        dy, dweights, dbias = ext().expert_combine_backward(dout.contiguous(), indices, bins, y, weights,
+                                                            list(ctx.needs_input_grad[:3]), ctx.top_k, ctx.capacity)
+        return (dy, dweights, dbias) + (None,) * 5
 
 
 def _hooked(module: torch.nn.Module) -> bool:
@@ -96,7 +122,8 @@ def expert_block(x, expert_weights, top_experts, w1, w2, v1, bias, gemm_bins, nu
     tensors = (x, expert_weights, w1, w2, v1, bias)
     if not (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)):
         out, counts = ext().expert_block_forward(x, top_experts, expert_weights, w1, w2, v1, bias, gemm_bins, num_experts,
-                                                 top_k, act, capacity, False, G._PAIR_MODE)
+                                                 top_k, act, capacity, G._PAIR_MODE)
         return out, counts
-    return _ExpertBlock.apply(x, expert_weights, top_experts, w1, w2, v1, bias, gemm_bins, num_experts, top_k, act,
-                              capacity, memory_optimized, wgrad_scale)
+    y, counts, indices, inverse, bins = _Experts.apply(x, top_experts, w1, w2, v1, gemm_bins, num_experts, top_k, act,
+                                                       capacity, memory_optimized, wgrad_scale)
+    return _Combine.apply(y, expert_weights, bias, indices, inverse, bins, top_k, capacity), counts

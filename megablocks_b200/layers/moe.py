@@ -178,6 +178,9 @@ class ParallelMLP(torch.nn.Module):
         args = self.args
         if torch.is_grad_enabled() and not expert_weights.requires_grad and (x.requires_grad or w1.requires_grad):
             return None         # a frozen router: the step-by-step path keeps less for the backward pass
+        rows = self.num_experts * capacity if capacity > 0 else top_experts.numel()
+        if torch.is_grad_enabled() and x.requires_grad and rows * w2.shape[1] < x.numel():
+            return None         # narrow experts: what the block frees before it allocates dx would not make room for it
         if not expert_block.route(x, expert_weights, top_experts, self.mlp, w1, w2, v1, bias, args.activation_fn):
             return None
         out, counts = expert_block.expert_block(x, expert_weights, top_experts, w1, w2, v1, bias, gemm_bins,

@@ -4,6 +4,7 @@ Mirrors the reference layer tests (tests/layers/dmoe_test.py:17-241, moe_test.py
 glu_test.py:64-123) and adds backward numerics, which the reference only smoke-tests.
 """
 
+import gc
 from functools import partial
 
 import pytest
@@ -437,6 +438,33 @@ def test_output_gradient_at_any_address(kind, offset):
             torch.testing.assert_close(g, w, rtol=2 ** -7, atol=1e-5 * 37)
         else:
             torch.testing.assert_close(g, w, rtol=2 ** -7, atol=2 ** -8 * float(w.float().abs().max()))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('kind', ['mlp', 'glu', 'dropping'])
+@pytest.mark.parametrize('top_k,memory_optimized,ffn', [(1, True, 512), (2, True, 256), (2, False, 1024), (1, True, 128)])
+def test_native_block_holds_no_more_memory_than_the_separate_ops(kind, top_k, memory_optimized, ffn):
+    """Peak of a training pass: the rows before the un-permutation are free before the experts' backward."""
+    layer = _stock_layer(kind, hidden=512, ffn=ffn, experts=4, top_k=top_k, memory_optimized_mlp=memory_optimized)
+    x = torch.randn(4096, 1, 512, device='cuda').bfloat16().requires_grad_(True)
+    dy = torch.randn_like(x)
+
+    def peak():
+        for _ in range(2):          # the second pass finds what the first one laid out
+            gc.collect()            # nothing of an earlier test is freed in between
+            torch.cuda.reset_peak_memory_stats()
+            base = torch.cuda.memory_stats()['requested_bytes.all.current']
+            y = layer(x)
+            moe_mod.clear_load_balancing_loss()
+            grads = torch.autograd.grad(y, [x] + list(layer.parameters()), dy)
+            top = torch.cuda.memory_stats()['requested_bytes.all.peak'] - base
+            del y, grads
+        return top
+
+    fast = peak()
+    layer.experts.mlp.register_forward_hook(lambda *a: None)
+    slow = peak()
+    assert fast <= slow + 8 * 4 * 4096 * top_k      # index arrays, of 4 bytes a copy
 
 
 @pytest.mark.gpu
