@@ -176,7 +176,8 @@ class ParallelMLP(torch.nn.Module):
         bias = self.bias if self.bias is not None and not self.args.return_bias else None
         top_experts, expert_weights = top_experts.flatten(), expert_weights.flatten()
         args = self.args
-        if torch.is_grad_enabled() and not expert_weights.requires_grad and (x.requires_grad or w1.requires_grad):
+        if torch.is_grad_enabled() and not expert_weights.requires_grad and any(
+                t is not None and t.requires_grad for t in (x, w1, w2, v1, bias)):
             return None         # a frozen router: the step-by-step path keeps less for the backward pass
         rows = self.num_experts * capacity if capacity > 0 else top_experts.numel()
         if torch.is_grad_enabled() and x.requires_grad and rows * w2.shape[1] < x.numel():

@@ -468,6 +468,34 @@ def test_native_block_holds_no_more_memory_than_the_separate_ops(kind, top_k, me
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize('kind', ['mlp', 'glu', 'dropping'])
+@pytest.mark.parametrize('trained', ['experts.bias', 'router', 'w1', 'w2', 'x', 'all'])
+def test_native_block_keeps_no_more_for_backward_than_the_separate_ops(kind, trained):
+    """Bytes saved by a forward pass when only some of the layer is trained."""
+    layer = _stock_layer(kind)
+    for name, p in layer.named_parameters():
+        p.requires_grad_(trained == 'all' or trained in name)
+    x = torch.randn(300, 1, 72, device='cuda').bfloat16().requires_grad_(trained in ('x', 'all'))
+    own = {t.untyped_storage().data_ptr() for t in [x, *layer.parameters()]}
+
+    def kept():
+        held = {}
+
+        def pack(t):
+            held.setdefault(t.untyped_storage().data_ptr(), t)
+            return t
+
+        with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t):
+            layer(x)
+        moe_mod.clear_load_balancing_loss()
+        return sum(t.untyped_storage().nbytes() for ptr, t in held.items() if ptr not in own)
+
+    fast = kept()
+    layer.experts.mlp.register_forward_hook(lambda *a: None)
+    assert fast <= kept() + 600 * 4         # one index of 4 bytes a copy
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
 def test_column_sum_of_rows_at_any_address(dtype):
     from megablocks_b200._ext import ext
