@@ -130,9 +130,15 @@ class ParallelMLP(torch.nn.Module):
         return indices, bin_ids, bins, tokens_per_expert
 
     # -- output bias ----------------------------------------------------------
-    # Steps between `forward` and the un-permutation; a subclass that replaces one of them gets the
-    # bias added after it, as before.
+    # Steps between `forward` and the un-permutation; a subclass or an instance that replaces one of them
+    # gets the bias added after it.
     _bias_steps = ('forward_once', '_forward_once', 'permute_and_compute')
+
+    def _stock(self, steps) -> bool:
+        """Whether the layer still runs the library's own ``steps`` on one device."""
+        base, cls, own = self._bias_base, type(self), self.__dict__
+        return getattr(self.forward_fn, '__func__', None) is base.forward_once and not any(
+            name in own or getattr(cls, name) is not getattr(base, name) for name in steps)
 
     def _unpermute_bias(self, x: torch.Tensor):
         """The output bias if the un-permutation kernel can add it on its way out, else ``None``.
@@ -144,10 +150,7 @@ class ParallelMLP(torch.nn.Module):
                 or x.dtype not in (torch.bfloat16, torch.float16, torch.float32) or not bias.is_contiguous()
                 or bias.device != x.device or hasattr(bias, 'to_local') or torch.is_autocast_enabled('cuda')):
             return None
-        base, cls = self._bias_base, type(self)
-        stock = getattr(self.forward_fn, '__func__', None) is base.forward_once and all(
-            getattr(cls, name) is getattr(base, name) for name in base._bias_steps)
-        return bias if stock else None
+        return bias if self._stock(self._bias_base._bias_steps) else None
 
     # -- single device --------------------------------------------------------
     def permute_and_compute(self, x, tokens_per_expert, indices, bin_ids, expert_weights, bins, expert_capacity,
@@ -165,9 +168,7 @@ class ParallelMLP(torch.nn.Module):
     def _block_call(self, x: torch.Tensor, expert_weights: torch.Tensor, top_experts: torch.Tensor):
         """``(out, tokens_per_expert, whether the bias is in it)`` from the single native call, or ``None``
         where the layer has to run step by step."""
-        base, cls = self._bias_base, type(self)
-        if (getattr(self.forward_fn, '__func__', None) is not base.forward_once
-                or any(getattr(cls, name) is not getattr(base, name) for name in base._block_steps)):
+        if not self._stock(self._bias_base._block_steps):
             return None
         experts = self._block_experts(x.numel() // x.shape[-1])
         if experts is None:

@@ -496,6 +496,30 @@ def test_native_block_keeps_no_more_for_backward_than_the_separate_ops(kind, tra
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize('kind,step', [('mlp', 'indices_and_bins'), ('mlp', 'grouped_permute_and_compute'),
+                                       ('mlp', 'grouped_forward_once'), ('glu', 'grouped_permute_and_compute'),
+                                       ('dropping', 'permute_and_compute'), ('dropping', 'expert_capacity'),
+                                       ('dropping', 'indices_and_bins'), ('sparse', 'sparse_forward_once'),
+                                       ('sparse', 'topology')])
+def test_step_replaced_on_the_instance_is_called(kind, step):
+    """A step of the layer patched on one object is honoured, with the arguments the step always had."""
+    layer = _stock_layer(kind, hidden=128, ffn=256)
+    x = torch.randn(37, 1, 128, device='cuda').bfloat16()
+    want = layer(x)
+    plain, calls = getattr(layer.experts, step), []
+
+    def replaced(*args):
+        calls.append(step)
+        return plain(*args)
+
+    setattr(layer.experts, step, replaced)
+    got = layer(x)
+    assert calls
+    # The bias is added by the kernel or afterwards: one rounding of the sum apart.
+    torch.testing.assert_close(got, want, rtol=2 ** -7, atol=2 ** -7 * float(layer.experts.bias.abs().max()))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
 def test_column_sum_of_rows_at_any_address(dtype):
     from megablocks_b200._ext import ext
