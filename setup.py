@@ -47,6 +47,9 @@ setup(
             name='megablocks_b200._C',
             sources=sources,
             include_dirs=[os.path.join(ROOT, CSRC)],
+            # The shared C++ runtime that torch uses, also where the compiler would link a static copy: two
+            # copies share locales, and printing a number into an error message then crashes.
+            extra_link_args=['-l:libstdc++.so.6'],
             extra_compile_args={'cxx': ['-O3', '-std=c++17'] + DEFINES, 'nvcc': NVCC_FLAGS},
         )
     ],

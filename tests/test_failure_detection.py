@@ -9,13 +9,17 @@ exception, and leaves the CUDA context usable.
 
 import datetime
 import os
+import shutil
 import socket
+import subprocess
 import time
 
 import pytest
 import torch
 import torch.distributed as dist
 import torch.multiprocessing as mp
+
+from megablocks_b200 import _ext
 
 
 def _free_port():
@@ -165,3 +169,11 @@ def test_expert_parallel_exchange_fails_closed():
     got, _, _ = G.grouped_gemm(x, w, torch.tensor([64, 128], dtype=torch.int32, device=dev), trans_b=True)
     torch.testing.assert_close(got[:64].float(), ref, rtol=2e-2, atol=2e-1)
     status.check()
+
+
+def test_extension_shares_the_cpp_runtime_of_torch():
+    """A static copy of the C++ runtime beside torch's crashes when a number is printed into an error message."""
+    if _ext.try_ext() is None or shutil.which('nm') is None:
+        pytest.skip('needs the built extension and nm')
+    symbols = subprocess.run(['nm', '-D', '--defined-only', _ext.ext().__file__], capture_output=True, text=True, check=True)
+    assert '_ZNSo9_M_insert' not in symbols.stdout       # std::ostream << number, defined in libstdc++ alone
