@@ -523,19 +523,33 @@ EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
+// Two-dimensional map of a row-major [rows, cols] 16-bit tensor.  The driver call needs a current context,
+// which a thread whose first CUDA call this is does not have yet (autograd's worker, when the gradient's
+// storage came from the allocator's cache): the runtime makes it current, and the call is made again.
+CUresult encode_2d(CUtensorMap* map, const void* base, bool bf16, int64_t rows, int64_t cols, cuuint32_t box_rows,
+                   cuuint32_t box_cols, CUtensorMapSwizzle swizzle, CUtensorMapL2promotion promotion) {
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 2};
+  const cuuint32_t box[2] = {box_cols, box_rows};
+  const cuuint32_t elem_strides[2] = {1u, 1u};
+  auto encode = [&] {
+    return encode_tiled_fn()(
+        map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims,
+        strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, promotion, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  const CUresult rc = encode();
+  if (rc != CUDA_ERROR_INVALID_CONTEXT && rc != CUDA_ERROR_NOT_INITIALIZED) return rc;
+  C10_CUDA_CHECK(cudaSetDevice(at::cuda::current_device()));
+  return encode();
+}
+
 // Row-major [rows, cols] 16-bit tensor, box = box_rows x 64 columns, 128-byte swizzle.
 CUtensorMap make_tensor_map(const void* base, bool bf16, int64_t rows, int64_t cols, int box_rows) {
   TORCH_CHECK(reinterpret_cast<uintptr_t>(base) % 16 == 0, "grouped_gemm operands must be 16-byte aligned");
   TORCH_CHECK(cols % 8 == 0, "grouped_gemm operands need a row length that is a multiple of 8 elements");
   CUtensorMap map;
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(std::max<int64_t>(rows, 1))};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 2};
-  const cuuint32_t box[2] = {64u, static_cast<cuuint32_t>(box_rows)};
-  const cuuint32_t elem_strides[2] = {1u, 1u};
-  const CUresult rc = encode_tiled_fn()(
-      &map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base),
-      dims, strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const CUresult rc = encode_2d(&map, base, bf16, std::max<int64_t>(rows, 1), cols, cuuint32_t(box_rows), 64u,
+                                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
   TORCH_CHECK(rc == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed with code ", int(rc));
   return map;
 }
@@ -543,15 +557,8 @@ CUtensorMap make_tensor_map(const void* base, bool bf16, int64_t rows, int64_t c
 // Row-major [rows, cols] 16-bit output, box = 32 x 32, 64-byte swizzle (the epilogue's staging layout).
 bool make_output_map(CUtensorMap* map, const void* base, bool bf16, int64_t rows, int64_t cols) {
   if (reinterpret_cast<uintptr_t>(base) % 16 != 0 || cols % 8 != 0 || rows < 1) return false;
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 2};
-  const cuuint32_t box[2] = {32u, 32u};
-  const cuuint32_t elem_strides[2] = {1u, 1u};
-  const CUresult rc = encode_tiled_fn()(
-      map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims,
-      strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-      CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return rc == CUDA_SUCCESS;
+  return encode_2d(map, base, bf16, rows, cols, 32u, 32u, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE) ==
+         CUDA_SUCCESS;
 }
 
 at::Tensor& status_word(const at::Device& device) {

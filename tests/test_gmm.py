@@ -1,5 +1,9 @@
 """Grouped GEMM (all layouts and fused epilogues) against per-group fp32 matmuls."""
 
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 import torch.nn.functional as F
@@ -406,3 +410,30 @@ def test_cta_pair_gradient_norm():
     # The sum is over the fp32 values before their rounding to 16 bits (2^-9 each, random sign).
     want = float(out.double().square().sum())
     assert abs(float(sink.slots[sink.lookup(out)]) - want) <= 1e-3 * want
+
+
+_FIRST_IN_THREAD = """
+import sys, torch
+sys.path.insert(0, {root!r})
+from megablocks_b200.ops import gg
+a = torch.randn(100, 64, device='cuda').bfloat16().requires_grad_(True)
+b = torch.randn(2, 64, 72, device='cuda').bfloat16().requires_grad_(True)
+bins = torch.tensor([40, 100], dtype=torch.int32, device='cuda')
+y = gg.gmm_bins(a, b, bins)
+dy = torch.ones_like(y)
+room = [torch.empty(1 << 14, device='cuda') for _ in range(8)]      # what backward allocates is in the cache
+del room
+da, db = torch.autograd.grad(y, [a, b], dy)
+ref = torch.cat([dy[:40].float() @ b[0].float().t(), dy[40:].float() @ b[1].float().t()])
+torch.testing.assert_close(da.float(), ref, rtol=2e-2, atol=2e-2)
+print('done')
+"""
+
+
+@pytest.mark.gpu
+def test_backward_as_the_first_cuda_work_of_its_thread():
+    """Autograd's worker has no current CUDA context before its first runtime call, and the tensor maps are
+    made by a driver call."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    run = subprocess.run([sys.executable, '-c', _FIRST_IN_THREAD.format(root=root)], capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0 and 'done' in run.stdout, run.stderr[-2000:]
