@@ -136,12 +136,29 @@ __device__ __forceinline__ float erf_fast(float x) {
   return copysignf(y, x);
 }
 
+// 1 / (1 + e^-x) to a few units of fp32's last place.  e^-x is 2^(-x log2 e); what the product loses to
+// rounding is recovered by an fma and applied to first order.  The clamp keeps infinities out of that.
+__device__ __forceinline__ float sigmoid_full(float x) {
+  x = fminf(fmaxf(x, -1e4f), 1e4f);
+  const float t = -1.4426950409f * x;
+  const float lost = fmaf(-1.4426950409f, x, -t) - 1.9259630e-8f * x;     // log2 e = 1.44269502 + 1.926e-8
+  return __fdividef(1.f, 1.f + exp2f(t) * fmaf(lost, 0.6931471806f, 1.f));
+}
+// d(x sigmoid(u)) / dx from s = sigmoid(u) and x du/dx.
+__device__ __forceinline__ float sigmoid_slope(float s, float x_du) { return s * (1.f + x_du * (1.f - s)); }
+// Twice the argument of the tanh in the tanh form of GELU: 0.5 (1 + tanh(u)) = sigmoid(2 u), which does not
+// cancel where tanh is close to -1.
+__device__ __forceinline__ float gelu_arg2(float x) { return 1.5957691216f * (x + 0.044715f * x * x * x); }
+
 template <int ACT>
 __device__ __forceinline__ float act_fwd(float x) {
   if constexpr (ACT == kActGeluTanh) return 0.5f * x * (1.f + tanh_fast(0.7978845608f * (x + 0.044715f * x * x * x)));
   else if constexpr (ACT == kActSilu) return x / (1.f + __expf(-x));
   else if constexpr (ACT == kActRelu) return fmaxf(x, 0.f);
   else if constexpr (ACT == kActGeluErf) return 0.5f * x * (1.f + erf_fast(x * 0.70710678f));
+  else if constexpr (ACT == kActGeluTanhFull) return x * sigmoid_full(gelu_arg2(x));
+  else if constexpr (ACT == kActSiluFull) return x * sigmoid_full(x);
+  else if constexpr (ACT == kActGeluErfFull) return 0.5f * x * (1.f + erff(x * 0.70710678f));
   else return x;
 }
 
@@ -157,6 +174,12 @@ __device__ __forceinline__ float act_bwd(float x) {
     return x > 0.f ? 1.f : 0.f;
   } else if constexpr (ACT == kActGeluErf) {
     return 0.5f * (1.f + erf_fast(x * 0.70710678f)) + x * 0.3989422804f * __expf(-0.5f * x * x);
+  } else if constexpr (ACT == kActGeluErfFull) {
+    return 0.5f * (1.f + erff(x * 0.70710678f)) + x * 0.3989422804f * __expf(-0.5f * x * x);
+  } else if constexpr (ACT == kActGeluTanhFull) {
+    return sigmoid_slope(sigmoid_full(gelu_arg2(x)), x * (1.5957691216f + 0.2140644488f * x * x));
+  } else if constexpr (ACT == kActSiluFull) {
+    return sigmoid_slope(sigmoid_full(x), x);
   } else {
     return 1.f;
   }
@@ -587,6 +610,14 @@ __device__ __forceinline__ void epilogue_by_act(const uint32_t (&raw)[32], const
                                                 int64_t row_stride, int rows_ok, int cols, int lane,
                                                 const GemmParams& p, const ScatterRows<T>* scatter, int col,
                                                 TmaOut tma) {
+  if constexpr (EPI == kEpiAct || EPI == kEpiDAct) {
+    switch (p.act) {
+      case kActGeluTanhFull: epilogue_chunk<T, EPI, kActGeluTanhFull, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); return;
+      case kActSiluFull: epilogue_chunk<T, EPI, kActSiluFull, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); return;
+      case kActGeluErfFull: epilogue_chunk<T, EPI, kActGeluErfFull, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); return;
+      default: break;
+    }
+  }
   switch (p.act) {
     case kActGeluTanh: epilogue_chunk<T, EPI, kActGeluTanh, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
     case kActSilu: epilogue_chunk<T, EPI, kActSilu, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;

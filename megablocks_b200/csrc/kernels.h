@@ -218,7 +218,12 @@ constexpr int kMaxGroups = 1024;
 
 enum Layout : int { kNT = 0, kNN = 1, kTN = 2 };
 enum Epilogue : int { kEpiNone = 0, kEpiAct = 1, kEpiDAct = 2, kEpiGlu = 3, kEpiDGlu = 4, kEpiAdd = 5, kEpiGluDual = 6 };
-enum Act : int { kActIdentity = 0, kActGeluTanh = 1, kActSilu = 2, kActRelu = 3, kActGeluErf = 4 };
+// The Full forms (epilogues kEpiAct and kEpiDAct) are as exact as the library's fp32 functions; the plain ones
+// use the hardware tanh and short forms of exp and erf.
+enum Act : int {
+  kActIdentity = 0, kActGeluTanh = 1, kActSilu = 2, kActRelu = 3, kActGeluErf = 4,
+  kActGeluTanhFull = 5, kActSiluFull = 6, kActGeluErfFull = 7
+};
 
 struct GemmParams {
   const int* bins;  // [num_groups] inclusive prefix sum of rows per group

@@ -665,6 +665,8 @@ std::vector<at::Tensor> grouped_gemm_outputs(const at::Tensor& a, const at::Tens
   };
   at::Tensor out2, out3;
   p.epilogue = int(epilogue);
+  TORCH_CHECK(act >= 0 && act <= kActGeluErfFull && (act <= kActGeluErf || epilogue == kEpiAct || epilogue == kEpiDAct),
+              "grouped_gemm: unknown activation for this epilogue");
   p.act = int(act);
   p.alpha = float(alpha);
   p.seq_base = seq_base_ptr(seq_base);

@@ -18,6 +18,7 @@ import torch
 from torch.autograd import forward_ad
 
 from megablocks_b200._ext import ext
+from megablocks_b200.layers.fused_mlp import capacity_act
 from megablocks_b200.ops import gg as G
 from megablocks_b200.utils import debug
 
@@ -118,7 +119,7 @@ def expert_block(x, expert_weights, top_experts, w1, w2, v1, bias, gemm_bins, nu
                  capacity, memory_optimized, wgrad_scale):
     """``(out[tokens, hidden], tokens_per_expert)`` for calls that :func:`route` accepts."""
     x = x.reshape(-1, x.shape[-1]).contiguous()
-    act = G.activation_id(activation_fn)
+    act = capacity_act(activation_fn) if capacity > 0 else G.activation_id(activation_fn)
     tensors = (x, expert_weights, w1, w2, v1, bias)
     if not (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)):
         out, counts = ext().expert_block_forward(x, top_experts, expert_weights, w1, w2, v1, bias, gemm_bins, num_experts,

@@ -162,10 +162,17 @@ def expert_mlp(x: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, bins: torch.
     return _ExpertMLP.apply(x, w1, w2, v1, bins, act, memory_optimized, wgrad_scale)
 
 
+def capacity_act(activation_fn: Optional[Callable]) -> Optional[int]:
+    """Kernel id of the token-dropping experts' activation, ``None`` for an unknown callable.  These experts
+    have the exact forms: their activation is the caller's own function in fp32, not the dropless layers'
+    hardware tanh."""
+    act = G.activation_id(activation_fn)
+    return G.ACT_FULL.get(act, act)
+
+
 def capacity_mlp_fused(x: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, activation_fn: Optional[Callable]) -> bool:
     """Whether :func:`capacity_mlp` takes the token-dropping experts: 16-bit CUDA tensors that the kernel
-    supports and an activation it knows.  fp16 keeps the library's tanh for the tanh form of GELU: the
-    epilogue's hardware tanh is good to 2^-11, below bf16's rounding but not below fp16's."""
+    supports and an activation it knows (fp16 with the tanh form of GELU has stayed on separate passes)."""
     act = G.activation_id(activation_fn)
     return (act is not None and x.is_cuda and x.dtype in (torch.bfloat16, torch.float16)
             and not (x.dtype == torch.float16 and act == G.ACT_GELU_TANH)
@@ -181,5 +188,5 @@ def capacity_mlp(x, w1, w2, bins, activation_fn, wgrad_scale: float = 1.0):
     ``[E * capacity, f]`` they took 45 and 55 us of a 734 us training pass (16384 x 512 x 2048, 64
     experts, bf16).
     """
-    return _ExpertMLP.apply(x, w1.contiguous(), w2.contiguous(), None, bins, G.activation_id(activation_fn), False,
+    return _ExpertMLP.apply(x, w1.contiguous(), w2.contiguous(), None, bins, capacity_act(activation_fn), False,
                             wgrad_scale, True)

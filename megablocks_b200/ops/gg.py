@@ -46,6 +46,10 @@ ACT_GELU_TANH = 1
 ACT_SILU = 2
 ACT_RELU = 3
 ACT_GELU_ERF = 4
+# As exact as the library's fp32 functions (EPI_ACT and EPI_DACT only); the plain ones use the hardware tanh
+# and short forms of exp and erf.
+ACT_FULL = {ACT_GELU_TANH: 5, ACT_SILU: 6, ACT_GELU_ERF: 7}
+_ACT_OF_FULL = {full: plain for plain, full in ACT_FULL.items()}
 
 _ACT_NAMES = {
     'identity': ACT_IDENTITY,
@@ -89,6 +93,7 @@ def activation_id(fn: Optional[Callable]) -> Optional[int]:
 
 
 def act_forward(z: torch.Tensor, act: int) -> torch.Tensor:
+    act = _ACT_OF_FULL.get(act, act)
     if act == ACT_IDENTITY:
         return z
     if act == ACT_GELU_TANH:
@@ -104,6 +109,7 @@ def act_forward(z: torch.Tensor, act: int) -> torch.Tensor:
 
 def act_derivative(z: torch.Tensor, act: int) -> torch.Tensor:
     """d act(z) / dz evaluated in the dtype of ``z`` (callers pass fp32)."""
+    act = _ACT_OF_FULL.get(act, act)
     if act == ACT_IDENTITY:
         return torch.ones_like(z)
     if act == ACT_GELU_TANH:

@@ -5,6 +5,7 @@ glu_test.py:64-123) and adds backward numerics, which the reference only smoke-t
 """
 
 import gc
+import math
 from functools import partial
 
 import pytest
@@ -14,6 +15,7 @@ from conftest import DEVICES
 
 import megablocks_b200 as mb
 from megablocks_b200 import ops
+from megablocks_b200.layers import mlp as mlp_mod
 from megablocks_b200.layers import moe as moe_mod
 from megablocks_b200.layers import router as router_mod
 from megablocks_b200.layers.arguments import from_megatron
@@ -368,6 +370,40 @@ def test_token_dropping_experts_in_gemm_epilogues(act, tokens, hidden, ffn):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize('act,exact', [
+    # In 64 bits, and in the forms that do not cancel where the function is close to zero.
+    (partial(F.gelu, approximate='tanh'), lambda z: z * torch.sigmoid(2 * (2 / math.pi) ** 0.5 * (z + 0.044715 * z ** 3))),
+    (F.silu, F.silu), (F.gelu, lambda z: 0.5 * z * torch.erfc(-z / 2 ** 0.5))], ids=['gelu_tanh', 'silu', 'gelu'])
+def test_token_dropping_activation_is_as_exact_as_the_library(dtype, act, exact):
+    """Activation and derivative at every 16-bit value up to 1e4, through experts whose weights are the
+    identity, in units of the last place from the 64-bit function: the largest and the mean square error are
+    at most the library's fp32 function's, or what one rounding leaves (a half)."""
+    args = mb.Arguments(hidden_size=64, ffn_hidden_size=64, moe_num_experts=1, activation_fn=act, bias=False,
+                        fp16=dtype == torch.float16, bf16=dtype == torch.bfloat16, device=torch.device('cuda'))
+    experts = mlp_mod.MLP(args)
+    with torch.no_grad():
+        experts.w1.copy_(torch.eye(64))
+        experts.w2.copy_(torch.eye(64))
+    z = torch.arange(-32768, 32768, dtype=torch.int32).to(torch.int16).view(dtype)
+    z = torch.where(z.abs() <= 1e4, z, torch.zeros_like(z)).cuda()
+
+    def both(fn, t):
+        t = t.clone().requires_grad_(True)
+        y = fn(t)
+        return [y.detach().double().view(-1), torch.autograd.grad(y, t, torch.ones_like(y))[0].double().view(-1)]
+
+    exact = both(exact, z.double())
+    floor = max(torch.finfo(dtype).smallest_normal, 1e-30)
+    for got, lib, want in zip(both(experts, z.view(1, 1024, 64)), both(act, z), exact):
+        unit = torch.finfo(dtype).eps * torch.exp2(torch.floor(torch.log2(want.abs().clamp_min(floor))))
+        e, ref = (got - want).abs() / unit, (lib - want).abs() / unit
+        # fp32's last place is 2^-13 of fp16's: eight of them may tip a rounding that the library does not.
+        assert float(e.max()) <= max(float(ref.max()), 0.5) + 8 * 2 ** -13
+        assert float(e.square().mean()) <= 1.0001 * float(ref.square().mean())
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize('kind', ['mlp', 'glu', 'dropping'])
 @pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize('tokens,top_k,bias,memory_optimized', [(1, 1, True, False), (37, 2, False, True), (300, 1, True, True)])
@@ -516,7 +552,7 @@ def test_step_replaced_on_the_instance_is_called(kind, step):
     got = layer(x)
     assert calls
     # The bias is added by the kernel or afterwards: one rounding of the sum apart.
-    torch.testing.assert_close(got, want, rtol=2 ** -7, atol=2 ** -7 * float(layer.experts.bias.abs().max()))
+    torch.testing.assert_close(got, want, rtol=2 ** -7, atol=2 ** -7 * float(layer.experts.bias.detach().abs().max()))
 
 
 @pytest.mark.gpu
