@@ -150,11 +150,15 @@ __device__ __forceinline__ float sigmoid_slope(float s, float x_du) { return s *
 // cancel where tanh is close to -1.
 __device__ __forceinline__ float gelu_arg2(float x) { return 1.5957691216f * (x + 0.044715f * x * x * x); }
 
+// Whether ReLU gives zero: every x <= 0, but not NaN, which has to stay visible.  On the bits, since the
+// comparison takes positive subnormals for zero (they are flushed).
+__device__ __forceinline__ bool relu_zeroes(float x) { return __float_as_int(x) <= 0 && x == x; }
+
 template <int ACT>
 __device__ __forceinline__ float act_fwd(float x) {
   if constexpr (ACT == kActGeluTanh) return 0.5f * x * (1.f + tanh_fast(0.7978845608f * (x + 0.044715f * x * x * x)));
   else if constexpr (ACT == kActSilu) return x / (1.f + __expf(-x));
-  else if constexpr (ACT == kActRelu) return fmaxf(x, 0.f);
+  else if constexpr (ACT == kActRelu) return relu_zeroes(x) ? 0.f : x;
   else if constexpr (ACT == kActGeluErf) return 0.5f * x * (1.f + erf_fast(x * 0.70710678f));
   else if constexpr (ACT == kActGeluTanhFull) return x * sigmoid_full(gelu_arg2(x));
   else if constexpr (ACT == kActSiluFull) return x * sigmoid_full(x);
@@ -171,7 +175,7 @@ __device__ __forceinline__ float act_bwd(float x) {
     const float s = 1.f / (1.f + __expf(-x));
     return s * (1.f + x * (1.f - s));
   } else if constexpr (ACT == kActRelu) {
-    return x > 0.f ? 1.f : 0.f;
+    return relu_zeroes(x) ? 0.f : 1.f;
   } else if constexpr (ACT == kActGeluErf) {
     return 0.5f * (1.f + erf_fast(x * 0.70710678f)) + x * 0.3989422804f * __expf(-0.5f * x * x);
   } else if constexpr (ACT == kActGeluErfFull) {
@@ -444,6 +448,9 @@ __device__ __forceinline__ void dact_values(float acc, float z, float& dz, float
     const float sg = 1.f / (1.f + __expf(-z));
     h = z * sg;
     dz = acc * (sg * (1.f + z * (1.f - sg)));
+  } else if constexpr (ACT == kActRelu) {
+    h = act_fwd<ACT>(z);
+    dz = relu_zeroes(z) ? 0.f : acc;      // a closed unit passes no gradient, not even an infinite one
   } else {
     h = act_fwd<ACT>(z);
     dz = acc * act_bwd<ACT>(z);

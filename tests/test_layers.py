@@ -404,6 +404,32 @@ def test_token_dropping_activation_is_as_exact_as_the_library(dtype, act, exact)
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float16])
+def test_token_dropping_relu_shows_nan_and_closes_like_the_library(dtype):
+    """ReLU in the epilogues against the library's: NaN stays NaN, closed units pass no gradient (an infinite
+    one included), and every other 16-bit value goes through."""
+    args = mb.Arguments(hidden_size=64, ffn_hidden_size=64, moe_num_experts=2, activation_fn=F.relu, bias=False,
+                        fp16=dtype == torch.float16, bf16=dtype == torch.bfloat16, device=torch.device('cuda'))
+    experts = mlp_mod.MLP(args)
+    with torch.no_grad():
+        for w in experts.parameters():
+            w.copy_(torch.eye(64))
+    z = torch.arange(-32768, 32768, dtype=torch.int32).to(torch.int16).view(dtype).cuda()
+    z = torch.where(z.abs() < float('inf'), z, torch.zeros_like(z)).view(2, 512, 64).requires_grad_(True)
+    y = experts(z)
+    dz, = torch.autograd.grad(y, z, torch.ones_like(y))
+    lib = F.relu(z.detach())
+    # The multiplication by one flushes fp32 subnormals (bf16's own) to zero.
+    normal = (lib >= 2.0 ** -120) | (lib == 0)
+    assert torch.equal(y[normal], lib[normal]) and float(y[~normal].abs().max() if (~normal).any() else 0) < 2.0 ** -119
+    assert torch.equal(dz[normal], (z > 0).to(dtype)[normal])
+    x = torch.randn(2, 8, 64, device='cuda').to(dtype)
+    x[1, 3, 5] = float('nan')
+    out = experts(x)
+    assert out[1, 3].isnan().all() and int(out.isnan().sum()) == 64
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize('kind', ['mlp', 'glu', 'dropping'])
 @pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize('tokens,top_k,bias,memory_optimized', [(1, 1, True, False), (37, 2, False, True), (300, 1, True, True)])
