@@ -582,6 +582,21 @@ def test_step_replaced_on_the_instance_is_called(kind, step):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize('kind', ['mlp', 'sparse', 'dropping'])
+def test_tangent_of_the_output_bias(kind):
+    """Forward-mode differentiation with respect to the output bias: its tangent on every row."""
+    from torch.autograd import forward_ad
+    experts = _stock_layer(kind, hidden=128, ffn=256).experts.requires_grad_(False)
+    x, scores, weights = (torch.rand(37, n, device='cuda').bfloat16() for n in (128, 5, 2))
+    ids = torch.randint(0, 5, (37, 2), device='cuda')
+    tangent = torch.randn(128, device='cuda').bfloat16()
+    with forward_ad.dual_level():
+        bias = forward_ad.make_dual(experts.bias.detach(), tangent)
+        out = torch.func.functional_call(experts, {'bias': bias}, (x, scores, weights, ids))
+        assert torch.equal(forward_ad.unpack_dual(out).tangent, tangent.expand(37, 128))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
 def test_column_sum_of_rows_at_any_address(dtype):
     from megablocks_b200._ext import ext
