@@ -118,7 +118,7 @@ def route(x, expert_weights, top_experts, mlp, w1, w2, v1, bias, activation_fn) 
 def expert_block(x, expert_weights, top_experts, w1, w2, v1, bias, gemm_bins, num_experts, top_k, activation_fn,
                  capacity, memory_optimized, wgrad_scale):
     """``(out[tokens, hidden], tokens_per_expert)`` for calls that :func:`route` accepts."""
-    x = x.reshape(-1, x.shape[-1]).contiguous()
+    x, top_experts = x.reshape(-1, x.shape[-1]).contiguous(), top_experts.contiguous()
     act = capacity_act(activation_fn) if capacity > 0 else G.activation_id(activation_fn)
     tensors = (x, expert_weights, w1, w2, v1, bias)
     if not (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)):

@@ -597,6 +597,17 @@ def test_tangent_of_the_output_bias(kind):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize('kind', ['mlp', 'dropping'])
+def test_expert_ids_of_any_stride(kind):
+    experts = _stock_layer(kind, top_k=1).experts
+    x, scores, weights = (torch.rand(37, n, device='cuda').bfloat16() for n in (72, 5, 1))
+    ids = torch.randint(0, 5, (37, 2), device='cuda')[:, 0]
+    assert not ids.is_contiguous()
+    with torch.no_grad():
+        assert torch.equal(experts(x, scores, weights, ids), experts(x, scores, weights, ids.contiguous()))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
 def test_column_sum_of_rows_at_any_address(dtype):
     from megablocks_b200._ext import ext
