@@ -65,6 +65,12 @@ _ACT_NAMES = {
 _PAIR_MODE = int(os.environ.get('MB200_GEMM_PAIR', '-1'))
 
 
+def _plain(fn, cls) -> bool:
+    """Whether calling ``fn`` is ``cls``'s own forward and nothing else (no subclass's, no hooks)."""
+    return (isinstance(fn, cls) and type(fn).forward is cls.forward and 'forward' not in fn.__dict__
+            and not (fn._forward_hooks or fn._forward_pre_hooks or fn._backward_hooks or fn._backward_pre_hooks))
+
+
 def activation_id(fn: Optional[Callable]) -> Optional[int]:
     """Kernel id of a known activation callable; ``None`` for anything else."""
     if fn is None:
@@ -83,11 +89,11 @@ def activation_id(fn: Optional[Callable]) -> Optional[int]:
         return ACT_SILU
     if fn is F.relu or fn is torch.relu:
         return ACT_RELU
-    if isinstance(fn, torch.nn.GELU):
+    if _plain(fn, torch.nn.GELU):
         return ACT_GELU_TANH if fn.approximate == 'tanh' else ACT_GELU_ERF
-    if isinstance(fn, torch.nn.SiLU):
+    if _plain(fn, torch.nn.SiLU):
         return ACT_SILU
-    if isinstance(fn, torch.nn.ReLU):
+    if _plain(fn, torch.nn.ReLU):
         return ACT_RELU
     return None
 

@@ -19,6 +19,7 @@ from megablocks_b200.layers import mlp as mlp_mod
 from megablocks_b200.layers import moe as moe_mod
 from megablocks_b200.layers import router as router_mod
 from megablocks_b200.layers.arguments import from_megatron
+from megablocks_b200.ops import gg as ops_gg
 
 CONFIGS = [(8, 16, 128, 1, 1), (8, 16, 128, 2, 1), (8, 16, 128, 4, 1), (8, 16, 128, 4, 2), (8, 16, 256, 8, 4),
            (2, 64, 128, 8, 2), (1, 33, 128, 5, 3)]
@@ -272,6 +273,31 @@ def test_arguments_defaults_and_from_megatron():
 
     b = from_megatron(NS())
     assert b.hidden_size == 64 and b.moe_num_experts == 4
+
+
+@pytest.mark.parametrize('device', DEVICES)
+@pytest.mark.parametrize('dropless', [True, False])
+def test_activation_modules_with_a_forward_or_hooks_of_their_own(device, dropless):
+    """A subclass of a known activation module computes what it says, and hooks on one are called."""
+
+    class Twice(torch.nn.GELU):
+
+        def forward(self, z):
+            return 2 * super().forward(z)
+
+    def run(act):
+        torch.manual_seed(0)
+        layer = (mb.dMoE if dropless else mb.MoE)(_args(device, activation_fn=act, mlp_impl='grouped', bias=False,
+                                                        return_bias=False))
+        return layer(torch.randn(8, 2, 128).to(device, next(layer.parameters()).dtype)).float()
+
+    torch.testing.assert_close(run(Twice()), run(lambda z: 2 * F.gelu(z)), **_tol(device))
+    act, calls = torch.nn.SiLU(), []
+    act.register_forward_hook(lambda *a: calls.append(1))
+    run(act)
+    assert calls
+    assert [ops_gg.activation_id(m) for m in (torch.nn.GELU(), torch.nn.GELU('tanh'), torch.nn.SiLU(), torch.nn.ReLU())] == [
+        ops_gg.ACT_GELU_ERF, ops_gg.ACT_GELU_TANH, ops_gg.ACT_SILU, ops_gg.ACT_RELU]
 
 
 @pytest.mark.parametrize('device', DEVICES)
