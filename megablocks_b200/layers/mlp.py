@@ -106,6 +106,10 @@ class _ExpertWeights(torch.nn.Module):
             return w
         return scale_gradient(w, self.gradient_scale)
 
+    def _scales_as_usual(self) -> bool:
+        """Whether ``wgrad_scale`` says all that ``scale_grad`` does (neither replaced)."""
+        return type(self).scale_grad is _ExpertWeights.scale_grad and 'scale_grad' not in self.__dict__
+
     def wgrad_scale(self) -> float:
         """Factor for the fused expert MLP, which scales weight gradients inside their GEMMs."""
         return 1.0 if self.gradient_scale is None else float(self.gradient_scale)
@@ -141,7 +145,7 @@ class MLP(_ExpertWeights):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         experts, capacity, hidden = x.shape
-        if capacity > 0:
+        if capacity > 0 and self._scales_as_usual():
             w1, w2 = resolve_dtensor(self.w1), resolve_dtensor(self.w2)
             if capacity_mlp_fused(x, w1, w2, self.args.activation_fn):
                 y = capacity_mlp(x.reshape(experts * capacity, hidden), w1, w2,

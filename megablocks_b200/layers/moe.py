@@ -197,8 +197,8 @@ class ParallelMLP(torch.nn.Module):
         """Expert tensors of the single native call: ``(w1, w2, v1, gemm_bins, capacity, memory_optimized)``."""
         m = self.mlp
         capacity = self.expert_capacity(tokens)
-        if type(m) is not mlp.MLP or capacity <= 0 or not m.w1.is_cuda or not capacity_mlp_fused(
-                m.w1, m.w1, m.w2, self.args.activation_fn):
+        if (type(m) is not mlp.MLP or capacity <= 0 or not m.w1.is_cuda or not m._scales_as_usual()
+                or not capacity_mlp_fused(m.w1, m.w1, m.w2, self.args.activation_fn)):
             return None
         return m.w1, m.w2, None, m._uniform_bins(self.num_experts, capacity, m.w1.device), capacity, False
 

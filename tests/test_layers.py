@@ -276,6 +276,24 @@ def test_arguments_defaults_and_from_megatron():
 
 
 @pytest.mark.parametrize('device', DEVICES)
+@pytest.mark.parametrize('on_instance', [True, False])
+def test_replaced_scaling_of_the_token_dropping_weights_is_used(device, on_instance):
+    layer = mb.MoE(_args(device, activation_fn=F.silu, bias=False, return_bias=False))
+    x = torch.randn(64, 1, 128).to(device, next(layer.parameters()).dtype)
+    with torch.no_grad():
+        for w in layer.experts.mlp.parameters():
+            w.mul_(2)
+        want = layer(x)
+        for w in layer.experts.mlp.parameters():
+            w.mul_(0.5)
+        if on_instance:
+            layer.experts.mlp.scale_grad = lambda w: w * 2
+        else:
+            layer.experts.mlp.__class__ = type('Scaled', (mlp_mod.MLP,), {'scale_grad': lambda self, w: w * 2})
+        torch.testing.assert_close(layer(x), want, **_tol(device))
+
+
+@pytest.mark.parametrize('device', DEVICES)
 @pytest.mark.parametrize('dropless', [True, False])
 def test_activation_modules_with_a_forward_or_hooks_of_their_own(device, dropless):
     """A subclass of a known activation module computes what it says, and hooks on one are called."""
