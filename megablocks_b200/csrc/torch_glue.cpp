@@ -656,12 +656,17 @@ std::vector<at::Tensor> grouped_gemm_outputs(const at::Tensor& a, const at::Tens
   TORCH_CHECK(!only_out2 || (layout != kTN && !c_in.has_value() && !scatter.has_value() && want_out2 &&
                              (epilogue == kEpiAct || epilogue == kEpiGluDual)),
               "an activation alone: activation epilogues of the NT / NN layouts only");
-  TORCH_CHECK(only_out2 || (c.is_contiguous() && c.scalar_type() == a.scalar_type()), "bad output buffer");
+  // Outputs and auxiliary operands move 16 bytes at a time, too.
+  TORCH_CHECK(only_out2 || (c.is_contiguous() && c.scalar_type() == a.scalar_type() &&
+                            reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 == 0),
+              "grouped_gemm: the output buffer must be contiguous, of the operands' type and 16-byte aligned");
+  TORCH_CHECK(!c_in.has_value() || c.numel() >= (layout == kTN ? num_groups * int64_t(p.M) : a.size(0)) * int64_t(p.N),
+              "grouped_gemm: the output buffer is too small");
   const int64_t out_numel = scatter.has_value() || only_out2 ? a.size(0) * int64_t(p.N) : c.numel();
   auto check_aux = [&](const c10::optional<at::Tensor>& t, const char* name) {
     TORCH_CHECK(t.has_value() && t->is_cuda() && t->is_contiguous() && t->numel() == out_numel &&
-                    t->scalar_type() == a.scalar_type(),
-                name, " must match the output in shape and dtype");
+                    t->scalar_type() == a.scalar_type() && reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0,
+                name, " must match the output in shape and dtype and be 16-byte aligned");
   };
   at::Tensor out2, out3;
   p.epilogue = int(epilogue);

@@ -1,5 +1,6 @@
 """Grouped GEMM (all layouts and fused epilogues) against per-group fp32 matmuls."""
 
+import math
 import os
 import subprocess
 import sys
@@ -437,3 +438,23 @@ def test_backward_as_the_first_cuda_work_of_its_thread():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     run = subprocess.run([sys.executable, '-c', _FIRST_IN_THREAD.format(root=root)], capture_output=True, text=True, timeout=300)
     assert run.returncode == 0 and 'done' in run.stdout, run.stderr[-2000:]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('which', ['a', 'b', 'c', 'aux1'])
+def test_misaligned_operands_and_short_outputs_are_refused_on_the_host(which):
+    """Everything a grouped GEMM touches moves 16 bytes at a time: a contiguous tensor that starts at an odd
+    element is an error and not an access."""
+    bins = torch.tensor([40, 100], dtype=torch.int32, device='cuda')
+    odd = lambda *shape: torch.randn(math.prod(shape) + 8, device='cuda').bfloat16()[1:1 + math.prod(shape)].view(shape)
+    even = lambda *shape: torch.randn(*shape, device='cuda').bfloat16()
+    shapes = dict(a=(100, 64), b=(2, 64, 72), c=(100, 72), aux1=(100, 72))
+    t = {name: (odd if name == which else even)(*shape) for name, shape in shapes.items()}
+    with pytest.raises(RuntimeError):
+        G.grouped_gemm(t['a'], t['b'], bins, c=t['c'], aux1=t['aux1'], epilogue=G.EPI_ADD)
+    with pytest.raises(RuntimeError):
+        G.grouped_gemm(even(100, 64), even(2, 64, 72), bins, c=even(99, 72))
+    # The refused launches have left the device usable.
+    out, _, _ = G.grouped_gemm(even(100, 64), even(2, 64, 72), bins, c=even(100, 72), aux1=even(100, 72),
+                               epilogue=G.EPI_ADD)
+    assert bool(out.isfinite().all())
