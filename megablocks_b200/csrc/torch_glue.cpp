@@ -230,6 +230,13 @@ std::vector<at::Tensor> route_plan_rows(const at::Tensor& top_experts, int64_t n
   return plan;
 }
 
+static void check_out_bias(const c10::optional<at::Tensor>& bias, const at::Tensor& x) {
+  if (!bias.has_value()) return;
+  TORCH_CHECK(bias->is_cuda() && bias->get_device() == x.get_device() && bias->is_contiguous() && bias->dim() == 1 &&
+                  bias->scalar_type() == x.scalar_type() && bias->numel() == x.size(-1),
+              "bias must be a contiguous vector of one value per column, of the rows' type");
+}
+
 // out[t] = sum of the rows of token t's copies (weighted, plus bias); `inverse` as above.
 at::Tensor combine_rows_op(const at::Tensor& x, const at::Tensor& inverse, const c10::optional<at::Tensor>& weights,
                            int64_t top_k, int64_t tokens, const c10::optional<at::Tensor>& bias) {
@@ -238,6 +245,7 @@ at::Tensor combine_rows_op(const at::Tensor& x, const at::Tensor& inverse, const
   check_index(inverse, "inverse");
   TORCH_CHECK(inverse.numel() == tokens * top_k, "one row per copy expected");
   check_weights(weights, x, inverse.numel());
+  check_out_bias(bias, x);
   c10::cuda::CUDAGuard guard(x.device());
   at::Tensor out = at::empty({tokens, x.size(1)}, x.options());
   if (out.numel() == 0) return out;
@@ -331,13 +339,6 @@ at::Tensor gather_rows_op(const at::Tensor& x, const at::Tensor& indices, const 
                          out_rows, int(x.size(1)), out.data_ptr(), stream()));
   MB_LAUNCHED(1);
   return out;
-}
-
-static void check_out_bias(const c10::optional<at::Tensor>& bias, const at::Tensor& x) {
-  if (!bias.has_value()) return;
-  TORCH_CHECK(bias->is_cuda() && bias->get_device() == x.get_device() && bias->is_contiguous() && bias->dim() == 1 &&
-                  bias->scalar_type() == x.scalar_type() && bias->numel() == x.size(-1),
-              "bias must be a contiguous vector of one value per column, of the rows' type");
 }
 
 at::Tensor scatter_rows_op(const at::Tensor& x, const at::Tensor& indices, const at::Tensor& bin_ids,

@@ -110,7 +110,7 @@ def route(x, expert_weights, top_experts, mlp, w1, w2, v1, bias, activation_fn) 
             return False
     if (hidden % 8 or ffn % 8 or hidden < 64 or ffn < 64 or experts > 1024 or (v1 is not None and ffn < 128)
             or hidden != x.shape[-1] or top_experts.numel() != expert_weights.numel()
-            or (bias is not None and bias.data_ptr() % 16)):
+            or (bias is not None and (bias.data_ptr() % 16 or bias.shape != (hidden,)))):
         return False
     return G.activation_id(activation_fn) is not None and not _hooked(mlp) and not special_mode()
 

@@ -144,13 +144,14 @@ class ParallelMLP(torch.nn.Module):
     def _unpermute_bias(self, x: torch.Tensor):
         """The output bias if the un-permutation kernel can add it on its way out, else ``None``.
 
-        Only where the sum has the type of the activations (no autocast, no sharded parameter) and no tangent
+        Only where the sum has the type of the activations (no autocast, no sharded parameter), the bias one
+        value per column (an addition would broadcast any other) and no tangent
         rides on the bias (the un-permutation's node has no forward-mode derivative).
         """
         bias = self.bias
         if (bias is None or self.args.return_bias or not x.is_cuda or bias.dtype != x.dtype
                 or x.dtype not in (torch.bfloat16, torch.float16, torch.float32) or not bias.is_contiguous()
-                or bias.device != x.device or hasattr(bias, 'to_local') or torch.is_autocast_enabled('cuda')
+                or bias.device != x.device or bias.shape != x.shape[-1:] or hasattr(bias, 'to_local') or torch.is_autocast_enabled('cuda')
                 or forward_ad._current_level >= 0):
             return None
         return bias if self._stock(self._bias_base._bias_steps) else None

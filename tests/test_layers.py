@@ -652,6 +652,24 @@ def test_expert_ids_of_any_stride(kind):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize('kind', ['mlp', 'sparse', 'dropping'])
+@pytest.mark.parametrize('shape', [(1,), (37, 128), ()])
+def test_output_bias_of_another_shape_is_broadcast(kind, shape):
+    """A bias that is not one value per column never reaches the kernels, which read one per column."""
+    layer = _stock_layer(kind, hidden=128, ffn=256)
+    x = torch.randn(37, 128, device='cuda').bfloat16()
+    with torch.no_grad():
+        layer.experts.bias.zero_()
+        plain = layer(x)
+        layer.experts.bias = torch.nn.Parameter(torch.randn(shape, device='cuda').bfloat16())
+        assert torch.equal(layer(x), plain + layer.experts.bias)
+    from megablocks_b200._ext import ext
+    rows = torch.arange(37, dtype=torch.int32, device='cuda')
+    with pytest.raises(RuntimeError, match='bias'):
+        ext().combine_rows(x, rows, None, 1, 37, x.new_zeros(64))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
 def test_column_sum_of_rows_at_any_address(dtype):
     from megablocks_b200._ext import ext
