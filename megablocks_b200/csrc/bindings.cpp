@@ -73,9 +73,9 @@ std::vector<at::Tensor> expert_block_forward(const at::Tensor& x, const at::Tens
                                              const c10::optional<at::Tensor>& v1, const c10::optional<at::Tensor>& bias,
                                              const c10::optional<at::Tensor>& gemm_bins, int64_t num_experts,
                                              int64_t top_k, int64_t act, int64_t capacity, int64_t pair);
-std::vector<at::Tensor> expert_combine_backward(const at::Tensor& dout, const at::Tensor& indices, const at::Tensor& bins,
-                                                const at::Tensor& y, const at::Tensor& weights,
-                                                const std::vector<bool>& needs, int64_t top_k, int64_t capacity);
+at::Tensor expert_combine(const at::Tensor& y, const at::Tensor& weights, const c10::optional<at::Tensor>& bias,
+                          const at::Tensor& indices, const at::Tensor& inverse, const at::Tensor& bins, int64_t top_k,
+                          int64_t capacity);
 std::vector<at::Tensor> expert_rows_backward(
     const at::Tensor& dy, const at::Tensor& inverse, const at::Tensor& bins, const c10::optional<at::Tensor>& gemm_bins,
     const at::Tensor& rows, const at::Tensor& z1, const c10::optional<at::Tensor>& z2,
@@ -176,7 +176,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("expert_block_forward", &mb::expert_block_forward);
   m.def("expert_rows_forward", &mb::expert_rows_forward);
   m.def("expert_rows_backward", &mb::expert_rows_backward);
-  m.def("expert_combine_backward", &mb::expert_combine_backward);
+  m.def("expert_combine", &mb::expert_combine);
   m.def("read_status", &mb::read_status);
   m.def("launch_count", &mb::launch_count);
   m.def("count_launches", &mb::count_launches);

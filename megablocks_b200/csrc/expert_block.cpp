@@ -1,6 +1,6 @@
 // The routed expert computation of one device - plan, permute, expert GEMMs, weighted un-permute - as one
-// native call where nothing is differentiated, else as two each way (the experts, the un-permutation),
-// each behind an autograd node.  The kernels are those behind the separate ops; what this saves is the
+// native call where nothing is differentiated, else as two each way (the experts, the un-permutation), each
+// behind an autograd node.  The kernels are those behind the separate ops; what this saves is the
 // host's time between them: some 20 us of Python per op (an autograd node, argument checks and
 // conversions), which bounds small calls (a decode step of 8 tokens has 60 us of kernels, a 256-token
 // training pass 110).  Two nodes and not one, because y, which only the un-permutation's backward reads,
@@ -106,23 +106,52 @@ std::vector<at::Tensor> expert_block_forward(const at::Tensor& x, const at::Tens
   return {combine_rows_op(o[0], o[3], weights, top_k, x.size(0), bias), o[1]};
 }
 
-// {dy, dweights, dbias} of the un-permutation, undefined where `needs` says so.
-std::vector<at::Tensor> expert_combine_backward(const at::Tensor& dout, const at::Tensor& indices, const at::Tensor& bins,
-                                                const at::Tensor& y, const at::Tensor& weights,
-                                                const std::vector<bool>& needs, int64_t top_k, int64_t capacity) {
-  const bool binned = capacity > 0;
-  const at::Tensor slots = binned ? y.view({bins.numel(), capacity, y.size(1)}) : y;
-  at::Tensor dy, dweights, dbias;
-  if (needs[2]) dbias = column_sum_op(dout);
-  if (needs[0]) {
-    auto un = scatter_backward_op(slots, dout, indices, weights, bins, binned ? OptTensor() : OptTensor(bins), top_k);
-    dy = rows_of(un[0]);
-    if (needs[1]) dweights = un[1];
-  } else if (needs[1]) {
-    dweights = binned ? binned_scatter_wgrad(slots, dout, indices, bins, top_k)
-                      : scatter_wgrad_op(slots, dout, indices, indices, bins, bins, top_k);
+namespace {
+
+// Weighted un-permutation and output bias behind a node of its own: it alone keeps y, and frees it before the
+// experts' backward starts.  A C++ node, which the host passes in a few microseconds each way where a Python
+// one takes some 15.
+struct Combine : torch::autograd::Function<Combine> {
+  static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& y, const at::Tensor& weights,
+                            const OptTensor& bias, const at::Tensor& indices, const at::Tensor& inverse,
+                            const at::Tensor& bins, int64_t top_k, int64_t capacity) {
+    ctx->save_for_backward({y, weights, indices, bins});
+    ctx->saved_data["top_k"] = top_k;
+    ctx->saved_data["capacity"] = capacity;
+    ctx->saved_data["bias"] = bias.has_value();
+    ctx->set_materialize_grads(false);
+    return combine_rows_op(y, inverse, weights, top_k, inverse.numel() / top_k, bias);
   }
-  return {dy, dweights, dbias};
+
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
+                                                 torch::autograd::variable_list grads) {
+    torch::autograd::variable_list out(8);      // undefined: no gradient
+    if (!grads[0].defined()) return out;
+    const auto saved = ctx->get_saved_variables();
+    const at::Tensor &weights = saved[1], &indices = saved[2], &bins = saved[3];
+    const int64_t top_k = ctx->saved_data["top_k"].toInt(), capacity = ctx->saved_data["capacity"].toInt();
+    const at::Tensor dout = grads[0].contiguous();
+    const bool binned = capacity > 0;
+    const at::Tensor y = binned ? saved[0].view({bins.numel(), capacity, saved[0].size(1)}) : saved[0];
+    if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2)) out[2] = column_sum_op(dout);
+    if (ctx->needs_input_grad(0)) {
+      auto un = scatter_backward_op(y, dout, indices, weights, bins, binned ? OptTensor() : OptTensor(bins), top_k);
+      out[0] = rows_of(un[0]);
+      if (ctx->needs_input_grad(1)) out[1] = un[1];
+    } else if (ctx->needs_input_grad(1)) {
+      out[1] = binned ? binned_scatter_wgrad(y, dout, indices, bins, top_k)
+                      : scatter_wgrad_op(y, dout, indices, indices, bins, bins, top_k);
+    }
+    return out;
+  }
+};
+
+}  // namespace
+
+at::Tensor expert_combine(const at::Tensor& y, const at::Tensor& weights, const OptTensor& bias,
+                          const at::Tensor& indices, const at::Tensor& inverse, const at::Tensor& bins, int64_t top_k,
+                          int64_t capacity) {
+  return Combine::apply(y, weights, bias, indices, inverse, bins, top_k, capacity);
 }
 
 // {dx, dw1, dw2, dv1} from the gradient of y, undefined where `needs` says so.  `slots`: per weight gradient

@@ -24,11 +24,13 @@ from megablocks_b200.utils import debug
 
 
 class _Experts(torch.autograd.Function):
-    """Plan, permutation and expert GEMMs: the copies' results in expert order, and the plan."""
+    """Plan, permutation and expert GEMMs: the copies' results in expert order.  ``plan`` is a list that
+    receives ``(tokens_per_expert, indices, inverse, bins)``; as outputs of the node they would each cost the
+    host a wrapper."""
 
     @staticmethod
-    def forward(ctx: Any, x, top_experts, w1, w2, v1, gemm_bins, num_experts, top_k, act, capacity, memory_optimized,
-                wgrad_scale):
+    def forward(ctx: Any, x, top_experts, w1, w2, v1, gemm_bins, plan, num_experts, top_k, act, capacity,
+                memory_optimized, wgrad_scale):
         need = ctx.needs_input_grad
         keep = need[0] or need[2] or need[3] or need[4]
         y, counts, indices, inverse, bins, *kept = ext().expert_rows_forward(
@@ -38,14 +40,14 @@ class _Experts(torch.autograd.Function):
             ctx.save_for_backward(w1, w2, v1, gemm_bins, inverse, bins, rows, z1, z2 if v1 is not None else None,
                                   None if memory_optimized else h)
         ctx.top_k, ctx.act, ctx.capacity, ctx.wgrad_scale = top_k, act, capacity, wgrad_scale
-        ctx.mark_non_differentiable(counts, indices, inverse, bins)
-        ctx.set_materialize_grads(False)        # no zero tensors for the plan
-        return y, counts, indices, inverse, bins
+        ctx.set_materialize_grads(False)
+        plan += (counts, indices, inverse, bins)
+        return y
 
     @staticmethod
-    def backward(ctx: Any, dy, *_plan):
+    def backward(ctx: Any, dy):
         if dy is None:
-            return (None,) * 12
+            return (None,) * 13
         w1, w2, v1, gemm_bins, inverse, bins, rows, z1, z2, h = ctx.saved_tensors
         need = ctx.needs_input_grad
         needs = [need[0], need[2], need[3], need[4]]
@@ -61,28 +63,7 @@ class _Experts(torch.autograd.Function):
         for k in (1, 0, 2):
             if slots[k] is not None:
                 sink._record(dw[k], slots[k])
-        return (dx, None, *dw) + (None,) * 7
-
-
-class _Combine(torch.autograd.Function):
-    """Weighted un-permutation and output bias.  A node of its own: it alone keeps ``y``, and frees it before
-    the experts' backward starts."""
-
-    @staticmethod
-    def forward(ctx: Any, y, weights, bias, indices, inverse, bins, top_k, capacity):
-        ctx.save_for_backward(y, weights, indices, bins)
-        ctx.top_k, ctx.capacity = top_k, capacity
-        ctx.set_materialize_grads(False)
-        return ext().combine_rows(y, inverse, weights, top_k, inverse.numel() // top_k, bias)
-
-    @staticmethod
-    def backward(ctx: Any, dout):
-        if dout is None:
-            return (None,) * 8
-        y, weights, indices, bins = ctx.saved_tensors
-        dy, dweights, dbias = ext().expert_combine_backward(dout.contiguous(), indices, bins, y, weights,
-                                                            list(ctx.needs_input_grad[:3]), ctx.top_k, ctx.capacity)
-        return (dy, dweights, dbias) + (None,) * 5
+        return (dx, None, *dw) + (None,) * 8
 
 
 def _hooked(module: torch.nn.Module) -> bool:
@@ -125,6 +106,8 @@ def expert_block(x, expert_weights, top_experts, w1, w2, v1, bias, gemm_bins, nu
         out, counts = ext().expert_block_forward(x, top_experts, expert_weights, w1, w2, v1, bias, gemm_bins, num_experts,
                                                  top_k, act, capacity, G._PAIR_MODE)
         return out, counts
-    y, counts, indices, inverse, bins = _Experts.apply(x, top_experts, w1, w2, v1, gemm_bins, num_experts, top_k, act,
-                                                       capacity, memory_optimized, wgrad_scale)
-    return _Combine.apply(y, expert_weights, bias, indices, inverse, bins, top_k, capacity), counts
+    plan = []
+    y = _Experts.apply(x, top_experts, w1, w2, v1, gemm_bins, plan, num_experts, top_k, act, capacity,
+                       memory_optimized, wgrad_scale)
+    counts, indices, inverse, bins = plan
+    return ext().expert_combine(y, expert_weights, bias, indices, inverse, bins, top_k, capacity), counts
