@@ -3,6 +3,8 @@
 
 #include <vector>
 
+#include "torch_ops.h"
+
 namespace mb {
 
 // torch_glue.cpp: metadata
@@ -15,27 +17,13 @@ at::Tensor replicate_forward(const at::Tensor& x, const at::Tensor& bins, int64_
 at::Tensor replicate_backward(const at::Tensor& grad, const at::Tensor& bins);
 
 // torch_glue.cpp: permutation
-at::Tensor gather_rows_op(const at::Tensor& x, const at::Tensor& indices, const at::Tensor& bin_ids,
-                       const c10::optional<at::Tensor>& weights, const at::Tensor& bins,
-                       const at::Tensor& padded_bins, int64_t top_k, int64_t out_rows);
 at::Tensor scatter_rows_op(const at::Tensor& x, const at::Tensor& indices, const at::Tensor& bin_ids,
                         const c10::optional<at::Tensor>& weights, const at::Tensor& bins,
                         const at::Tensor& padded_bins, int64_t top_k, int64_t tokens,
                         const c10::optional<at::Tensor>& bias);
-std::vector<at::Tensor> scatter_backward_op(const at::Tensor& x, const at::Tensor& grad, const at::Tensor& indices,
-                                            const at::Tensor& weights, const at::Tensor& bins,
-                                            const c10::optional<at::Tensor>& padded_bins, int64_t top_k);
-at::Tensor scatter_wgrad_op(const at::Tensor& x, const at::Tensor& grad, const at::Tensor& indices,
-                         const at::Tensor& bin_ids, const at::Tensor& bins, const at::Tensor& padded_bins,
-                         int64_t top_k);
-at::Tensor binned_gather_rows(const at::Tensor& x, const at::Tensor& indices,
-                              const c10::optional<at::Tensor>& weights, const at::Tensor& bins, int64_t capacity,
-                              int64_t top_k);
 at::Tensor binned_scatter_rows(const at::Tensor& x, const at::Tensor& indices,
                                const c10::optional<at::Tensor>& weights, const at::Tensor& bins, int64_t top_k,
                                int64_t tokens, const c10::optional<at::Tensor>& bias);
-at::Tensor binned_scatter_wgrad(const at::Tensor& x, const at::Tensor& grad, const at::Tensor& indices,
-                                const at::Tensor& bins, int64_t top_k);
 
 // torch_glue.cpp: router
 std::vector<at::Tensor> router_topk_forward(const at::Tensor& logits, int64_t top_k, double norm_p);
@@ -45,23 +33,6 @@ at::Tensor router_topk_backward(const at::Tensor& scores, const at::Tensor& weig
 // torch_glue.cpp: grouped GEMM
 bool grouped_gemm_supported(const at::Tensor& a, const at::Tensor& b, bool trans_a, bool trans_b,
                             int64_t num_groups);
-std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, const at::Tensor& bins, bool trans_a,
-                                     bool trans_b, int64_t epilogue, int64_t act,
-                                     const c10::optional<at::Tensor>& aux1, const c10::optional<at::Tensor>& aux2,
-                                     bool want_out2, bool want_out3, int64_t num_groups,
-                                     const c10::optional<at::Tensor>& c_in, bool zero_tail,
-                                     const c10::optional<at::Tensor>& wait_flags, int64_t wait_count,
-                                     int64_t wait_stride, int64_t wait_seq, int64_t rows_hint, int64_t pair_mode,
-                                     const c10::optional<std::vector<at::Tensor>>& scatter,
-                                     const std::vector<int64_t>& scatter_args, double alpha,
-                                     const c10::optional<at::Tensor>& a2, const c10::optional<at::Tensor>& b2,
-                                     const c10::optional<at::Tensor>& sqnorm,
-                                     const c10::optional<at::Tensor>& seq_base);
-std::vector<at::Tensor> route_plan_rows(const at::Tensor& top_experts, int64_t num_experts, int64_t block,
-                                        int64_t capacity);
-
-at::Tensor combine_rows_op(const at::Tensor& x, const at::Tensor& inverse, const c10::optional<at::Tensor>& weights,
-                           int64_t top_k, int64_t tokens, const c10::optional<at::Tensor>& bias);
 
 // expert_block.cpp
 std::vector<at::Tensor> expert_rows_forward(const at::Tensor& x, const at::Tensor& top_experts, const at::Tensor& w1,
@@ -137,7 +108,6 @@ at::Tensor lbl_forward_op(const std::vector<at::Tensor>& scores, const std::vect
 std::vector<at::Tensor> lbl_backward_op(const std::vector<at::Tensor>& scores, const std::vector<at::Tensor>& counts,
                                         double scale, const at::Tensor& gout);
 at::Tensor rope_op(const at::Tensor& x, const at::Tensor& cosv, const at::Tensor& sinv, bool inverse);
-at::Tensor column_sum_op(const at::Tensor& x);
 
 // torch_glue.cpp: optimizer
 int64_t adam_record_size();

@@ -9,40 +9,10 @@
 // Two layouts, as in the layers (megablocks/layers/dmoe.py:196-249, moe.py:185-245 of the reference):
 //   capacity < 0   dropless: ragged row groups, weights [E, f, h], groups given by the plan's `bins`;
 //   capacity > 0   token-dropping: [E, capacity, h] slots, w1 [E, h, f], groups given by `gemm_bins`.
-#include <torch/extension.h>
-
 #include "kernels.h"
+#include "torch_ops.h"
 
 namespace mb {
-
-using OptTensor = c10::optional<at::Tensor>;
-
-std::vector<at::Tensor> route_plan_rows(const at::Tensor& top_experts, int64_t num_experts, int64_t block,
-                                        int64_t capacity);
-at::Tensor combine_rows_op(const at::Tensor& x, const at::Tensor& inverse, const OptTensor& weights, int64_t top_k,
-                           int64_t tokens, const OptTensor& bias);
-at::Tensor gather_rows_op(const at::Tensor& x, const at::Tensor& indices, const at::Tensor& bin_ids,
-                          const OptTensor& weights, const at::Tensor& bins, const at::Tensor& padded_bins,
-                          int64_t top_k, int64_t out_rows);
-at::Tensor binned_gather_rows(const at::Tensor& x, const at::Tensor& indices, const OptTensor& weights,
-                              const at::Tensor& bins, int64_t capacity, int64_t top_k);
-std::vector<at::Tensor> scatter_backward_op(const at::Tensor& x, const at::Tensor& grad, const at::Tensor& indices,
-                                            const at::Tensor& weights, const at::Tensor& bins,
-                                            const OptTensor& padded_bins, int64_t top_k);
-at::Tensor scatter_wgrad_op(const at::Tensor& x, const at::Tensor& grad, const at::Tensor& indices,
-                            const at::Tensor& bin_ids, const at::Tensor& bins, const at::Tensor& padded_bins,
-                            int64_t top_k);
-at::Tensor binned_scatter_wgrad(const at::Tensor& x, const at::Tensor& grad, const at::Tensor& indices,
-                                const at::Tensor& bins, int64_t top_k);
-at::Tensor column_sum_op(const at::Tensor& x);
-std::vector<at::Tensor> grouped_gemm_outputs(const at::Tensor& a, const at::Tensor& b, const at::Tensor& bins, bool trans_a,
-                                     bool trans_b, int64_t epilogue, int64_t act, const OptTensor& aux1,
-                                     const OptTensor& aux2, bool want_out2, bool want_out3, int64_t num_groups,
-                                     const OptTensor& c_in, bool zero_tail, const OptTensor& wait_flags,
-                                     int64_t wait_count, int64_t wait_stride, int64_t wait_seq, int64_t rows_hint,
-                                     int64_t pair_mode, const c10::optional<std::vector<at::Tensor>>& scatter,
-                                     const std::vector<int64_t>& scatter_args, double alpha, const OptTensor& a2,
-                                     const OptTensor& b2, const OptTensor& sqnorm, const OptTensor& seq_base, bool only_out2);
 
 namespace {
 
@@ -54,7 +24,7 @@ struct Gemm {
   double alpha = 1.0;
 
   std::vector<at::Tensor> run(const at::Tensor& a, const at::Tensor& b, const at::Tensor& bins, int64_t pair) const {
-    return grouped_gemm_outputs(a, b, bins, trans_a, trans_b, epilogue, act, aux1, aux2, want_out2, want_out3, bins.numel(), {},
+    return grouped_gemm(a, b, bins, trans_a, trans_b, epilogue, act, aux1, aux2, want_out2, want_out3, bins.numel(), {},
                         true, {}, 0, 0, 0, 0, pair, {}, {}, alpha, a2, b2, sqnorm, {}, only_out2);
   }
 };

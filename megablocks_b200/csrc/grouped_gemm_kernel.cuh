@@ -635,19 +635,19 @@ __device__ __forceinline__ void epilogue_by_act(const uint32_t (&raw)[32], const
 }
 
 // One dispatch per 32-column chunk (uniform across the warp); straight-line code inside.
-template <typename T, bool FRAG = false>
+template <typename T>
 __device__ __forceinline__ void epilogue_dispatch(const uint32_t (&raw)[32], const PackedRow& a1,
                                                   const PackedRow& a2, Staging& stage, int64_t base_off,
                                                   int64_t row_stride, int rows_ok, int cols, int lane,
                                                   const GemmParams& p, const ScatterRows<T>* scatter = nullptr,
                                                   int col = 0, TmaOut tma = TmaOut{false, 0}) {
   switch (p.epilogue) {
-    case kEpiNone: epilogue_chunk<T, kEpiNone, kActIdentity, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
-    case kEpiAdd: epilogue_chunk<T, kEpiAdd, kActIdentity, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
-    case kEpiAct: epilogue_by_act<T, kEpiAct, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
-    case kEpiDAct: epilogue_by_act<T, kEpiDAct, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
-    case kEpiGlu: epilogue_by_act<T, kEpiGlu, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
-    case kEpiDGlu: epilogue_by_act<T, kEpiDGlu, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
+    case kEpiNone: epilogue_chunk<T, kEpiNone, kActIdentity, false>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
+    case kEpiAdd: epilogue_chunk<T, kEpiAdd, kActIdentity, false>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
+    case kEpiAct: epilogue_by_act<T, kEpiAct>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
+    case kEpiDAct: epilogue_by_act<T, kEpiDAct>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
+    case kEpiGlu: epilogue_by_act<T, kEpiGlu>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
+    case kEpiDGlu: epilogue_by_act<T, kEpiDGlu>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
     default: break;
   }
 }

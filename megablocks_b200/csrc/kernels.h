@@ -57,7 +57,7 @@ cudaError_t gather_rows(DType type, const void* x, const int* indices, const voi
 cudaError_t inverse_map(const int* indices, const int* bins, const int* padded_bins, int num_bins, int n,
                         int capacity, int* inverse_filled_minus_one, cudaStream_t stream);
 cudaError_t combine_rows(DType type, const void* x, const int* inverse, const void* weights, const void* bias,
-                         int top_k, int64_t tokens, int cols, void* out, cudaStream_t stream);
+                         int top_k, int64_t tokens, int cols, int sms, void* out, cudaStream_t stream);
 cudaError_t scatter_bwd(DType type, const void* x, const void* grad, const int* indices, const void* weights,
                         const int* bins, const int* padded_bins, int num_bins, int capacity, int top_k, int64_t copies,
                         int64_t out_rows, int cols, void* dx, void* dweights, cudaStream_t stream);

@@ -126,8 +126,9 @@ __device__ void block_scan_totals(const int* __restrict__ totals, int nbins, int
 }
 
 // Row of the copy at sorted position `pos` of bin d: the position itself, or (capacity > 0) its slot of the
-// bin's `capacity` slots, -1 past them.  An id beyond the experts belongs to none: -1.  The plan knows it where it places the copy; the un-permutation
-// would otherwise search it again with a launch of its own, forward and backward.
+// bin's `capacity` slots, -1 past them.  An id beyond the experts belongs to none: -1.  The plan knows the
+// row where it places the copy; the un-permutation would otherwise search it again with a launch of its
+// own, forward and backward.
 __device__ __forceinline__ int row_of_copy(int pos, int bin_start, int d, int num_experts, int capacity) {
   if (d >= num_experts) return -1;
   if (capacity <= 0) return pos;

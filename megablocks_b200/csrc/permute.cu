@@ -64,9 +64,9 @@ __device__ __forceinline__ int copy_of_row(int64_t r, const int* __restrict__ in
 // out[r] = x[copy / top_k] (* weight[copy]) for every row r of the expert-ordered buffer, zero for pad rows.
 template <typename T, int VEC>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
-gather_rows_kernel(const T* __restrict__ x, const int* __restrict__ indices, const T* __restrict__ weights, const int* __restrict__ bins,
-                   const int* __restrict__ padded_bins, int num_bins, int capacity, int top_k, int64_t out_rows, int cols,
-                   T* __restrict__ out) {
+gather_rows_kernel(const T* __restrict__ x, const int* __restrict__ indices, const T* __restrict__ weights,
+                   const int* __restrict__ bins, const int* __restrict__ padded_bins, int num_bins, int capacity,
+                   int top_k, int64_t out_rows, int cols, T* __restrict__ out) {
   const int lane = threadIdx.x & 31;
   const int64_t r = int64_t(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
   if (r >= out_rows) return;
@@ -353,7 +353,7 @@ cudaError_t inverse_map(const int* indices, const int* bins, const int* padded_b
 }
 
 cudaError_t combine_rows(DType type, const void* x, const int* inverse, const void* weights, const void* bias,
-                         int top_k, int64_t tokens, int cols, void* out, cudaStream_t stream) {
+                         int top_k, int64_t tokens, int cols, int sms, void* out, cudaStream_t stream) {
   if (tokens == 0 || cols == 0) return cudaSuccess;
   MB_SWITCH_FLOAT(type, T, {
     constexpr int kFull = 16 / sizeof(T);
@@ -361,8 +361,8 @@ cudaError_t combine_rows(DType type, const void* x, const int* inverse, const vo
     const bool single = top_k == 1;
     const int step = (single ? 1 : kCombineChunks) * 32 * (wide ? kFull : 1);
     const int steps = ceil_div(cols, step);
-    // Top-1: slices enough for 64 warps on each of 148 SMs.  Otherwise one step a warp.
-    const int64_t wanted = (148 * 64 + tokens - 1) / tokens;
+    // Top-1: slices enough for 64 warps on every SM.  Otherwise one step a warp.
+    const int64_t wanted = (int64_t(sms) * 64 + tokens - 1) / tokens;
     int per_slice = single ? ceil_div(steps, wanted < steps ? static_cast<int>(wanted) : steps) : 1;
     per_slice = max(per_slice, ceil_div(steps, 65535));       // the grid's limit
     const int slices = ceil_div(steps, per_slice);

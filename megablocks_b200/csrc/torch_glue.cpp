@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "kernels.h"
+#include "torch_ops.h"
 
 namespace mb {
 
@@ -250,7 +251,8 @@ at::Tensor combine_rows_op(const at::Tensor& x, const at::Tensor& inverse, const
   at::Tensor out = at::empty({tokens, x.size(1)}, x.options());
   if (out.numel() == 0) return out;
   MB_CUDA_OK(combine_rows(float_code(x.scalar_type()), x.data_ptr(), inverse.data_ptr<int>(), opt_ptr(weights),
-                          opt_ptr(bias), int(top_k), tokens, int(x.size(1)), out.data_ptr(), stream()));
+                          opt_ptr(bias), int(top_k), tokens, int(x.size(1)), sm_count(), out.data_ptr(),
+                          stream()));
   MB_LAUNCHED(1);
   return out;
 }
@@ -356,7 +358,8 @@ at::Tensor scatter_rows_op(const at::Tensor& x, const at::Tensor& indices, const
   if (out.numel() == 0) return out;
   at::Tensor inverse = build_inverse(indices, bins, padded_bins, -1);
   MB_CUDA_OK(combine_rows(float_code(x.scalar_type()), x.data_ptr(), inverse.data_ptr<int>(), opt_ptr(weights),
-                          opt_ptr(bias), int(top_k), tokens, int(x.size(1)), out.data_ptr(), stream()));
+                          opt_ptr(bias), int(top_k), tokens, int(x.size(1)), sm_count(), out.data_ptr(),
+                          stream()));
   MB_LAUNCHED(1);
   return out;
 }
@@ -440,7 +443,8 @@ at::Tensor binned_scatter_rows(const at::Tensor& x, const at::Tensor& indices,
   if (out.numel() == 0) return out;
   at::Tensor inverse = build_inverse(indices, bins, bins, int(x.size(1)));
   MB_CUDA_OK(combine_rows(float_code(x.scalar_type()), x.data_ptr(), inverse.data_ptr<int>(), opt_ptr(weights),
-                          opt_ptr(bias), int(top_k), tokens, int(x.size(2)), out.data_ptr(), stream()));
+                          opt_ptr(bias), int(top_k), tokens, int(x.size(2)), sm_count(), out.data_ptr(),
+                          stream()));
   MB_LAUNCHED(1);
   return out;
 }
@@ -612,9 +616,7 @@ bool grouped_gemm_supported(const at::Tensor& a, const at::Tensor& b, bool trans
   return K == Kb && K % 8 == 0 && N % 8 == 0 && N >= 64 && K >= 8;
 }
 
-// `only_out2`: the activation epilogues (kEpiAct, kEpiGluDual) store nothing but the activation; c and
-// out3 come back undefined.
-std::vector<at::Tensor> grouped_gemm_outputs(const at::Tensor& a, const at::Tensor& b, const at::Tensor& bins, bool trans_a,
+std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, const at::Tensor& bins, bool trans_a,
                                      bool trans_b, int64_t epilogue, int64_t act,
                                      const c10::optional<at::Tensor>& aux1, const c10::optional<at::Tensor>& aux2,
                                      bool want_out2, bool want_out3, int64_t num_groups,
@@ -877,23 +879,6 @@ std::vector<at::Tensor> grouped_gemm_outputs(const at::Tensor& a, const at::Tens
   MB_CUDA_OK(launch(bf16, layout, block_n, ta, tb, p, grid, stream()));
   MB_LAUNCHED(1);
   return {c, out2, out3};
-}
-
-std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, const at::Tensor& bins, bool trans_a,
-                                     bool trans_b, int64_t epilogue, int64_t act,
-                                     const c10::optional<at::Tensor>& aux1, const c10::optional<at::Tensor>& aux2,
-                                     bool want_out2, bool want_out3, int64_t num_groups,
-                                     const c10::optional<at::Tensor>& c_in, bool zero_tail,
-                                     const c10::optional<at::Tensor>& wait_flags, int64_t wait_count,
-                                     int64_t wait_stride, int64_t wait_seq, int64_t rows_hint, int64_t pair_mode,
-                                     const c10::optional<std::vector<at::Tensor>>& scatter,
-                                     const std::vector<int64_t>& scatter_args, double alpha,
-                                     const c10::optional<at::Tensor>& a2, const c10::optional<at::Tensor>& b2,
-                                     const c10::optional<at::Tensor>& sqnorm,
-                                     const c10::optional<at::Tensor>& seq_base) {
-  return grouped_gemm_outputs(a, b, bins, trans_a, trans_b, epilogue, act, aux1, aux2, want_out2, want_out3, num_groups, c_in, zero_tail,
-                              wait_flags, wait_count, wait_stride, wait_seq, rows_hint, pair_mode, scatter, scatter_args, alpha, a2,
-                              b2, sqnorm, seq_base, false);
 }
 
 // ---------------------------------------------------------------------------

@@ -287,7 +287,7 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, bins: torch.Tensor, *, trans_
                                   int(count), int(stride), int(seq), int(rows_hint), pair_mode,
                                   scatter[0] if scatter is not None else None,
                                   scatter[1] if scatter is not None else [], float(alpha), a2, b2, slot_view,
-                                  seq_base)
+                                  seq_base, False)
         if slot is not None:
             sink._record(outs[0], slot)
         return outs
