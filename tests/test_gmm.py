@@ -440,6 +440,80 @@ def test_backward_as_the_first_cuda_work_of_its_thread():
     assert run.returncode == 0 and 'done' in run.stdout, run.stderr[-2000:]
 
 
+def _ragged(z, low, high):
+    return torch.randint(low, high, (z,), generator=torch.Generator().manual_seed(z + high)).tolist()
+
+
+def _fp32_groups(a, b, counts, trans_b):
+    """Per-group products in fp32 on the device."""
+    ends = torch.cumsum(torch.tensor(counts), 0).tolist()
+    out = torch.zeros(a.shape[0], b.shape[1] if trans_b else b.shape[2], device=a.device)
+    for e, (n, end) in enumerate(zip(counts, ends)):
+        w = b[e].float()
+        out[end - n:end] = a[end - n:end].float() @ (w.t() if trans_b else w)
+    return out
+
+
+# 74 pairs: some three ragged tiles a pair, and more than the 32 that a warp decodes at once.
+_MANY_TILES = [(_ragged(8, 500, 900), 72, 2304), (_ragged(66, 1, 20), 64, 9728)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('counts,k,n', _MANY_TILES, ids=['three', 'over-33'])
+@pytest.mark.parametrize('trans_b,epilogue', [(True, 'none'), (True, 'act'), (True, 'dact'), (True, 'dglu'),
+                                              (False, 'none'), (False, 'add'), (False, 'concat')])
+def test_cta_pair_over_several_tiles(counts, k, n, trans_b, epilogue):
+    """What a pair carries from one tile to the next: accumulator stages, the ring, prefetched auxiliary chunks,
+    the deal of chunks to warps, the second contraction."""
+    from megablocks_b200.utils import status
+    dtype = torch.bfloat16
+    a, b, bins = _pair_case(counts, k, n, trans_b, dtype)
+    aux1, aux2 = (torch.randn(a.shape[0], n, device='cuda').to(dtype) for _ in range(2))
+    acc = _fp32_groups(a, b, counts, trans_b)
+    if epilogue == 'concat':
+        a2, b2 = torch.randn_like(a), torch.randn_like(b) * 0.1
+        got, = G.grouped_gemm(a, b, bins, a2=a2, b2=b2, pair=1)[:1]
+        want = [acc + _fp32_groups(a2, b2, counts, False)]
+        got = [got]
+    else:
+        epi = getattr(G, 'EPI_' + epilogue.upper())
+        act = G.ACT_SILU if epilogue == 'dglu' else G.ACT_GELU_TANH
+        got = G.grouped_gemm(a, b, bins, trans_b=trans_b, epilogue=epi, act=act, aux1=aux1, aux2=aux2, pair=1)
+        want = G._cpu_epilogue(acc, epi, act, aux1, aux2, dtype)
+    status.check()
+    for g, w in zip(got, want):
+        if g is not None:
+            _close(g, w.float(), dtype)
+
+
+@pytest.mark.gpu
+def test_cta_pair_weight_gradient_over_more_tiles_than_a_window():
+    """140 groups x 2 x 9 tiles on 74 pairs, groups of 0 to 70 rows (whole, ragged and empty contractions)."""
+    from megablocks_b200.utils import status
+    counts = _ragged(140, 0, 71)
+    counts[3], counts[4] = 0, 64
+    a, _, bins = _pair_case(counts, 264, 264, True, torch.bfloat16)
+    dy = torch.randn(a.shape[0], 2304, device='cuda').bfloat16()
+    out, _, _ = G.grouped_gemm(a, dy, bins, trans_a=True, num_groups=140, pair=1)
+    status.check()
+    end = 0
+    for e, n in enumerate(counts):
+        _close(out[e], a[end:end + n].float().t() @ dy[end:end + n].float(), torch.bfloat16)
+        end += n
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('counts,k,n,trans_b', [
+    ([16] * 8, 64, 2304, True), ([16] * 7 + [17], 64, 2304, True), ([16] * 8, 64, 1792, False),     # streams weights
+    ([512] * 7 + [510], 2048, 4096, False), ([512] * 7 + [510], 2040, 4096, False),                  # few waves
+    ([3] * 224, 64, 512, True), ([3] * 225, 64, 512, True)])                                         # small tables
+def test_kernel_choice_on_both_sides_of_its_limits(counts, k, n, trans_b):
+    """The default choice between the pair and the single-CTA kernel, just inside and outside each rule."""
+    a, b, bins = _pair_case(counts, k, n, trans_b, torch.bfloat16)
+    out, _, _ = G.grouped_gemm(a, b, bins, trans_b=trans_b)
+    _close(out, _fp32_groups(a, b, counts, trans_b), torch.bfloat16)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize('which', ['a', 'b', 'c', 'aux1'])
 def test_misaligned_operands_and_short_outputs_are_refused_on_the_host(which):

@@ -499,7 +499,8 @@ def test_native_expert_block_equals_the_separate_ops(kind, dtype, tokens, top_k,
         moe_mod.clear_load_balancing_loss()
         return [y, plain] + list(torch.autograd.grad(y, [x] + list(layer.parameters()), dy))
 
-    assert layer.experts._block_call(x, *layer.router(x)[1:]) is not None or tokens * top_k < 5
+    assert layer.experts._block_call(x, *layer.router(x)[1:]) is not None or (
+        kind == 'dropping' and layer.experts.expert_capacity(tokens) == 0)
     moe_mod.clear_load_balancing_loss()
     fast = run()
     hook = layer.experts.mlp.register_forward_hook(lambda *a: None)
