@@ -103,7 +103,8 @@ __device__ void block_scan_totals(const int* __restrict__ totals, int nbins, int
   int sum = 0;
   for (int j = 0; j < per; ++j) {
     const int b = first + j;
-    local[j] = b < nbins ? ((totals[b] + block - 1) / block) * block : 0;
+    const int t = b < nbins ? totals[b] : 0;
+    local[j] = block == 1 ? t : ((t + block - 1) / block) * block;      // (a division is 2 us of a 37 us sort)
     sum += local[j];
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -138,7 +139,7 @@ __device__ __forceinline__ int row_of_copy(int pos, int bin_start, int d, int nu
 
 // Pass 3: stable placement.  Optionally (route plan) CTA 0 also writes the
 // per-bin totals, their inclusive prefix sums and the block-padded prefix sums.
-template <typename K, typename KO, typename V>
+template <typename K, typename KO, typename V, bool ROWS>
 __global__ void __launch_bounds__(kSortThreads)
 sort_place_kernel(const K* __restrict__ keys, const V* __restrict__ vals_in, int64_t n, int shift, int bits,
                   bool flip_sign, int chunk, int num_chunks, const int* __restrict__ partial,
@@ -186,7 +187,7 @@ sort_place_kernel(const K* __restrict__ keys, const V* __restrict__ vals_in, int
     if (valid) {
       keys_out[pos] = static_cast<KO>(key);
       vals_out[pos] = vals_in != nullptr ? vals_in[i] : static_cast<V>(i);
-      if (inverse != nullptr) inverse[i] = row_of_copy(pos, bin_base[d], d, num_real_bins, capacity);
+      if (ROWS && inverse != nullptr) inverse[i] = row_of_copy(pos, bin_base[d], d, num_real_bins, capacity);
     }
   }
 }
@@ -197,8 +198,8 @@ sort_place_kernel(const K* __restrict__ keys, const V* __restrict__ vals_in, int
 // Bound by latency, not by the 12 bytes an element moves: the three-launch sort takes 2 + 2 + 4.5 us
 // of kernels for 8 copies, and a launch to narrow the ids before it; this takes one launch.  Warps own
 // contiguous chunks and walk them in order twice (count, place), which keeps the order stable.  Up to
-// 4096 copies: 2.7 us for 8 and 4.5 for 4096 against 8.6 and 13.4 of the sort as it was; at 8192 one
-// CTA's walk takes 11.8 us, longer than the three launches (9.1 us at 32768).
+// 4096 copies over 64 experts, launches replayed back to back: 3.2 us for 8 and 8.4 for 4096 against 9.4 and
+// 17.1 of narrowing and sorting; from there on the three launches are no slower (9.2 us for 4097 and 8192).
 constexpr int kPlanThreads = 1024;
 constexpr int kPlanWarps = kPlanThreads / 32;
 
@@ -301,7 +302,7 @@ cudaError_t sort_pass(DType key_type, const void* keys, const void* vals_in, int
                                                                     flip_sign, chunk, num_chunks, partial);
     sort_scan_kernel<<<nbins, 256, 0, stream>>>(partial, num_chunks, totals);
     // Values carry the key dtype (the reference returns the permutation in it).
-    sort_place_kernel<K, K, K><<<grid, kSortThreads, place_smem, stream>>>(
+    sort_place_kernel<K, K, K, false><<<grid, kSortThreads, place_smem, stream>>>(
         static_cast<const K*>(keys), static_cast<const K*>(vals_in), n, shift, bits, flip_sign, chunk, num_chunks,
         partial, totals, static_cast<K*>(keys_out), static_cast<K*>(vals_out), tpe, bins, padded_bins,
         num_real_bins, block, nullptr, 0);
@@ -319,7 +320,7 @@ cudaError_t route_sort64(const int64_t* keys, int64_t n, int bits, int chunk, in
   sort_hist_kernel<int64_t><<<grid, kSortThreads, size_t(kSortWarps) * nbins * sizeof(int), stream>>>(
       keys, n, 0, bits, false, chunk, num_chunks, partial);
   sort_scan_kernel<<<nbins, 256, 0, stream>>>(partial, num_chunks, totals);
-  sort_place_kernel<int64_t, int, int>
+  sort_place_kernel<int64_t, int, int, true>
       <<<grid, kSortThreads, size_t(nbins + 8 + kSortWarps * nbins) * sizeof(int), stream>>>(
           keys, nullptr, n, 0, bits, false, chunk, num_chunks, partial, totals, bin_ids, indices, tpe, bins, padded_bins,
           num_experts, block, inverse, capacity);
