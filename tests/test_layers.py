@@ -788,16 +788,19 @@ def test_plan_drops_copies_of_no_expert(copies, capacity):
 @pytest.mark.gpu
 @pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize('top_k', [1, 2, 3, 5])
-@pytest.mark.parametrize('hidden', [8, 100, 512, 520, 1032])
-def test_combine_slices_and_copy_pairs(dtype, top_k, hidden):
-    """Un-permutation over row lengths around a warp's slice and odd numbers of copies, some dropped."""
+@pytest.mark.parametrize('tokens,hidden', [(19, 8), (19, 100), (19, 512), (19, 520), (19, 1032), (5000, 8), (9600, 264),
+                                           (9600, 8)])
+def test_combine_slices_and_copy_pairs(dtype, top_k, tokens, hidden):
+    """Un-permutation over row lengths around a warp's slice, odd numbers of copies, some dropped, and token
+    counts on both sides of those that fill the SMs."""
     torch.manual_seed(hidden)
-    tokens, experts, capacity = 19, 4, 9
+    experts, capacity = 4, tokens // 2
     top = torch.randint(0, experts, (tokens * top_k,))
     indices, _, bins, _, _ = ops.route_plan(top, experts)
     x = torch.randn(experts, capacity, hidden).to(dtype)
     w = torch.rand(tokens * top_k).to(dtype)
     got = ops.binned_scatter(x.cuda(), indices.cuda(), w.cuda(), bins.cuda(), top_k)
     want = ops.binned_scatter(x, indices, w, bins, top_k)
-    # The same products and the same order of the sum: one rounding at most apart.
-    torch.testing.assert_close(got.cpu().float(), want.float(), rtol=torch.finfo(dtype).eps, atol=1e-6)
+    # The same products, then one rounding; fp32 sums of top_k terms below 6 in any order.
+    torch.testing.assert_close(got.cpu().float(), want.float(), rtol=torch.finfo(dtype).eps,
+                               atol=1e-6 + 6 * top_k ** 2 * 2 ** -24)
