@@ -786,34 +786,48 @@ std::vector<at::Tensor> grouped_gemm(const at::Tensor& a, const at::Tensor& b, c
   // pair_mode: 1 = whenever supported, 0 = never, anything else = the rule.
   (void)rows_hint;
   //
-  // Rule: pairs, except where a launch only streams weights - at most 16 rows a group, and enough column
-  // tiles to give half of the SMs one.  There the single-CTA kernel keeps more weight bytes in flight per
-  // SM (128 KB against 80): 32 rows over 8 groups of 14336 x 4096, NN 159 us against 178, NT 191 against
-  // 194.  With fewer tiles the pairs' halved tile width wins: 8 rows over 64 groups of 3072 x 768, NN 34
-  // us against 26.  With more rows pairs win or draw on every shape measured (TFLOP/s sustained, single |
-  // pair): 8192 x 4096 x 14336, 8 groups, NT + GELU 1013 | 1053, GELU-bwd 988 | 1035, GLU-bwd 860 | 936,
-  // NN 985 | 1017, TN 980 | 1073; 32768 x 768 x 3072, 64 groups: 645 | 731, 535 | 658, 322 | 479,
-  // 824 | 821, 750 | 779; 10006 x 1024 x 4096, 32 groups: 625 | 692, 543 | 641, 349 | 511, 717 | 763,
-  // 588 | 635.
+  // Rule: pairs, except
+  // (1) where a launch only streams weights - at most 16 rows a group, and enough column tiles to give half
+  // of the SMs one.  There the single-CTA kernel keeps more weight bytes in flight per SM (128 KB against
+  // 80): 32 rows over 8 groups of 14336 x 4096, NN 159 us against 178, NT 191 against 194.  With fewer tiles
+  // the pairs' halved tile width wins: 8 rows over 64 groups of 3072 x 768, NN 34 us against 26;
+  // (2) where a pair's last wave of tiles costs more than its loop gains: a pair's tiles are twice as large.
+  // Compared by waves x cycles of a tile, for launches of up to six waves without auxiliary operands: per K
+  // step 512 on one CTA, and 256 for the weights' load and one per token on a pair; 2000 once per tile for
+  // the eight epilogue warps of the one against the twelve of the other; half a tile per group for the
+  // raggedness.  us, single | pair: 4094 x 14336 -> 4096, 8 groups 508 | 583; 2048 x 8192 -> 2048, 4 groups 75 |
+  // 114; 1000 x 768 -> 3072, 8 groups 14.5 | 16.9; and outside the rule 4096 x 4096 -> 1024, 16 groups 67 | 62;
+  // (3) activation backward over deep contractions whose weights stream past L2, below 128 rows a group (one row
+  // tile): the single-CTA kernel's extra bytes in flight again, against the pair's auxiliary buffers, which
+  // cost it a stage.  8 groups of 14336 x 4096, 64 to 800 rows, GELU-bwd 183..192 | 201..216, GLU-bwd 190..207 |
+  // 203..225; 32 groups of 2880 x 2880, 4000 rows, 127 | 142, 142 | 151.  At a depth of 2048 GELU-bwd takes 62 | 68
+  // (256 rows, 8 groups of 8192) but GLU-bwd 75 | 70, and at 1024 pairs win both.
+  //
+  // Over 666 launches (NT plain / GELU / GELU-bwd / GLU-bwd, NN, two pairs; 256 to 65536 ragged rows, 4 to 64
+  // groups, hidden 256 to 4096) the rule costs 2 % against the better kernel each time.  Pairs lose where the
+  // draw of the group sizes spills a few tiles into one more wave (4096 x 3072 -> 768, 16 groups: NN 34 | 46).
+  // Long launches under the power cap (back to back, single | pair us): 32768 rows, 768 / 3072, 64 groups
+  // TN 209 | 205, NN 184 | 189, two pairs 340 | 350; 8192 rows, 4096 / 14336, 8 groups 991 | 915, 969 | 928,
+  // 1925 | 1849; 10006 rows, 1024 / 4096, 32 groups 148 | 135, 119 | 111, 224 | 213.
   const bool streams_weights = layout != kTN && a.size(0) <= 16 * num_groups &&
                                (1 + std::min<int64_t>(num_groups, a.size(0))) * ceil_div(p.N, 256) >= sm_count() / 2;
-  // A long contraction over few waves of tiles: a pair's tiles are twice as large, and the last wave can
-  // cost it more than its loop gains.  Compared by waves x cycles of a K step (256 for the weights' load
-  // and one per token of a tile; the single-CTA loop runs 7 % longer), with half a tile per group for the
-  // raggedness.  4094 rows over 8 groups, 14336 -> 4096: single 447 us, pair 502.
   auto few_waves_lose = [&] {
-    if (layout == kTN || p.K < 2048 || (epilogue != kEpiNone && epilogue != kEpiAct)) return false;
-    const double rows = double(a.size(0)), groups = double(num_groups), nb = double(ceil_div(p.N, 256));
+    if (layout == kTN || (epilogue != kEpiNone && epilogue != kEpiAct)) return false;
+    const double rows = double(a.size(0)), groups = double(std::min<int64_t>(num_groups, a.size(0)));
+    const double steps = double(ceil_div(p.K, 64)) * (concat ? 2 : 1), nb = double(ceil_div(p.N, 256));
     const double tiles2 = rows / 256 + 0.5 * groups, tiles1 = rows / 128 + 0.5 * groups;
     const double waves2 = std::ceil(tiles2 * nb / (sm_count() / 2)), waves1 = std::ceil(tiles1 * nb / sm_count());
-    return waves2 <= 6 && waves1 * 512 * 1.07 < waves2 * (256 + rows / tiles2);
+    return waves2 <= 6 && waves1 * (512 * steps + 2000) < waves2 * (256 + rows / tiles2) * steps;
   };
+  const int64_t aux_depth = epilogue == kEpiDAct ? 2048 : (epilogue == kEpiDGlu ? 2560 : 0);
+  const bool streams_with_aux = layout != kTN && aux_depth > 0 && p.K >= aux_depth && a.size(0) < 128 * num_groups &&
+                                num_groups * int64_t(p.N) * p.K * 2 >= (int64_t(200) << 20);
   bool pair_ok = block_n == 256 && !dual && p.N >= 256 && sm_count() >= 2 && !scatter.has_value() &&
                  !wait_flags.has_value() && num_groups <= kSmallGroupsHost &&
                  (layout != kTN || epilogue == kEpiNone) && pair_mode != 0;
   if (pair_ok && p.aux1) pair_ok = make_output_map(&p.aux_map[0], p.aux1, bf16, out_numel / p.N, p.N);
   if (pair_ok && p.aux2) pair_ok = make_output_map(&p.aux_map[1], p.aux2, bf16, out_numel / p.N, p.N);
-  const bool pair = pair_ok && (pair_mode == 1 || !(streams_weights || few_waves_lose()));
+  const bool pair = pair_ok && (pair_mode == 1 || !(streams_weights || streams_with_aux || few_waves_lose()));
   if (!scatter.has_value() && store_tma_enabled()) {
     // Full 32-row quarters of a tile leave through the TMA unit (one instruction per chunk).
     const int64_t out_rows = out_numel / p.N;

@@ -440,6 +440,21 @@ def test_backward_as_the_first_cuda_work_of_its_thread():
     assert run.returncode == 0 and 'done' in run.stdout, run.stderr[-2000:]
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize('rows,k,epilogue', [(127, 2048, 'dact'), (128, 2048, 'dact'), (127, 2560, 'dglu'), (127, 2552, 'dglu')])
+def test_activation_backward_on_both_sides_of_its_streaming_rule(rows, k, epilogue):
+    """Deep contractions below 128 rows a group over more weights than L2 holds: the default choice of kernel."""
+    counts, n = [rows] * 4, 13312
+    a, b, bins = _pair_case(counts, k, n, True, torch.bfloat16)
+    aux1, aux2 = (torch.randn(a.shape[0], n, device='cuda').bfloat16() for _ in range(2))
+    epi, act = getattr(G, 'EPI_' + epilogue.upper()), G.ACT_SILU
+    got = G.grouped_gemm(a, b, bins, trans_b=True, epilogue=epi, act=act, aux1=aux1, aux2=aux2)
+    want = G._cpu_epilogue(_fp32_groups(a, b, counts, True), epi, act, aux1, aux2, torch.bfloat16)
+    for g, w in zip(got, want):
+        if g is not None:
+            _close(g, w.float(), torch.bfloat16)
+
+
 def _ragged(z, low, high):
     return torch.randint(low, high, (z,), generator=torch.Generator().manual_seed(z + high)).tolist()
 
@@ -505,7 +520,7 @@ def test_cta_pair_weight_gradient_over_more_tiles_than_a_window():
 @pytest.mark.gpu
 @pytest.mark.parametrize('counts,k,n,trans_b', [
     ([16] * 8, 64, 2304, True), ([16] * 7 + [17], 64, 2304, True), ([16] * 8, 64, 1792, False),     # streams weights
-    ([512] * 7 + [510], 2048, 4096, False), ([512] * 7 + [510], 2040, 4096, False),                  # few waves
+    ([512] * 7 + [510], 2048, 4096, False), ([125] * 8, 768, 3072, True), ([512] * 8, 768, 3072, False),   # few waves
     ([3] * 224, 64, 512, True), ([3] * 225, 64, 512, True)])                                         # small tables
 def test_kernel_choice_on_both_sides_of_its_limits(counts, k, n, trans_b):
     """The default choice between the pair and the single-CTA kernel, just inside and outside each rule."""
