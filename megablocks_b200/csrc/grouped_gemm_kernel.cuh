@@ -611,13 +611,14 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&raw)[32], const 
   }
 }
 
-template <typename T, int EPI, bool FRAG = false>
+// FULL: which activations the caller's kernel holds - 0 the plain ones, 1 the Full ones, 2 both.
+template <typename T, int EPI, bool FRAG = false, int FULL = 2>
 __device__ __forceinline__ void epilogue_by_act(const uint32_t (&raw)[32], const PackedRow& a1,
                                                 const PackedRow& a2, Staging& stage, int64_t base_off,
                                                 int64_t row_stride, int rows_ok, int cols, int lane,
                                                 const GemmParams& p, const ScatterRows<T>* scatter, int col,
                                                 TmaOut tma) {
-  if constexpr (EPI == kEpiAct || EPI == kEpiDAct) {
+  if constexpr (FULL > 0 && (EPI == kEpiAct || EPI == kEpiDAct)) {
     switch (p.act) {
       case kActGeluTanhFull: epilogue_chunk<T, EPI, kActGeluTanhFull, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); return;
       case kActSiluFull: epilogue_chunk<T, EPI, kActSiluFull, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); return;
@@ -625,6 +626,7 @@ __device__ __forceinline__ void epilogue_by_act(const uint32_t (&raw)[32], const
       default: break;
     }
   }
+  if constexpr (FULL == 1) return;
   switch (p.act) {
     case kActGeluTanh: epilogue_chunk<T, EPI, kActGeluTanh, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
     case kActSilu: epilogue_chunk<T, EPI, kActSilu, FRAG>(raw, a1, a2, stage, base_off, row_stride, rows_ok, cols, lane, p, scatter, col, tma); break;
